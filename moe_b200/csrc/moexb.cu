@@ -6,7 +6,7 @@
 #include "formats.cuh"
 #include "stream.cuh"
 #include "tiled.cuh"
-#include "prefill.cuh"
+#include "grouped.cuh"
 #include "decode_stack.cuh"
 #include "ep.cuh"
 #include "gguf_ingest.h"
@@ -138,7 +138,7 @@ struct moexb_ctx {
     uint16_t *xs = nullptr, *act_split = nullptr;       // activations / act as 16-bit hi + lo halves, permuted
     moexb_pair_item* subs = nullptr;                    // sub-items of at most 8 pairs
     int *nsub = nullptr, *err = nullptr;
-    moexb_pair_item* subs2 = nullptr; int* nsub2 = nullptr;   // second sub-item list (the down tiles of the tensor-core path)
+    float *sx = nullptr, *sx_act = nullptr;             // grouped GEMM, zero point: activation sums per 32-input chunk, of the tokens and of act
     int* route_done = nullptr;                          // per token tile: blocks of the routing kernel that have finished (returns to zero)
     int sms = 0, path = 0;                              // path: 0 = streaming kernels, 1 = fp32 SIMT kernels
     int fused_decode = 1;                               // one-token residual stacks run as one cooperative launch
@@ -481,7 +481,7 @@ int moexb_ctx_create(int device, int max_tokens, int max_experts, int top_k, moe
     A(&c->counts, (size_t)max_experts); A(&c->nitems, 1); A(&c->items, (size_t)max_experts + 1); A(&c->pairs, P);
     A(&c->slots, (size_t)top_k + 1); A(&c->wts, (size_t)top_k + 1);
     A(&c->xs, T * 2 * EH); A(&c->act_split, P * 2 * EI); A(&c->subs, (size_t)max_experts + 1 + P / ST_MAXP + 1);
-    A(&c->nsub, 2); A(&c->err, 1); A(&c->subs2, (size_t)max_experts + 1 + P / (PF_NMAX / 2) + 1); A(&c->nsub2, 1); A(&c->route_done, (size_t)max_tokens); A(&c->staging, (size_t)STAGING_BLOBS * expert_bytes(FMT_ZP));
+    A(&c->nsub, 2); A(&c->err, 1); A(&c->sx, T * (EH / 32)); A(&c->sx_act, P * (EI / 32)); A(&c->route_done, (size_t)max_tokens); A(&c->staging, (size_t)STAGING_BLOBS * expert_bytes(FMT_ZP));
     if (rc == MOEXB_OK && cudaMemset(c->err, 0, sizeof(int)) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: memset");
     if (rc == MOEXB_OK && cudaMemset(c->route_done, 0, (size_t)max_tokens * sizeof(int)) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: memset");
     if (rc == MOEXB_OK && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: device attribute");
@@ -1044,39 +1044,42 @@ static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* 
 // ---- prefill: grouped GEMM on tcgen05 ----------------------------------------------------------------------------------------
 
 template <int FMT, bool DOWN>
-static int prefill_launch_one(moexb_ctx* c, const PrefillArgs& a, void* stream) {
-    constexpr int SMEM = pf_smem_bytes<FMT, DOWN>();
+static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, void* stream) {
+    constexpr int SMEM = gg_smem_bytes<FMT>();
     static PerDeviceOnce once;
-    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(prefill_k<FMT, DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
-    if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "prefill kernel shared memory: %s", cudaGetErrorString(attr_err));
+    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(grouped_k<FMT, DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
+    if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "grouped GEMM shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
-    prefill_k<FMT, DOWN><<<c->sms, PF_THREADS, SMEM, S(stream)>>>(a);
-    LAUNCHED(DOWN ? "prefill_down" : "prefill_gate_up");
+    CUDA_TRY(launch_dep(grouped_k<FMT, DOWN>, c->sms, GG_THREADS, SMEM, S(stream), a));
+    LAUNCHED(DOWN ? "grouped_down" : "grouped_gate_up");
     return MOEXB_OK;
 }
 
-// Experts of a large batch on the tensor-core grouped GEMM: items/nitems = the grouped work list (tiled blobs), xf = the
-// activations as fp32 [T][H]; parts = 1 when xf holds exact bf16 values, else 2.
-static int prefill_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, const float* xf, int T, int parts, float* ypair, void* stream,
-                           bool pre_split = false) {
-    if (!pre_split) {   // pre_split: the context already holds the fp16 columns (expert parallelism: the token owners made them)
-        PROF(c, MOEXB_PROF_OTHER, stream);
-        const size_t n = (size_t)T * EH;
-        split8_rows_k<<<(unsigned)((n + 255) / 256), 256, 0, S(stream)>>>(xf, c->xs, EH, parts, n);
-        LAUNCHED("split8_rows");
-    }
-    // the planner left two tile lists in the context: subs (up to 128 / parts pairs: gate/up) and subs2 (up to 64 pairs: down,
-    // whose act columns are always hi + lo)
-    auto run = [&]<int FMT>() {
-        PrefillArgs a{c->subs, c->nsub, pairs, c->xs, c->act_split, nullptr, ypair, c->err, parts};
-        int rc = prefill_launch_one<FMT, false>(c, a, stream);
+// Batches from this size on run on the grouped GEMM.
+static int grouped_min_tokens(const moexb_ctx* c, int fmt) { return c->prefill_min_tokens; }
+
+// Pairs per tile of the grouped GEMM.
+static int grouped_maxp(int fmt) { return fmt == FMT_ZP ? gg_nmax<FMT_ZP>() : gg_nmax<FMT_SYM_F16>(); }
+
+// The activations as the grouped GEMM's rows, into the context. parts = 1 when x holds exact bf16 values, else 2.
+static int grouped_rows(moexb_ctx* c, int fmt, const float* x, uint16_t* xs, int rows, int parts, void* stream) {
+    PROF(c, MOEXB_PROF_OTHER, stream);
+    if (fmt == FMT_ZP) grouped_rows_k<true><<<rows, 256, 0, S(stream)>>>(x, xs, c->sx, parts);
+    else grouped_rows_k<false><<<rows, 256, 0, S(stream)>>>(x, xs, nullptr, parts);
+    LAUNCHED("grouped_rows");
+    return MOEXB_OK;
+}
+
+// Experts of a large batch on the tensor-core grouped GEMM: the planner left the tiles in the context (subs, nsub), grouped_rows or
+// the token owners (expert parallelism) the activation rows.
+static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int parts, float* ypair, void* stream) {
+    return by_fmt(fmt, [&]<int FMT>() {
+        GroupedArgs a{c->subs, c->nsub, pairs, c->xs, c->sx, c->act_split, c->sx_act, ypair, c->err, parts};
+        int rc = grouped_launch_one<FMT, false>(c, a, stream);
         if (rc != MOEXB_OK) return rc;
-        PrefillArgs d = a;
-        d.tiles = c->subs2; d.ntiles = c->nsub2; d.xs = c->act_split; d.parts = 2;
-        return prefill_launch_one<FMT, true>(c, d, stream);
-    };
-    if (fmt == FMT_SYM_F16) return run.template operator()<FMT_SYM_F16>();
-    return fail(MOEXB_ERR_UNSUPPORTED, "prefill kernels: format %d", fmt);
+        a.xs = c->act_split; a.sx = c->sx_act; a.parts = 2;
+        return grouped_launch_one<FMT, true>(c, a, stream);
+    });
 }
 
 // f16: the consumer is the tiled kernel of a symmetric format (fp16 operands); otherwise bf16
@@ -1230,8 +1233,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
     cudaStream_t st = S(stream);
     const bool tiled = L->layout == MOEXB_LAYOUT_TILED;
     const bool streaming = tiled || c->path == 0;
-    // large batches of symmetric-format experts go to the tcgen05 grouped GEMM (bf16 operands); the rest to the streaming kernels
-    const bool prefill = tiled && L->fmt == FMT_SYM_F16 && T >= c->prefill_min_tokens;
+    // large batches go to the tcgen05 grouped GEMM; the rest to the streaming kernels
+    const bool prefill = tiled && T >= grouped_min_tokens(c, L->fmt);
     const bool f16 = tiled && L->fmt != FMT_ZP && !prefill;  // element type of the split activations the streaming kernels read
     const float* xf = xin;  // what the router and the experts see
     if (block) {
@@ -1239,14 +1242,14 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
         if (!pre_normed) {
             PROF(c, MOEXB_PROF_OTHER, stream);
             if (f16) rmsnorm_split_k<true><<<T, 256, 0, st>>>(xin, c->xn, c->xs, 1e-6f);
-            else rmsnorm_split_k<false><<<T, 256, 0, st>>>(xin, c->xn, c->xs, 1e-6f);
+            else rmsnorm_split_k<false><<<T, 256, 0, st>>>(xin, c->xn, prefill ? nullptr : c->xs, 1e-6f);
             LAUNCHED("rmsnorm_split");
         }
     } else if (streaming && !prefill) {
         const int rc = split_launch(c, xf, T, f16, stream);
         if (rc != MOEXB_OK) return rc;
     }
-    const bool decode = T == 1 && all_local && shared && !partial;
+    const bool decode = T == 1 && all_local && shared && !partial && !prefill;
     int rc = layer_route(c, L, xf, T, K, stream, decode);
     if (rc != MOEXB_OK) return rc;
     int ranks = K;                  // rows of ypair per token that the final reduction adds
@@ -1269,7 +1272,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
         ranks = K + 1;
     } else {
         const int parts = (x_bf16 && !block) ? 1 : 2;
-        const int maxp = prefill ? PF_NMAX / parts : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
+        const int maxp = prefill ? grouped_maxp(L->fmt) : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
         const bool in_kernel = tiled && !prefill && plan_in_kernel(c, L->fmt, T, K, E);
         const PlanArgs plan{c->idx, c->w, T, K, E, L->slot_table, L->first_local, L->first_local + L->n_local, shared ? c->logits + E : nullptr, ld, sh0, sh1, maxp, c->subs, c->pairs, c->nsub, nullptr, nullptr, 0u};
         if (!in_kernel) {
@@ -1280,14 +1283,18 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
             const cudaError_t plan_attr = plan_once.run([] { return cudaFuncSetAttribute(group_plan1_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_STAGE_MAX); });
             const int stage_pairs = plan_attr == cudaSuccess && (size_t)T * K * 12 <= PLAN_STAGE_MAX ? T * K : 0;
             CUDA_TRY(launch_dep(group_plan1_k<false>, 1, 1024, (size_t)stage_pairs * 12, st, c->idx, c->w, T, K, E, L->slot_table, c->items, c->pairs, c->nitems, c->subs, c->nsub, maxp,
-                                prefill ? c->subs2 : nullptr, c->nsub2, PF_NMAX / 2, shared ? c->logits + E : nullptr, ld, sh0, sh1, stage_pairs,
+                                shared ? c->logits + E : nullptr, ld, sh0, sh1, stage_pairs,
                                 (const unsigned*)nullptr, (const unsigned*)nullptr, 0u, 0, 0, (int*)nullptr));
             LAUNCHED("group_plan");
             // pairs of experts that are not held here are never written: the SIMT reduction path needs zeros there, the fused
             // reduction skips them by expert id
             if (!all_local && !streaming) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)T * K * EH * sizeof(float), st));
         }
-        rc = prefill ? prefill_experts(c, L->fmt, c->pairs, xf, T, parts, c->ypair, stream)
+        if (prefill) {
+            rc = grouped_rows(c, L->fmt, xf, c->xs, T, parts, stream);
+            if (rc != MOEXB_OK) return rc;
+        }
+        rc = prefill ? grouped_experts(c, L->fmt, c->pairs, parts, c->ypair, stream)
            : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, in_kernel ? &plan : nullptr)
            : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream)
                        : pairs_launch(c, L->fmt, c->items, c->nitems, min(E, T * K) + 1, c->pairs, xf, c->act, c->ypair, stream);
@@ -1300,7 +1307,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
         float* xn_next = next_norm ? c->xn : nullptr;
         const int* held = (!all_local && ranks == K) ? c->idx : nullptr;
         if (f16) CUDA_TRY(launch_dep(reduce_residual_norm_k<true>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local));
-        else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local));
+        else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, prefill ? (uint16_t*)nullptr : c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local));
         LAUNCHED("reduce_residual_norm");
     }
     if (idx_out) CUDA_TRY(cudaMemcpyAsync(idx_out, c->idx, (size_t)T * K * sizeof(int), cudaMemcpyDeviceToDevice, st));
@@ -1675,7 +1682,8 @@ int moexb_ep_dispatch(moexb_ep* e, moexb_layer* L, int l, const void* X, int x_d
     const int T = e->g.T, K = e->g.K, t0 = e->g.tok0[e->g.rank], n_own = e->g.tok0[e->g.rank + 1] - t0;
     const bool tiled = L->layout == MOEXB_LAYOUT_TILED;
     REQUIRE(tiled || c->path == 0, "ep_dispatch: expert parallelism runs on the streaming kernels");
-    const bool prefill = tiled && L->fmt == FMT_SYM_F16 && T >= c->prefill_min_tokens;
+    // (zero point stays on the streaming kernels: the grouped GEMM's chunk sums are not among what the owners send)
+    const bool prefill = tiled && L->fmt != FMT_ZP && T >= grouped_min_tokens(c, L->fmt);
     const bool f16 = tiled && L->fmt != FMT_ZP && !prefill;
     // activation columns per token: the grouped GEMM takes one when the layer input is exactly bf16, else hi + lo
     const int parts = prefill && x_dtype == MOEXB_BF16 && !residual && l == 0 ? 1 : 2;
@@ -1708,9 +1716,8 @@ int moexb_ep_dispatch(moexb_ep* e, moexb_layer* L, int l, const void* X, int x_d
     }
     if (prefill) {
         PROF(c, MOEXB_PROF_OTHER, stream);
-        const size_t n = (size_t)n_own * EH;
-        split8_rows_k<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * parts * EH, EH, parts, n);
-        LAUNCHED("split8_rows");
+        rc = grouped_rows(c, L->fmt, xn_own, c->xs + (size_t)t0 * parts * EH, n_own, parts, stream);
+        if (rc != MOEXB_OK) return rc;
     }
     // the routing kernel sends each token to the peers as soon as its experts are selected and raises the tokens' flags
     const RouteEp rep{e->dev, parts * EH * 2, (unsigned)(l + 1), e->step};
@@ -1724,7 +1731,7 @@ int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
     cudaStream_t st = S(stream);
     const int T = e->g.T, K = e->g.K, E = L->n_routed, t0 = e->g.tok0[e->g.rank], t1 = e->g.tok0[e->g.rank + 1];
     const bool tiled = L->layout == MOEXB_LAYOUT_TILED, prefill = e->prefill;
-    const int maxp = prefill ? PF_NMAX / e->parts : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
+    const int maxp = prefill ? grouped_maxp(L->fmt) : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
     const unsigned* flags = reinterpret_cast<const unsigned*>(e->peers.base[e->g.rank] + e->lay.flag_a);
     const bool in_kernel = tiled && !prefill && plan_in_kernel(c, L->fmt, T, K, E, true);
     // the dispatch flags of all tokens are waited for by whoever makes the work list: the gate/up CTAs, or the planning kernel
@@ -1736,11 +1743,11 @@ int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
         const cudaError_t plan_attr = plan_once.run([] { return cudaFuncSetAttribute(group_plan1_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PLAN_STAGE_MAX); });
         const int stage_pairs = plan_attr == cudaSuccess && (size_t)T * K * 12 <= PLAN_STAGE_MAX ? T * K : 0;
         CUDA_TRY(launch_dep(group_plan1_k<true>, 1, 1024, (size_t)stage_pairs * 12, st, (const int*)c->idx, (const float*)c->w, T, K, E, L->slot_table, c->items, c->pairs, c->nitems,
-                            c->subs, c->nsub, maxp, prefill ? c->subs2 : nullptr, c->nsub2, PF_NMAX / 2, (const float*)(c->logits + E), E + 1, t0, t1, stage_pairs,
+                            c->subs, c->nsub, maxp, (const float*)(c->logits + E), E + 1, t0, t1, stage_pairs,
                             flags, (const unsigned*)e->step, (unsigned)(l + 1), e->g.world, e->g.rank, c->err));
         LAUNCHED("group_plan");
     }
-    rc = prefill ? prefill_experts(c, L->fmt, c->pairs, nullptr, T, e->parts, c->ypair, stream, true)
+    rc = prefill ? grouped_experts(c, L->fmt, c->pairs, e->parts, c->ypair, stream)
        : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, in_kernel ? &plan : nullptr)
                : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream);
     if (rc != MOEXB_OK) return rc;

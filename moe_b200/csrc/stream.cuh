@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(256) rmsnorm_split_k(const float* __restrict__
     float v[8];
     const float4 a = *reinterpret_cast<const float4*>(x + t * EH + 4 * threadIdx.x), b = *reinterpret_cast<const float4*>(x + t * EH + 1024 + 4 * threadIdx.x);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    norm_split_row<F16>(v, xn + t * EH, xs + t * 2 * EH, eps);
+    norm_split_row<F16>(v, xn + t * EH, xs ? xs + t * 2 * EH : nullptr, eps);
 }
 
 // The end of a layer in one pass over the token's row: moe[t] = sum_{r<K} ypair[t*K+r] in rank order (+ extra[t]: the
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __res
         *reinterpret_cast<float4*>(out + t * EH + k0) = acc;
         v[4 * h] = acc.x; v[4 * h + 1] = acc.y; v[4 * h + 2] = acc.z; v[4 * h + 3] = acc.w;
     }
-    if (xn_next) norm_split_row<F16>(v, xn_next + t * EH, xs_next + t * 2 * EH, eps);
+    if (xn_next) norm_split_row<F16>(v, xn_next + t * EH, xs_next ? xs_next + t * 2 * EH : nullptr, eps);
 }
 
 // Exclusive prefix sum over the 1024 threads of a block; every thread also gets the total.
@@ -488,12 +488,11 @@ __device__ __forceinline__ int block_scan_1024(int v, int& total) {
 }
 
 // Grouping and planning of a batch in one block of 1024 threads (one expert per thread; E <= 1024): the (token, rank) pairs
-// bucketed by expert (the host loop of moex.cu:1466-1486), the sub-items of at most maxp pairs that the streaming kernels
-// walk, and optionally a second sub-item list with another width (the tensor-core kernels take 128 / parts pairs per tile
-// for gate/up and 64 for down). Histogram of the T*K pairs in shared memory, block scans, then
+// bucketed by expert (the host loop of moex.cu:1466-1486), and the sub-items of at most maxp pairs that the streaming kernels
+// and the grouped GEMM walk. Histogram of the T*K pairs in shared memory, block scans, then
 // every pair takes the next free place of its expert (an atomic cursor: the order of an expert's pairs is not the token
-// order and may change from run to run - every pair's result is independent of its place). List 1 keeps sub-items of more
-// than maxp / 2 pairs first (nsub[1] = their number); list 2 is in expert order. The shared expert (slot_table[E], when
+// order and may change from run to run - every pair's result is independent of its place). Sub-items of more than maxp / 2
+// pairs come first (nsub[1] = their number). The shared expert (slot_table[E], when
 // gate_logits is given) gets the tokens [sh0, sh1) with weight sigmoid(gate logit), as the last item.
 // EP: the ids and weights of the tokens outside [sh0, sh1) were stored by other GPUs (ep.cuh): the block first waits (bounded)
 // until every such token's dispatch flag ep_flags[t] has reached *ep_step * EP_PHASES + ep_phase, and the lists are then read
@@ -503,7 +502,6 @@ __global__ void __launch_bounds__(1024) group_plan1_k(const int* __restrict__ id
                                                       const uint8_t* const* __restrict__ slot_table, moexb_pair_item* __restrict__ items,
                                                       moexb_pair* __restrict__ pairs, int* __restrict__ nitems,
                                                       moexb_pair_item* __restrict__ subs, int* __restrict__ nsub, int maxp,
-                                                      moexb_pair_item* __restrict__ subs2, int* __restrict__ nsub2, int maxp2,
                                                       const float* __restrict__ gate_logits, int gl_stride, int sh0, int sh1,
                                                       int stage_pairs, const unsigned* ep_flags = nullptr, const unsigned* ep_step = nullptr,
                                                       unsigned ep_phase = 0, int ep_world = 0, int ep_rank = 0, int* err = nullptr) {
@@ -550,10 +548,9 @@ __global__ void __launch_bounds__(1024) group_plan1_k(const int* __restrict__ id
     const int c = slot ? cnt[e] : 0;   // pairs of experts that are not held here are dropped
     auto wide = [](int c, int mp) { return c / mp + (c % mp > mp / 2); };
     auto narrow = [](int c, int mp) { return (int)(c % mp > 0 && c % mp <= mp / 2); };
-    int np, ni, nw, nn, n2 = 0;
+    int np, ni, nw, nn;
     const int at = block_scan_1024(c, np), item = block_scan_1024(c != 0, ni);
     const int wat = block_scan_1024(wide(c, maxp), nw), nat = block_scan_1024(narrow(c, maxp), nn);
-    const int at2 = subs2 ? block_scan_1024((c + maxp2 - 1) / maxp2, n2) : 0;
     start[e] = slot ? at : -1;
     const bool staged = stage_pairs >= n;
     const int all_wide = nw + wide(Ts, maxp);   // the routed experts' wide sub-items, then the shared expert's
@@ -561,7 +558,6 @@ __global__ void __launch_bounds__(1024) group_plan1_k(const int* __restrict__ id
         items[item] = {slot, at, c};
         const int cw = wide(c, maxp);
         for (int j = 0; j * maxp < c; j++) subs[j < cw ? wat + j : all_wide + nat] = {slot, at + j * maxp, min(maxp, c - j * maxp)};
-        if (subs2) for (int j = 0; j * maxp2 < c; j++) subs2[at2 + j] = {slot, at + j * maxp2, min(maxp2, c - j * maxp2)};
     }
     __syncthreads();
     auto place = [&](int p, int ex, float wp) {
@@ -593,15 +589,12 @@ __global__ void __launch_bounds__(1024) group_plan1_k(const int* __restrict__ id
             pairs[np + t] = {sh0 + t, n + sh0 + t, 1.f / (1.f + expf(-gl))};
         }
         for (int j = e; j * maxp < Ts; j += 1024) subs[j < cw ? nw + j : ns] = {sslot, np + j * maxp, min(maxp, Ts - j * maxp)};
-        if (subs2) for (int j = e; j * maxp2 < Ts; j += 1024) subs2[n2 + j] = {sslot, np + j * maxp2, min(maxp2, Ts - j * maxp2)};
         if (e == 0) {
             items[ni] = {sslot, np, Ts}; *nitems = ni + 1;
             nsub[0] = ns + narrow(Ts, maxp); nsub[1] = all_wide;
-            if (subs2) *nsub2 = n2 + (Ts + maxp2 - 1) / maxp2;
         }
     } else if (e == 0) {
         *nitems = ni; nsub[0] = all_wide + nn; nsub[1] = all_wide;
-        if (subs2) *nsub2 = n2;
     }
 }
 

@@ -1,0 +1,39 @@
+"""The tcgen05 grouped GEMM at the sizes where it can go wrong, against the oracle: every format, one and two activation rows per
+token, one token, tiles of one column more or less than a block of 16 and than a full tile (the shared expert's tiles hold T
+tokens), several tiles per expert. Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+import moe_b200 as m
+from oracle import oracle as o
+from parity import check_ffn
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("lib_built")]
+DEV, E, K = "cuda:0", 32, 8
+
+
+@pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_SYM_F32, m.FMT_ZP])
+@pytest.mark.parametrize("block", [False, True])
+def test_grouped_gemm_edges(fmt, block):
+    c = m.Context(0, max_tokens=300, max_experts=E, top_k=K)
+    c.set_prefill_min_tokens(1)
+    L = m.Layer(c, fmt, E)
+    L.fill_synth(3, 0)
+    rng = np.random.default_rng(5)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    host = [m.synth_expert_host(fmt, 3, 0, e) for e in range(E + 1)]
+    try:
+        for T in (1, 15, 17, 48, 49, 80, 81, 300):
+            X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32))
+            for x in (X, X.to(torch.bfloat16)):
+                idx = torch.empty(T, K, dtype=torch.int32, device=DEV)
+                xf = x.float().numpy()
+                got = L.forward(x.to(DEV), T, K, idx=idx, flags=2 if block else 0).cpu().numpy()
+                assert c.status() == 0
+                ref, ri, _, _ = o.layer_forward(fmt, host, W, o.rmsnorm(xf) if block else xf, K)
+                assert np.array_equal(idx.cpu().numpy(), ri)
+                check_ffn(got, xf + ref if block else ref, fmt, f"grouped GEMM T={T} {x.dtype} block={block}")
+    finally:
+        L.close(); c.close()
