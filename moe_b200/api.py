@@ -13,17 +13,22 @@ from . import _lib
 from ._lib import EH, EI, F32, BF16, F16, check, lib
 
 
+_ITEM_BYTES, _PAIR_BYTES = C.sizeof(_lib.PairItem), C.sizeof(_lib.Pair)
+
+
 def _ptr(t):
     if t is None:
         return None
     if isinstance(t, torch.Tensor):
-        assert t.is_cuda and t.is_contiguous(), "device-resident contiguous tensor expected"
-        return t.data_ptr()
+        if t.is_cuda and t.is_contiguous():
+            return t.data_ptr()
+        raise AssertionError("device-resident contiguous tensor expected")
     return int(t)
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle of the current stream of the current device, without building a Stream object on every call
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def expert_bytes(fmt):
@@ -94,13 +99,12 @@ def shared_expert_add(fmt, blob, gl, gl_stride, X, T, out, scratch=None):
 def group_pairs(idx, w, T, K, E, slot_table):
     """Device pair grouping; returns (items uint8 [E*16], pairs uint8 [T*K*12], nitems int32 [1])."""
     dev = idx.device
-    items = torch.zeros(E * C.sizeof(_lib.PairItem), device=dev, dtype=torch.uint8)
-    pairs = torch.zeros(T * K * C.sizeof(_lib.Pair), device=dev, dtype=torch.uint8)
-    nitems = torch.zeros(1, device=dev, dtype=torch.int32)
-    counts = torch.zeros(E, device=dev, dtype=torch.int32)
-    check(lib().moexb_group_pairs(_ptr(idx), _ptr(w), T, K, E, _ptr(slot_table), _ptr(items), _ptr(pairs), _ptr(nitems),
-                                  _ptr(counts), _stream()))
-    return items, pairs, nitems
+    items = torch.empty(E * _ITEM_BYTES, device=dev, dtype=torch.uint8)
+    pairs = torch.empty(T * K * _PAIR_BYTES, device=dev, dtype=torch.uint8)
+    counts = torch.empty(1 + E, device=dev, dtype=torch.int32)   # the number of items, then scratch
+    p = counts.data_ptr()
+    check(lib().moexb_group_pairs(_ptr(idx), _ptr(w), T, K, E, _ptr(slot_table), items.data_ptr(), pairs.data_ptr(), p, p + 4, _stream()))
+    return items, pairs, counts[:1]
 
 
 def dequant(fmt, blob):

@@ -142,10 +142,13 @@ __global__ void __launch_bounds__(WARPS * 32) pairs_down_k(const moexb_pair_item
 // extra term is the CPU experts' share; here it also carries the shared expert's rows).
 __global__ void pairs_reduce_k(const float* __restrict__ ypair, const float* __restrict__ extra, float* __restrict__ moe, int K, int D,
                                const int* __restrict__ use_extra) {
+    pdl_wait();
+    pdl_trigger();
     if (use_extra && !*use_extra) extra = nullptr;
     const int t = blockIdx.y, d = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (d >= D) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
     for (int r = 0; r < K; r++) {
         const float4 v = *reinterpret_cast<const float4*>(ypair + ((size_t)t * K + r) * D + d);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
@@ -163,11 +166,64 @@ __global__ void gated_add_rows_k(float* __restrict__ out, const float* __restric
     if (d < D) out[(size_t)t * D + d] += sh[(size_t)t * D + d] / (1.f + expf(-gl[(size_t)t * gl_stride]));
 }
 
-// One item over all T tokens with weight 1 and p = t: the work list of an expert applied to every token.
-__global__ void identity_pairs_k(const uint8_t* blob, int T, moexb_pair_item* item, moexb_pair* pairs) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) *item = {blob, 0, T};
-    if (t < T) pairs[t] = {t, t, 1.f};
+// The shared expert, one blob for every token, in the arithmetic of pairs_gate_up_k / pairs_down_k. A block takes SH_T tokens, whose
+// rows it stages together (16 tokens: 8 + 10 us; walked one after the other by the blocks of pairs_gate_up_k / pairs_down_k 27 + 21).
+constexpr int SH_T = 4;
+template <int FMT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) shared_gate_up_k(const uint8_t* __restrict__ blob, const float* __restrict__ X, float* __restrict__ act, int T) {
+    __shared__ __align__(16) float xs[SH_T][pad32_size(EH)];
+    const int t0 = blockIdx.y * SH_T;
+    const int row = blockIdx.x * WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_wait();
+    pdl_trigger();
+    uint4 qg[2], qu[2]; float2 sg[2], su[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int c = lane + 32 * i;
+        qg[i] = __ldg(reinterpret_cast<const uint4*>(blob + (size_t)row * (EH / 2)) + c);
+        qu[i] = __ldg(reinterpret_cast<const uint4*>(blob + (size_t)(EI + row) * (EH / 2)) + c);
+        sg[i] = chunk_scale<FMT>(blob, (size_t)row * (EH / 32) + c);
+        su[i] = chunk_scale<FMT>(blob, (size_t)(EI + row) * (EH / 32) + c);
+    }
+#pragma unroll
+    for (int j = 0; j < SH_T; j++)   // (the last block may repeat a token)
+        for (int i = threadIdx.x * 4; i < EH; i += WARPS * 128) cp_async16(smem_u32(xs[j] + pad32(i)), X + (size_t)min(t0 + j, T - 1) * EH + i);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    float ag[SH_T] = {}, au[SH_T] = {};
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int c = lane + 32 * i;
+#pragma unroll
+        for (int j = 0; j < SH_T; j++) { ag[j] += dot32<FMT>(qg[i], xs[j] + 36 * c, sg[i]); au[j] += dot32<FMT>(qu[i], xs[j] + 36 * c, su[i]); }
+    }
+#pragma unroll
+    for (int j = 0; j < SH_T; j++) {
+        const float g = warp_sum(ag[j]), u = warp_sum(au[j]);
+        if (lane == j && t0 + j < T) act[(size_t)(t0 + j) * EI + row] = silu_mul(g, u);
+    }
+}
+// out[t][d] += (down[d] . act[t]) * sigmoid(gl[t * gl_stride])
+template <int FMT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) shared_down_k(const uint8_t* __restrict__ blob, const float* __restrict__ act, const float* __restrict__ gl, int gl_stride,
+                                                            float* __restrict__ out, int T) {
+    __shared__ __align__(16) float as[SH_T][pad32_size(EI)];
+    const int t0 = blockIdx.y * SH_T;
+    const int d = blockIdx.x * WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31, hf = lane >> 4, c = lane & 15;
+    pdl_wait();
+    pdl_trigger();
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(blob + DOWN_Q_OFF + (size_t)d * (EI / 2)) + c);
+    const float2 sm = chunk_scale<FMT>(blob, DOWN_C_OFF + (size_t)d * (EI / 32) + c);
+    for (int i = threadIdx.x * 4; i < SH_T * EI; i += WARPS * 128)
+        cp_async16(smem_u32(as[i / EI] + pad32(i % EI)), act + (size_t)min(t0 + i / EI, T - 1) * EI + i % EI);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int j0 = 0; j0 < SH_T; j0 += 2) {
+        const int j = j0 + hf;
+        const float v = half_warp_sum(dot32<FMT>(q, as[j] + 36 * c, sm));
+        if (c == 0 && t0 + j < T) out[(size_t)(t0 + j) * EH + d] += v / (1.f + expf(-gl[(size_t)(t0 + j) * gl_stride]));
+    }
 }
 
 // ---- glue of the layer-level calls ------------------------------------------------------------------------------------

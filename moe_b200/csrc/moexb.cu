@@ -197,8 +197,10 @@ template <typename WT>
 static int gemv_any(const WT* W, const float* x, float* y, int I, int O, void* stream, int rows) {
     REQUIRE(W && x && y, "gemv: null pointer");
     REQUIRE(I > 0 && I % 128 == 0 && O > 0 && rows > 0, "gemv: I=%d must be a positive multiple of 128, O=%d, rows=%d", I, O, rows);
-    if (rows >= 8) {
-        constexpr int WARPS = 4, TO = 4, TR = 8;  // 16 outputs x 8 rows per block: 17 x 8 blocks for the 64-token router
+    // A warp per (row, output) re-reads the weights from L2 for every row, which up to 24 rows costs less than the tiles of the batched
+    // kernel, of which a small batch has too few to reach every SM (16 rows: 3 us against 19).
+    if (rows > 24) {
+        constexpr int WARPS = 8, TO = 2, TR = 8;  // 16 outputs x 8 rows per block: 17 x 8 blocks for the 64-token router
         const int smem = TR * I * (int)sizeof(float);
         REQUIRE(smem <= 200 * 1024, "gemv: I=%d is too large for the batched kernel", I);
         static PerDeviceOnce once;
@@ -263,7 +265,7 @@ static int decode_launch(moexb_ctx* prof, int fmt, const uint8_t* const* slots, 
 static std::mutex g_default_lock;
 static moexb_ctx* g_default_ctx[MAX_DEVICES] = {};
 static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, void* stream);
-static int split_launch(moexb_ctx* c, const float* x, int rows, bool f16, void* stream);
+static int split_launch(moexb_ctx* c, const float* x, int rows, bool f16, void* stream, const SidePlan* plan = nullptr);
 
 extern "C" {
 
@@ -289,14 +291,14 @@ int moexb_experts_forward(int fmt, const uint8_t* const* slots, const float* w, 
     REQUIRE(K > 0 && K <= 16, "experts_forward: K=%d out of range 1..16", K);
     REQUIRE(fmt_ok(fmt), "experts_forward: unknown expert format %d", fmt);
     cudaStream_t st = S(stream);
-    plan_decode_k<<<1, 32, 0, st>>>(slots, w, K, nh, c->subs, c->pairs, c->nsub);
-    LAUNCHED("plan_decode");
-    int rc = split_launch(c, x, 1, false, stream);
+    SidePlan plan{};
+    plan.slots = slots; plan.w = w; plan.K = K; plan.nh = nh; plan.subs = c->subs; plan.pairs = c->pairs; plan.nsub = c->nsub;
+    int rc = split_launch(c, x, 1, false, stream, &plan);
     if (rc != MOEXB_OK) return rc;
     if (nh) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)K * EH * sizeof(float), st));   // rows of the experts beyond *nh stay zero
     rc = stream_experts(c, fmt, c->pairs, act, c->ypair, stream);
     if (rc != MOEXB_OK) return rc;
-    pairs_reduce_k<<<dim3((EH / 4 + 255) / 256, 1), 256, 0, st>>>(c->ypair, nullptr, out, K, EH, nullptr);
+    CUDA_TRY(launch_dep(pairs_reduce_k, dim3((EH / 4 + 255) / 256, 1), 256, 0, st, (const float*)c->ypair, (const float*)nullptr, out, K, EH, (const int*)nullptr));
     LAUNCHED("pairs_reduce");
     return MOEXB_OK;
 }
@@ -332,7 +334,7 @@ int moexb_pairs_forward_dev(int fmt, const moexb_pair_item* items, const int* ni
 int moexb_pairs_reduce(const float* ypair, const float* ycpu, float* moe, int K, int D, int T, const int* use_cpu, void* stream) {
     REQUIRE(ypair && moe, "pairs_reduce: null pointer");
     REQUIRE(K > 0 && D > 0 && D % 4 == 0 && T > 0 && T <= 65535, "pairs_reduce: K=%d D=%d T=%d", K, D, T);
-    pairs_reduce_k<<<dim3((D / 4 + 255) / 256, T), 256, 0, S(stream)>>>(ypair, ycpu, moe, K, D, use_cpu);
+    CUDA_TRY(launch_dep(pairs_reduce_k, dim3((D / 4 + 255) / 256, T), 256, 0, S(stream), ypair, ycpu, moe, K, D, use_cpu));
     LAUNCHED("pairs_reduce");
     return MOEXB_OK;
 }
@@ -349,11 +351,8 @@ int moexb_group_pairs(const int* idx, const float* w, int T, int K, int E, const
                       moexb_pair_item* items, moexb_pair* pairs, int* nitems, int* counts, void* stream) {
     REQUIRE(idx && w && slot_table && items && pairs && nitems && counts, "group_pairs: null pointer");
     REQUIRE(T > 0 && K > 0 && E > 0 && E <= 1024, "group_pairs: T=%d K=%d E=%d", T, K, E);
-    constexpr int WARPS = 8;
-    group_count_k<WARPS><<<(E + WARPS - 1) / WARPS, WARPS * 32, 0, S(stream)>>>(idx, T * K, E, counts);
-    LAUNCHED("group_count");
-    group_scatter_k<WARPS><<<(E + WARPS - 1) / WARPS, WARPS * 32, 0, S(stream)>>>(idx, w, T, K, E, slot_table, counts, items, pairs, nitems, nullptr, 0);
-    LAUNCHED("group_scatter");
+    CUDA_TRY(launch_dep(group_pairs_k, 1, 1024, 0, S(stream), idx, w, T, K, E, slot_table, items, pairs, nitems));
+    LAUNCHED("group_pairs");
     return MOEXB_OK;
 }
 
@@ -361,18 +360,16 @@ int moexb_shared_expert_add(int fmt, const uint8_t* blob, const float* gl, int g
                             float* out, float* scratch, void* stream) {
     REQUIRE(blob && gl && X && out && scratch, "shared_expert_add: null pointer");
     REQUIRE(T > 0 && T <= 65535, "shared_expert_add: T=%d", T);
-    // The shared expert is one item holding every token with weight 1; the gate enters in gated_add_rows.
-    // scratch: act [T][I], sh [T][H], then the item and its T pairs.
-    float *act = scratch, *sh = scratch + (size_t)T * EI;
-    moexb_pair_item* item = reinterpret_cast<moexb_pair_item*>(sh + (size_t)T * EH);
-    moexb_pair* pairs = reinterpret_cast<moexb_pair*>(item + 1);
-    identity_pairs_k<<<(T + 255) / 256, 256, 0, S(stream)>>>(blob, T, item, pairs);
-    LAUNCHED("identity_pairs");
-    int rc = pairs_launch(nullptr, fmt, item, nullptr, 1, pairs, X, act, sh, stream);
-    if (rc != MOEXB_OK) return rc;
-    gated_add_rows_k<<<dim3((EH + 255) / 256, T), 256, 0, S(stream)>>>(out, sh, gl, gl_stride, EH);
-    LAUNCHED("gated_add_rows");
-    return MOEXB_OK;
+    // scratch: act [T][I]
+    return by_fmt(fmt, [&]<int FMT>() {
+        constexpr int WARPS = 8;
+        const unsigned ty = (unsigned)((T + SH_T - 1) / SH_T);
+        CUDA_TRY(launch_dep(shared_gate_up_k<FMT, WARPS>, dim3(EI / WARPS, ty), WARPS * 32, 0, S(stream), blob, X, scratch, T));
+        LAUNCHED("shared_gate_up");
+        CUDA_TRY(launch_dep(shared_down_k<FMT, WARPS>, dim3(EH / WARPS, ty), WARPS * 32, 0, S(stream), blob, (const float*)scratch, gl, gl_stride, out, T));
+        LAUNCHED("shared_down");
+        return (int)MOEXB_OK;
+    });
 }
 
 // ---- formats ---------------------------------------------------------------------------------------------------------
@@ -963,13 +960,15 @@ int moexb_layer_load_st(moexb_layer* L, const moexb_st* s, const char* prefix, i
 
 template <int FMT, bool DOWN>
 static int stream_launch_one(moexb_ctx* c, const StreamArgs& a, void* stream) {
-    constexpr int NW = 4, STAGES = FMT == FMT_SYM_F16 ? 4 : 3;
+    // three CTAs per SM: the 12 consumer warps, not the ring's depth, are what the loop is short of with two
+    constexpr int NW = 4, CPS = 3, STAGES = DOWN ? 3 : 2;
     constexpr int SMEM = st_smem_bytes<FMT, DOWN, NW, STAGES>();
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(stream_k<FMT, DOWN, NW, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "stream kernel shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
-    stream_k<FMT, DOWN, NW, STAGES><<<2 * c->sms, (NW + 1) * 32, SMEM, S(stream)>>>(a);
+    static_assert(SMEM * CPS <= 227 * 1024, "shared memory of the resident CTAs");
+    CUDA_TRY(launch_dep(stream_k<FMT, DOWN, NW, STAGES>, CPS * c->sms, (NW + ST_NP) * 32, SMEM, S(stream), a));
     LAUNCHED(DOWN ? "stream_down" : "stream_gate_up");
     return MOEXB_OK;
 }
@@ -1082,12 +1081,11 @@ static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int p
     });
 }
 
-// f16: the consumer is the tiled kernel of a symmetric format (fp16 operands); otherwise bf16
-static int split_launch(moexb_ctx* c, const float* x, int rows, bool f16, void* stream) {
+// f16: the consumer is the tiled kernel of a symmetric format (fp16 operands); otherwise bf16. plan: made on the side by one more block.
+static int split_launch(moexb_ctx* c, const float* x, int rows, bool f16, void* stream, const SidePlan* plan) {
     PROF(c, MOEXB_PROF_OTHER, stream);
-    const size_t n = (size_t)rows * EH;
-    if (f16) split_rows_k<true><<<(unsigned)((n + 255) / 256), 256, 0, S(stream)>>>(x, c->xs, EH, n);
-    else split_rows_k<false><<<(unsigned)((n + 255) / 256), 256, 0, S(stream)>>>(x, c->xs, EH, n);
+    const SidePlan p = plan ? *plan : SidePlan{};
+    CUDA_TRY(launch_dep(f16 ? split_rows_k<true> : split_rows_k<false>, rows + (plan ? 1 : 0), 256, 0, S(stream), x, c->xs, rows, p));
     LAUNCHED("split_rows");
     return MOEXB_OK;
 }
@@ -1100,10 +1098,10 @@ extern "C" int moexb_pairs_forward_tc(moexb_ctx* c, int fmt, const moexb_pair_it
     REQUIRE(npairs > 0 && npairs <= c->max_tokens * (c->top_k + 1), "pairs_forward_tc: npairs=%d exceeds the context's capacity %d", npairs, c->max_tokens * (c->top_k + 1));
     REQUIRE(n_items >= 0 && n_items <= c->max_experts + 1, "pairs_forward_tc: n_items=%d exceeds the context's capacity %d", n_items, c->max_experts + 1);
     if (n_items == 0) return MOEXB_OK;
-    int rc = split_launch(c, X, T, false, stream);
+    SidePlan plan{};
+    plan.items = items; plan.n_items = n_items; plan.maxp = ST_MAXP; plan.subs = c->subs; plan.nsub = c->nsub;
+    int rc = split_launch(c, X, T, false, stream, &plan);
     if (rc != MOEXB_OK) return rc;
-    plan_subitems_k<<<1, 1024, 0, S(stream)>>>(items, nullptr, n_items, c->subs, c->nsub, ST_MAXP);
-    LAUNCHED("plan_subitems");
     return stream_experts(c, fmt, pairs, act, ypair, stream);
 }
 
@@ -1706,8 +1704,8 @@ int moexb_ep_dispatch(moexb_ep* e, moexb_layer* L, int l, const void* X, int x_d
             rmsnorm_rows_k<<<n_own, 256, 0, st>>>(e->x, xn_own, EH, 1e-6f);
             LAUNCHED("rmsnorm_rows");
         } else if (!prefill) {
-            if (f16) split_rows_k<true><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * 2 * EH, EH, n);
-            else split_rows_k<false><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * 2 * EH, EH, n);
+            if (f16) split_rows_k<true><<<n_own, 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * 2 * EH, n_own, SidePlan{});
+            else split_rows_k<false><<<n_own, 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * 2 * EH, n_own, SidePlan{});
             LAUNCHED("split_rows");
         }
     } else {

@@ -53,58 +53,81 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_rows_k(const WT* __restrict__
     if (lane == 0) y[(size_t)blockIdx.y * O + o] = acc;
 }
 
-// The same result for many rows (a batch or a prefill chunk). A block stages TR activation rows in shared memory and its
-// WARPS warps each own TO outputs; a lane still holds elements 128c+4j..4j+3 of every dot product, so every
-// (row, output) sum is formed in exactly the order of gemv_rows_k and the two kernels agree bit for bit.
-// grid (ceil(O / (WARPS*TO)), ceil(rows / TR)); dynamic shared memory TR * I floats.
-template <typename WT, int WARPS, int TO, int TR>
-__global__ void __launch_bounds__(WARPS * 32) gemm_rows_k(const WT* __restrict__ W, const float* __restrict__ x,
-                                                          float* __restrict__ y, int I, int O, int rows) {
+// One tile of the batched rows: a block stages TR activation rows in shared memory and its WARPS warps each own TO outputs, with the
+// weights of U steps requested at a time and the next U already in flight; a lane still holds elements 128c+4j..4j+3 of every dot
+// product, so every (row, output) sum is formed in exactly the order of gemv_rows_k and the kernels agree bit for bit.
+// Waits for the kernel before (pdl_wait); EARLY: only once its first weights, which that kernel must not write, are requested. Dynamic shared memory TR * I floats.
+template <typename WT, int WARPS, int TO, int TR, bool EARLY>
+__device__ __forceinline__ void gemm_tile(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int I, int O, int rows) {
     extern __shared__ __align__(16) float xsm[];  // [TR][I]
-    const int r0 = blockIdx.y * TR, lane = threadIdx.x & 31;
+    // steps per batch of weights: the small tile takes 8 (half of I = 2048) - the first batch, requested before the wait,
+    // arrives while the kernel before this one still runs (all 16 at once would spill)
+    constexpr int U = TO <= 2 ? 8 : 4;
+    const int r0 = blockIdx.y * TR, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int o0 = (blockIdx.x * WARPS + warp) * TO;
+    const WT* wr[TO];
+#pragma unroll
+    for (int i = 0; i < TO; i++) wr[i] = W + (size_t)min(o0 + i, O - 1) * I;
+    float4 wn[TO][U];  // the weights of the next U steps
+    auto load_w = [&](int c0) {
+#pragma unroll
+        for (int i = 0; i < TO; i++)
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (c0 + u < I / 128) wn[i][u] = ld_w4(wr[i], (size_t)128 * (c0 + u) + 4 * lane);
+    };
+    if (EARLY) load_w(0);
     pdl_wait();
     pdl_trigger();
-    for (int i = threadIdx.x * 4; i < TR * I; i += WARPS * 128) {
-        const int r = min(r0 + i / I, rows - 1);
-        *reinterpret_cast<float4*>(xsm + i) = __ldg(reinterpret_cast<const float4*>(x + (size_t)r * I + i % I));
+    if (!EARLY) load_w(0);
+    for (int r = 0; r < TR; r++) {   // the tile's token rows: 16-byte asynchronous copies, all in flight at once
+        const float* src = x + (size_t)min(r0 + r, rows - 1) * I;
+        for (int c = threadIdx.x * 4; c < I; c += WARPS * 128) cp_async16(smem_u32(xsm + r * I + c), src + c);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int o0 = (blockIdx.x * WARPS + (threadIdx.x >> 5)) * TO;
-    if (o0 >= O) return;
     float acc[TR][TO];
 #pragma unroll
     for (int r = 0; r < TR; r++)
 #pragma unroll
-        for (int o = 0; o < TO; o++) acc[r][o] = 0.f;
-    float4 wn[TO];  // the next step's weights are loaded while this step's products run
+        for (int i = 0; i < TO; i++) acc[r][i] = 0.f;
+    for (int c0 = 0; c0 < I / 128; c0 += U) {
+        float4 w[TO][U];
 #pragma unroll
-    for (int o = 0; o < TO; o++) wn[o] = ld_w4(W + (size_t)min(o0 + o, O - 1) * I, (size_t)4 * lane);
-    for (int c = 0; c < I / 128; c++) {
-        float4 w[TO];
+        for (int i = 0; i < TO; i++)
 #pragma unroll
-        for (int o = 0; o < TO; o++) w[o] = wn[o];
-        if (c + 1 < I / 128) {
+            for (int u = 0; u < U; u++) w[i][u] = wn[i][u];
+        if (c0 + U < I / 128) load_w(c0 + U);
 #pragma unroll
-            for (int o = 0; o < TO; o++) wn[o] = ld_w4(W + (size_t)min(o0 + o, O - 1) * I, (size_t)128 * (c + 1) + 4 * lane);
-        }
+        for (int u = 0; u < U; u++) {
+            if (c0 + u >= I / 128) break;
 #pragma unroll
-        for (int r = 0; r < TR; r++) {
-            const float4 v = *reinterpret_cast<const float4*>(xsm + r * I + 128 * c + 4 * lane);
+            for (int r = 0; r < TR; r++) {
+                const float4 v = *reinterpret_cast<const float4*>(xsm + r * I + 128 * (c0 + u) + 4 * lane);
 #pragma unroll
-            for (int o = 0; o < TO; o++) {
-                float a = acc[r][o];
-                a = fmaf(w[o].x, v.x, a); a = fmaf(w[o].y, v.y, a); a = fmaf(w[o].z, v.z, a); a = fmaf(w[o].w, v.w, a);
-                acc[r][o] = a;
+                for (int i = 0; i < TO; i++) {
+                    float a = acc[r][i];
+                    a = fmaf(w[i][u].x, v.x, a); a = fmaf(w[i][u].y, v.y, a); a = fmaf(w[i][u].z, v.z, a); a = fmaf(w[i][u].w, v.w, a);
+                    acc[r][i] = a;
+                }
             }
         }
     }
 #pragma unroll
     for (int r = 0; r < TR; r++)
 #pragma unroll
-        for (int o = 0; o < TO; o++) {
-            const float sum = warp_sum(acc[r][o]);
-            if (lane == 0 && r0 + r < rows && o0 + o < O) y[(size_t)(r0 + r) * O + o0 + o] = sum;
+        for (int i = 0; i < TO; i++) {
+            const float sum = warp_sum(acc[r][i]);
+            if (lane == 0 && r0 + r < rows && o0 + i < O) y[(size_t)(r0 + r) * O + o0 + i] = sum;
         }
+}
+
+// The same result for many rows (a batch or a prefill chunk).
+// grid (ceil(O / (WARPS*TO)), ceil(rows / TR)); dynamic shared memory TR * I floats.
+template <typename WT, int WARPS, int TO, int TR>
+__global__ void __launch_bounds__(WARPS * 32) gemm_rows_k(const WT* __restrict__ W, const float* __restrict__ x,
+                                                          float* __restrict__ y, int I, int O, int rows) {
+    gemm_tile<WT, WARPS, TO, TR, false>(W, x, y, I, O, rows);
 }
 
 // Softmax over E logits and the K largest by one warp (kernels.cuh:373-406 does it with a block per token).
@@ -312,74 +335,15 @@ __global__ void __launch_bounds__(WARPS * 32) route_gemv_k(const WT* __restrict_
     ep_raise_dispatch_flags(o, t, 1);
 }
 
-// The same for a batch: gemm_rows_k's tiling (a block stages TR token rows in shared memory, each of its WARPS warps owns
-// TO outputs, every dot product in gemv_rows_k's summation order) with the weights of U steps requested at a time and
-// the next U already in flight; the last block of a token tile to finish selects the experts of its TR tokens (warp r
-// takes tokens r, r + WARPS, ..). grid (ceil((E + 1) / (WARPS * TO)), ceil(T / TR)); dynamic shared memory TR * I floats;
+// The same for a batch in gemm_tile's tiles; the last block of a token tile to finish selects the experts of its TR tokens (warp r
+// takes tokens r, r + WARPS, ..).
+// grid (ceil((E + 1) / (WARPS * TO)), ceil(T / TR)); dynamic shared memory TR * I floats;
 // done[tile] zero before the first launch.
 template <typename WT, int WARPS, int TO, int TR, int NJ>
 __global__ void __launch_bounds__(WARPS * 32) route_gemm_k(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int I,
                                                            int E, int K, int norm, int T, int* __restrict__ done, const TopkOut o) {
-    extern __shared__ __align__(16) float xsm[];  // [TR][I]
-    // steps per batch of weights: the small tile takes 8 (half of I = 2048) - the first batch, requested before the wait,
-    // arrives while the kernel before this one still runs (all 16 at once would spill)
-    constexpr int U = TO <= 2 ? 8 : 4;
     const int O = E + 1, r0 = blockIdx.y * TR, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int o0 = (blockIdx.x * WARPS + warp) * TO;
-    const WT* wr[TO];
-#pragma unroll
-    for (int i = 0; i < TO; i++) wr[i] = W + (size_t)min(o0 + i, O - 1) * I;
-    float4 wn[TO][U];  // the weights of the next U steps
-    auto load_w = [&](int c0) {
-#pragma unroll
-        for (int i = 0; i < TO; i++)
-#pragma unroll
-            for (int u = 0; u < U; u++)
-                if (c0 + u < I / 128) wn[i][u] = ld_w4(wr[i], (size_t)128 * (c0 + u) + 4 * lane);
-    };
-    load_w(0);  // weights do not depend on the kernel before this one
-    pdl_wait();
-    pdl_trigger();
-    for (int r = 0; r < TR; r++) {   // the tile's token rows: 16-byte asynchronous copies, all in flight at once
-        const float* src = x + (size_t)min(r0 + r, T - 1) * I;
-        for (int c = threadIdx.x * 4; c < I; c += WARPS * 128) cp_async16(smem_u32(xsm + r * I + c), src + c);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    float acc[TR][TO];
-#pragma unroll
-    for (int r = 0; r < TR; r++)
-#pragma unroll
-        for (int i = 0; i < TO; i++) acc[r][i] = 0.f;
-    for (int c0 = 0; c0 < I / 128; c0 += U) {
-        float4 w[TO][U];
-#pragma unroll
-        for (int i = 0; i < TO; i++)
-#pragma unroll
-            for (int u = 0; u < U; u++) w[i][u] = wn[i][u];
-        if (c0 + U < I / 128) load_w(c0 + U);
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (c0 + u >= I / 128) break;
-#pragma unroll
-            for (int r = 0; r < TR; r++) {
-                const float4 v = *reinterpret_cast<const float4*>(xsm + r * I + 128 * (c0 + u) + 4 * lane);
-#pragma unroll
-                for (int i = 0; i < TO; i++) {
-                    float a = acc[r][i];
-                    a = fmaf(w[i][u].x, v.x, a); a = fmaf(w[i][u].y, v.y, a); a = fmaf(w[i][u].z, v.z, a); a = fmaf(w[i][u].w, v.w, a);
-                    acc[r][i] = a;
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < TR; r++)
-#pragma unroll
-        for (int i = 0; i < TO; i++) {
-            const float sum = warp_sum(acc[r][i]);
-            if (lane == 0 && r0 + r < T && o0 + i < O) y[(size_t)(r0 + r) * O + o0 + i] = sum;
-        }
+    gemm_tile<WT, WARPS, TO, TR, true>(W, x, y, I, O, T);
     if (!last_block_done(done + blockIdx.y, gridDim.x)) return;
     for (int r = warp; r < TR && r0 + r < T; r += WARPS) topk_token<NJ, true>(y + (size_t)(r0 + r) * O, r0 + r, E, K, norm, lane, o);
     ep_raise_dispatch_flags(o, r0, min(TR, T - r0));
@@ -469,63 +433,6 @@ __global__ void __launch_bounds__(256, 2) route_gemm2_k(const WT* __restrict__ W
     if (!last_block_done(done + blockIdx.y, gridDim.x)) return;
     for (int r = warp; r < RG2_TM && r0 + r < T; r += 8) topk_token<NJ, true>(y + (size_t)(r0 + r) * O, r0 + r, E, K, norm, lane, o);
     ep_raise_dispatch_flags(o, r0, min(RG2_TM, T - r0));
-}
-
-// ---- pair grouping: bucket the T*K (token, rank) pairs by expert (moex.cu:1466-1486; kernels.cuh:1030-1045) ----------
-
-// counts[e] = number of pairs that selected expert e. One warp per expert.
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) group_count_k(const int* __restrict__ idx, int n, int E, int* __restrict__ counts) {
-    const int e = blockIdx.x * WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (e >= E) return;
-    int c = 0;
-    for (int p = lane; p < n; p += 32) c += __ldg(idx + p) == e;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane == 0) counts[e] = c;
-}
-
-// Items in ascending expert id over the experts that are held (slot_table[e] != null) and selected; the pairs of an
-// expert in token order, p = t*K + rank. Every block rebuilds the (tiny) exclusive scan over experts, then one warp per
-// expert walks the pair list once and writes its matches in order. Optional shared expert: one more item holding every
-// token, p = T*K + t, w = sigmoid(gate logit of t). E <= 1024.
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) group_scatter_k(const int* __restrict__ idx, const float* __restrict__ w, int T, int K, int E,
-                                                              const uint8_t* const* __restrict__ slot_table, const int* __restrict__ counts,
-                                                              moexb_pair_item* __restrict__ items, moexb_pair* __restrict__ pairs,
-                                                              int* __restrict__ nitems, const float* __restrict__ gate_logits, int gl_stride) {
-    __shared__ int start[1024], item_of[1024];
-    __shared__ int s_ni, s_np;
-    if (threadIdx.x == 0) {
-        int ni = 0, np = 0;
-        for (int e = 0; e < E; e++) {
-            const int c = slot_table[e] ? counts[e] : 0;
-            start[e] = np; item_of[e] = c ? ni : -1;
-            np += c; ni += c != 0;
-        }
-        s_ni = ni; s_np = np;
-    }
-    __syncthreads();
-    const int n = T * K, lane = threadIdx.x & 31;
-    const int e = blockIdx.x * WARPS + (threadIdx.x >> 5);
-    if (e < E && item_of[e] >= 0) {
-        int at = start[e];
-        if (lane == 0) items[item_of[e]] = {slot_table[e], at, counts[e]};
-        for (int p0 = 0; p0 < n; p0 += 32) {
-            const int p = p0 + lane;
-            const bool hit = p < n && __ldg(idx + p) == e;
-            const unsigned b = __ballot_sync(0xffffffffu, hit);
-            if (hit) pairs[at + __popc(b & ((1u << lane) - 1))] = {p / K, p, __ldg(w + p)};
-            at += __popc(b);
-        }
-    }
-    if (blockIdx.x == 0) {
-        if (gate_logits && slot_table[E]) {
-            if (threadIdx.x == 0) { items[s_ni] = {slot_table[E], s_np, T}; *nitems = s_ni + 1; }
-            for (int t = threadIdx.x; t < T; t += blockDim.x)
-                pairs[s_np + t] = {t, n + t, 1.f / (1.f + expf(-gate_logits[(size_t)t * gl_stride]))};
-        } else if (threadIdx.x == 0) *nitems = s_ni;
-    }
 }
 
 }  // namespace moexb

@@ -1,10 +1,9 @@
 // Streaming expert kernels for 1..64 tokens: the bandwidth-bound skinny GEMM of the decode-size path.
 //
 // One kernel template serves both projections (gate/up with the SwiGLU epilogue, down with the routing-weight epilogue).
-// A persistent CTA has one producer warp and NW consumer warps. The producer pulls tiles from a global queue and streams
-// packed int4 rows through a ring of shared-memory stages with cp.async.bulk (the TMA bulk-copy engine), one 256-byte
-// row piece (512 weights = 8 scale groups) per copy, 64 pieces per stage, completion counted on an mbarrier; the scale
-// bytes of the same pieces follow with 16-byte cp.async copies on the same barrier. Consumer warps read 16 nibbles per
+// A persistent CTA has two producer warps and NW consumer warps. The producers stream packed int4 rows and their scale bytes
+// through a ring of shared-memory stages with 16-byte cp.async copies, 64 row pieces of 256 bytes (512 weights = 8 scale
+// groups) per stage, completion counted on an mbarrier. Consumer warps read 16 nibbles per
 // lane and row with 8-byte shared loads (the piece stride of 288 bytes keeps them conflict-free), turn them into exact
 // bf16 integers in registers (one lop3 + one bf16x2 subtract per two weights) and feed mma.sync.m16n8k16 with the
 // activations as the 8-wide operand. Activations arrive as bf16 hi + lo halves (16 significand bits) in adjacent
@@ -27,6 +26,7 @@ namespace moexb {
 constexpr int ST_PIECE = 256;    // bytes of one row piece: 512 int4 weights
 constexpr int ST_STRIDE = 288;   // piece stride in shared memory (rows g..g+3 of a half-warp land on distinct banks)
 constexpr int ST_SC_PER_PIECE = 48;  // zero point: 16 x [sc, mn] + 2 x (d, dm) = 40 scale bytes per piece, kept 16-byte aligned
+constexpr int ST_NP = 2;         // producer warps
 constexpr int ST_MAXP = 4;       // pairs per sub-item: 4 x (hi, lo) = the 8 columns of one MMA tile
 constexpr int ST_WAIT_LIMIT = 1 << 22;
 
@@ -155,7 +155,7 @@ struct StageInfo { int sub, tin, ks, first; };
 // DOWN = true : tile = 16*NW down rows, 1 stage (K = 512); ypair = w * (down . act).
 // CTA c of G works on tiles [c*U/G, (c+1)*U/G) of the U = nsub * TILES tiles, in order.
 template <int FMT, bool DOWN, int NW, int STAGES>
-__global__ void __launch_bounds__((NW + 1) * 32) stream_k(const StreamArgs a) {
+__global__ void __launch_bounds__((NW + ST_NP) * 32) stream_k(const StreamArgs a) {
     constexpr int PIECES = st_pieces<NW>();
     constexpr int SCB = st_scale_bytes<FMT>();
     constexpr int SLOT = st_slot_bytes<FMT, NW>();
@@ -170,44 +170,35 @@ __global__ void __launch_bounds__((NW + 1) * 32) stream_k(const StreamArgs a) {
     StageInfo* info = reinterpret_cast<StageInfo*>(bars + 2 * STAGES + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(smem_u32(bars + s), 33); mbar_init(smem_u32(bars + STAGES + s), NW); }
+        for (int s = 0; s < STAGES; s++) { mbar_init(smem_u32(bars + s), 32 * ST_NP + 1); mbar_init(smem_u32(bars + STAGES + s), NW); }
         mbar_init(smem_u32(bars + 2 * STAGES), NW);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    pdl_wait();
+    pdl_trigger();
     const long long U = (long long)*a.nsub * TILES;
     const int tile0 = (int)(U * blockIdx.x / gridDim.x), tile1 = (int)(U * (blockIdx.x + 1) / gridDim.x);
 
-    if (warp == NW) {
-        // ---- producer: one warp streams the tiles' row pieces and scale bytes into the ring ----
+    if (warp >= NW) {
+        // ---- producers: two warps bring the tiles' row pieces and scale bytes into the ring, half of a stage's pieces each, with
+        // 16-byte asynchronous copies (a row piece is 16 lanes of one instruction). As one bulk copy per 256-byte piece the stream
+        // was bound by the copies' issue: 1.9 TB/s ----
+        const int pw = warp - NW;
+        constexpr int PP = PIECES / ST_NP;
         int s = 0; uint32_t ph = 0;
-        uint32_t armed = 0, armed_ph = 0;   // per stage: a fill was requested, and the parity its full barrier completes with
-        // a wait ran out: wait (bounded) for the fills already requested, so that no copy is in flight into this CTA's
-        // shared memory when the producer leaves; the consumers run out of polls on their side
-        auto give_up = [&]() {
-            for (int i = 0; i < STAGES; i++)
-                if (armed >> i & 1) mbar_wait(smem_u32(bars + i), armed_ph >> i & 1, a.err, ST_ERR_EMPTY_WAIT);
-        };
         for (int tile = tile0; tile <= tile1; tile++) {
             const bool done = tile == tile1;  // one empty stage after the last tile tells the consumers to stop
             const int sub = done ? -1 : tile / TILES, tin = done ? 0 : tile % TILES;
             const uint8_t* slot = done ? nullptr : a.subs[sub].slot;
             for (int ks = 0; ks < (done ? 1 : KS); ks++) {
                 const uint32_t full = smem_u32(bars + s), empty = smem_u32(bars + STAGES + s);
-                if (!mbar_wait(empty, ph ^ 1, a.err, ST_ERR_EMPTY_WAIT)) { give_up(); return; }
-                armed |= 1u << s; armed_ph = (armed_ph & ~(1u << s)) | (ph << s);
-                if (lane == 0) {
-                    info[s] = {sub, tin, ks, ks == 0};
-                    mbar_arrive_expect_tx(full, done ? 0 : PIECES * ST_PIECE);
-                }
-                __syncwarp();
+                if (!mbar_wait(empty, ph ^ 1, a.err, ST_ERR_EMPTY_WAIT)) { asm volatile("cp.async.wait_all;" ::: "memory"); return; }
+                if (pw == 0 && lane == 0) { info[s] = {sub, tin, ks, ks == 0}; mbar_arrive(full); }
                 if (!done) {
                     const uint32_t base = smem_u32(smem + s * SLOT);
-#pragma unroll
-                    for (int i = 0; i < PIECES / 32; i++) {
-                        const int pi = lane + 32 * i;
-                        size_t c0;  // first 32-weight chunk of the piece inside the blob
-                        const uint8_t* src;
+                    // row and first 32-weight chunk of piece pi inside the blob
+                    auto piece = [&](int pi, const uint8_t*& src, size_t& c0) {
                         if (DOWN) {
                             const int d = tin * (16 * NW) + pi;
                             src = slot + DOWN_Q_OFF + (size_t)d * (EI / 2);
@@ -218,7 +209,18 @@ __global__ void __launch_bounds__((NW + 1) * 32) stream_k(const StreamArgs a) {
                             src = slot + row * (EH / 2) + ks * ST_PIECE;
                             c0 = row * (EH / 32) + ks * 16;
                         }
-                        bulk_g2s(base + pi * ST_STRIDE, src, ST_PIECE, full);
+                    };
+#pragma unroll 8
+                    for (int i = 0; i < PP / 2; i++) {
+                        const int pi = pw * PP + 2 * i + (lane >> 4);
+                        const uint8_t* src; size_t c0;
+                        piece(pi, src, c0);
+                        cp_async16(base + pi * ST_STRIDE + 16 * (lane & 15), src + 16 * (lane & 15));
+                    }
+                    for (int i = lane; i < PP; i += 32) {
+                        const int pi = pw * PP + i;
+                        const uint8_t* src; size_t c0;
+                        piece(pi, src, c0);
                         const uint32_t sdst = base + PIECES * ST_STRIDE + pi * SCB;
                         const uint8_t* sp = slot + Q_BYTES;
                         if constexpr (FMT == FMT_SYM_F16) cp_async16(sdst, sp + (c0 / 2) * 2);
@@ -230,11 +232,7 @@ __global__ void __launch_bounds__((NW + 1) * 32) stream_k(const StreamArgs a) {
                 if (++s == STAGES) { s = 0; ph ^= 1; }
             }
         }
-        // drain: every slot released, so no copy is in flight when the CTA exits
-        for (int i = 0; i < STAGES; i++) {
-            if (!mbar_wait(smem_u32(bars + STAGES + s), ph ^ 1, a.err, ST_ERR_EMPTY_WAIT)) { give_up(); return; }
-            if (++s == STAGES) { s = 0; ph ^= 1; }
-        }
+        asm volatile("cp.async.wait_all;" ::: "memory");   // no copy is in flight when the CTA exits
         return;
     }
 
@@ -349,16 +347,59 @@ __global__ void __launch_bounds__((NW + 1) * 32) stream_k(const StreamArgs a) {
     }
 }
 
-// x [rows][K] fp32 -> xs [rows][2][K] 16-bit: hi and lo halves (see split_hi_lo), both in the permuted order of split_pos.
+// What a kernel that splits activation rows plans on the side (its last block): nothing, sub-items of at most maxp pairs from the
+// items of a work list, or the K (or *nh) experts of one token as sub-items of one pair each, pair k = (token 0, row k, w[k]).
+struct SidePlan {
+    const moexb_pair_item* items; int n_items, maxp;                    // a work list
+    const uint8_t* const* slots; const float* w; int K; const int* nh;  // one token
+    moexb_pair_item* subs; moexb_pair* pairs; int* nsub;
+};
+__device__ __forceinline__ void side_plan(const SidePlan& p) {
+    __shared__ int wsum[8];
+    if (p.slots) {
+        const int k = threadIdx.x, n = p.nh ? min(max(*p.nh, 0), p.K) : p.K;
+        if (k < n) { p.subs[k] = {p.slots[k], k, 1}; p.pairs[k] = {0, k, p.w[k]}; }
+        if (k == 0) *p.nsub = n;
+        return;
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int done = 0;
+    for (int base = 0; base < p.n_items; base += 256) {
+        const int i = base + threadIdx.x;
+        moexb_pair_item it = {nullptr, 0, 0};
+        if (i < p.n_items) it = p.items[i];
+        const int mine = (it.count + p.maxp - 1) / p.maxp;
+        int inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += u; }
+        __syncthreads();   // wsum may still be read by the pass before
+        if (lane == 31) wsum[w] = inc;
+        __syncthreads();
+        int at = done + inc - mine;
+        for (int v = 0; v < 8; v++) { if (v < w) at += wsum[v]; done += wsum[v]; }
+        for (int j = 0; j < mine; j++) p.subs[at + j] = {it.slot, it.start + j * p.maxp, min(p.maxp, it.count - j * p.maxp)};
+    }
+    if (threadIdx.x == 0) *p.nsub = done;
+}
+
+// x [rows][H] fp32 -> xs [rows][2][H] 16-bit: hi and lo halves (see split_hi_lo), both in the permuted order of split_pos. Block r takes
+// row r, a thread 8 consecutive inputs, whose places are 8 consecutive ones too; block `rows`, when the launch has one, plans.
 template <bool F16>
-__global__ void split_rows_k(const float* __restrict__ x, uint16_t* __restrict__ xs, int K, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t r = i / K; const int k = (int)(i % K);
-    uint16_t hi, lo;
-    split_hi_lo<F16>(x[i], hi, lo);
-    uint16_t* dst = xs + r * 2 * K + split_pos(k);
-    dst[0] = hi; dst[K] = lo;
+__global__ void __launch_bounds__(256) split_rows_k(const float* __restrict__ x, uint16_t* __restrict__ xs, int rows, const SidePlan plan) {
+    pdl_wait();
+    pdl_trigger();
+    const int r = blockIdx.x, k = 8 * threadIdx.x;
+    if (r == rows) { side_plan(plan); return; }
+    const float4 p = *reinterpret_cast<const float4*>(x + (size_t)r * EH + k), q = *reinterpret_cast<const float4*>(x + (size_t)r * EH + k + 4);
+    const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+    uint16_t hi[8], lo[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) split_hi_lo<F16>(v[i], hi[i], lo[i]);
+    uint16_t* dst = xs + (size_t)r * 2 * EH + split_pos(k);
+    auto put = [&](uint16_t* d, const uint16_t (&w)[8]) {   // places in the order of inputs 0, 4, 1, 5, 2, 6, 3, 7
+        *reinterpret_cast<uint4*>(d) = make_uint4(w[0] | (uint32_t)w[4] << 16, w[1] | (uint32_t)w[5] << 16, w[2] | (uint32_t)w[6] << 16, w[3] | (uint32_t)w[7] << 16);
+    };
+    put(dst, hi); put(dst + EH, lo);
 }
 
 // One row of D = 2048 floats held 8 per thread (thread i: elements 4i..4i+3 and 1024+4i..1024+4i+3): the sum of squares
@@ -598,31 +639,49 @@ __global__ void __launch_bounds__(1024) group_plan1_k(const int* __restrict__ id
     }
 }
 
-// Sub-items of at most maxp pairs from the items of a work list. One block of 1024 threads, one item per thread
-// and pass.
-__global__ void __launch_bounds__(1024) plan_subitems_k(const moexb_pair_item* __restrict__ items, const int* __restrict__ nitems_dev, int nitems_host,
-                                                        moexb_pair_item* __restrict__ subs, int* __restrict__ nsub, int maxp) {
-    const int ni = nitems_dev ? *nitems_dev : nitems_host;
-    int done = 0;
-    for (int base = 0; base < ni; base += 1024) {
-        const int i = base + threadIdx.x;
-        moexb_pair_item it = {nullptr, 0, 0};
-        if (i < ni) it = items[i];
-        const int mine = (it.count + maxp - 1) / maxp;
-        int total;
-        const int at = done + block_scan_1024(mine, total);
-        for (int j = 0; j < mine; j++) subs[at + j] = {it.slot, it.start + j * maxp, min(maxp, it.count - j * maxp)};
-        done += total;
+// Pairs bucketed by expert (moex.cu:1466-1486; kernels.cuh:1030-1045) in one block of 1024 threads: items in ascending expert id over
+// the experts that are held (slot_table[e] != null) and selected, empty ones after them up to E; the pairs of an expert in token
+// order, p = t*K + rank, and empty ones after the last up to T*K. E <= 1024. The pairs are walked 1024 at a time; a pair's place is
+// its expert's running place + the equal ids in the warps before (a table of counts) + the equal ids in the lanes before (a match).
+__global__ void __launch_bounds__(1024) group_pairs_k(const int* __restrict__ idx, const float* __restrict__ w, int T, int K, int E,
+                                                      const uint8_t* const* __restrict__ slot_table, moexb_pair_item* __restrict__ items,
+                                                      moexb_pair* __restrict__ pairs, int* __restrict__ nitems) {
+    __shared__ int at[1024];                             // the expert's count, then its next place (-1 = not held)
+    __shared__ __align__(16) uint8_t wcnt[32][1024];     // [warp][expert] equal ids in the warp's 32 pairs
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = T * K;
+    at[tid] = 0;
+    pdl_wait();
+    pdl_trigger();
+    const uint8_t* slot = tid < E ? slot_table[tid] : nullptr;
+    __syncthreads();
+    for (int p = tid; p < n; p += 1024) { const int e = idx[p]; if (e >= 0 && e < E) atomicAdd(&at[e], 1); }
+    __syncthreads();
+    const int c = slot ? at[tid] : 0;
+    int np, ni;
+    const int start = block_scan_1024(c, np), item = block_scan_1024(c != 0, ni);
+    if (c) items[item] = {slot, start, c};
+    if (tid >= ni && tid < E) items[tid] = {nullptr, 0, 0};
+    if (tid == 0) *nitems = ni;
+    for (int p = np + tid; p < n; p += 1024) pairs[p] = {0, 0, 0.f};
+    at[tid] = slot ? start : -1;
+    for (int base = 0; base < n; base += 1024) {
+        for (int i = tid; i < 32 * 1024 / 16; i += 1024) reinterpret_cast<uint4*>(wcnt)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        const int p = base + tid;
+        int e = p < n ? idx[p] : -1;
+        if (e >= E || (e >= 0 && at[e] < 0)) e = -1;
+        const unsigned m = __match_any_sync(0xffffffffu, e);
+        const int rank = __popc(m & ((1u << lane) - 1));
+        if (e >= 0 && rank == 0) wcnt[warp][e] = (uint8_t)__popc(m);
+        __syncthreads();
+        int place = 0;
+        if (e >= 0) { place = at[e] + rank; for (int v = 0; v < warp; v++) place += wcnt[v][e]; }
+        __syncthreads();
+        if (e >= 0) {
+            pairs[place] = {p / K, p, w[p]};
+            if (rank == 0) atomicAdd(&at[e], (int)__popc(m));
+        }
     }
-    if (threadIdx.x == 0) *nsub = done;
-}
-
-// One token: the K (or *nh) decode experts as sub-items of one pair each, pair k = (token 0, row k, weight w[k]).
-__global__ void plan_decode_k(const uint8_t* const* __restrict__ slots, const float* __restrict__ w, int K, const int* __restrict__ nh,
-                              moexb_pair_item* __restrict__ subs, moexb_pair* __restrict__ pairs, int* __restrict__ nsub) {
-    const int k = threadIdx.x, n = nh ? min(max(*nh, 0), K) : K;
-    if (k < n) { subs[k] = {slots[k], k, 1}; pairs[k] = {0, k, w[k]}; }
-    if (k == 0) *nsub = n;
 }
 
 // Self-test of the bounded waits (moexb_ctx_selftest_timeout): one warp waits on an mbarrier that expects 16 bytes which
