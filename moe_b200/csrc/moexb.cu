@@ -139,6 +139,7 @@ struct moexb_ctx {
     moexb_pair_item* subs = nullptr;                    // sub-items of at most 8 pairs
     int *nsub = nullptr, *err = nullptr;
     float *sx = nullptr, *sx_act = nullptr;             // grouped GEMM, zero point: activation sums per 32-input chunk, of the tokens and of act
+    int* bcnt = nullptr; moexb_pair* bpairs = nullptr;  // the work list as buckets (null when they would be too large)
     int* route_done = nullptr;                          // per token tile: blocks of the routing kernel that have finished (returns to zero)
     int sms = 0, path = 0;                              // path: 0 = streaming kernels, 1 = fp32 SIMT kernels
     int fused_decode = 1;                               // one-token residual stacks run as one cooperative launch
@@ -479,6 +480,11 @@ int moexb_ctx_create(int device, int max_tokens, int max_experts, int top_k, moe
     A(&c->slots, (size_t)top_k + 1); A(&c->wts, (size_t)top_k + 1);
     A(&c->xs, T * 2 * EH); A(&c->act_split, P * 2 * EI); A(&c->subs, (size_t)max_experts + 1 + P / ST_MAXP + 1);
     A(&c->nsub, 2); A(&c->err, 1); A(&c->sx, T * (EH / 32)); A(&c->sx_act, P * (EI / 32)); A(&c->route_done, (size_t)max_tokens); A(&c->staging, (size_t)STAGING_BLOBS * expert_bytes(FMT_ZP));
+    // buckets of max_tokens places for every expert and the shared one, where that is at most 64 MB (6.3 MB for 2048 tokens, 256 experts)
+    if (max_experts <= BK_MAX_E && T * (max_experts + 1) * sizeof(moexb_pair) <= (64u << 20)) {
+        A(&c->bcnt, (size_t)max_experts); A(&c->bpairs, T * (max_experts + 1));
+        if (rc == MOEXB_OK && cudaMemset(c->bcnt, 0, (size_t)max_experts * sizeof(int)) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: memset");
+    }
     if (rc == MOEXB_OK && cudaMemset(c->err, 0, sizeof(int)) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: memset");
     if (rc == MOEXB_OK && cudaMemset(c->route_done, 0, (size_t)max_tokens * sizeof(int)) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: memset");
     if (rc == MOEXB_OK && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) rc = fail(MOEXB_ERR_CUDA, "ctx_create: device attribute");
@@ -986,15 +992,15 @@ static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float*
     });
 }
 
-template <int FMT, bool DOWN, int NW, int D, int NB = 1, int CPS = 2, bool PLAN = false>
-static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa, void* stream) {
-    constexpr int SMEM = tl_smem_bytes<FMT, DOWN, NW, D, NB, PLAN>();
+template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC>
+static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa, const BucketArgs& ba, void* stream) {
+    constexpr int SMEM = tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC>();
     static_assert(SMEM * CPS <= 227 * 1024, "shared memory of the resident CTAs");
     static PerDeviceOnce once;
-    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, PLAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
+    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "tiled stream kernel shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
-    CUDA_TRY(launch_dep(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, PLAN>, CPS * c->sms, NW * 32, SMEM, S(stream), a, pa));
+    CUDA_TRY(launch_dep(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, CPS * c->sms, NW * 32, SMEM, S(stream), a, pa, ba));
     LAUNCHED(DOWN ? "stream_tiled_down" : "stream_tiled_gate_up");
     return MOEXB_OK;
 }
@@ -1004,39 +1010,43 @@ static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa
 // (CTAs of 8 warps, 2 slices in flight each - the same bytes in flight, twice the issue slots in use).
 // From 8 tokens on the symmetric formats also take sub-items of up to 8 pairs (two column blocks; tiled_maxp below): the
 // gate/up columns of 8 pairs are 66 KB, so that kernel runs as one CTA of 16 warps per SM.
-// plan: the gate/up kernel makes the work list itself (no planning launch before it).
-template <int FMT, bool DOWN, bool PLAN = false>
-static int tiled_launch_one(moexb_ctx* c, const TiledArgs& a, int T, void* stream, const PlanArgs& pa = PlanArgs{}) {
-    static_assert(!PLAN || FMT == FMT_SYM_F16, "the in-kernel work list fits beside the ring of the fp16-scale format only");
-    if (T < 8) return tiled_launch_cfg<FMT, DOWN, 4, 4, 1, 2, PLAN>(c, a, pa, stream);
-    if (FMT == FMT_ZP || c->pairs_per_pass == 4) return tiled_launch_cfg<FMT, DOWN, 8, 2, 1, 2, PLAN>(c, a, pa, stream);
+template <int FMT, bool DOWN, int SRC>
+static int tiled_launch_one(moexb_ctx* c, const TiledArgs& a, int T, void* stream, const PlanArgs& pa, const BucketArgs& ba) {
+    static_assert(SRC != TL_PLAN || FMT == FMT_SYM_F16, "the in-kernel work list fits beside the ring of the fp16-scale format only");
+    if (T < 8) return tiled_launch_cfg<FMT, DOWN, 4, 4, 1, 2, SRC>(c, a, pa, ba, stream);
+    if (FMT == FMT_ZP || c->pairs_per_pass == 4) return tiled_launch_cfg<FMT, DOWN, 8, 2, 1, 2, SRC>(c, a, pa, ba, stream);
     if constexpr (FMT == FMT_ZP) return MOEXB_OK;
-    else if constexpr (DOWN) return tiled_launch_cfg<FMT, DOWN, 8, 2, 2, 2, PLAN>(c, a, pa, stream);
-    else return tiled_launch_cfg<FMT, DOWN, 16, 2, 2, 1, PLAN>(c, a, pa, stream);
+    else if constexpr (DOWN) return tiled_launch_cfg<FMT, DOWN, 8, 2, 2, 2, SRC>(c, a, pa, ba, stream);
+    else return tiled_launch_cfg<FMT, DOWN, 16, 2, 2, 1, SRC>(c, a, pa, ba, stream);
 }
 // Pairs per sub-item that tiled_launch_one's kernels take.
 static int tiled_maxp(const moexb_ctx* c, int fmt, int T) { return (T >= 8 && fmt != FMT_ZP) ? c->pairs_per_pass : 4; }
-// Whether the gate/up kernel can make the work list of this batch itself (tiled.cuh: plan_in_cta).
-// (fp16-scale format: with the wider slices of the other formats the list does not fit beside two CTAs' rings.)
-// One token on one GPU needs no list (the routing kernel writes the nine one-pair sub-items itself); across GPUs the list is
-// made in the kernel for any batch, because a planning launch would sit behind the wait for the peers.
-static bool plan_in_kernel(const moexb_ctx* c, int fmt, int T, int K, int E, bool ep = false) {
+// Expert parallelism: whether the gate/up kernel makes the work list of this batch itself (tiled.cuh: plan_in_cta) - a planning launch
+// would sit behind the wait for the peers. (fp16-scale format: with the wider slices of the others the list does not fit.)
+static bool plan_in_kernel(int fmt, int T, int K, int E) {
     static const bool on = [] { const char* e = getenv("MOEXB_PLAN_IN_KERNEL"); return !(e && e[0] == '0'); }();
-    return on && fmt == FMT_SYM_F16 && (T >= 2 || ep) && T <= PL_MAX_TOKENS && K <= PL_MAX_K && E <= PL_MAX_E;
+    return on && fmt == FMT_SYM_F16 && T <= PL_MAX_TOKENS && K <= PL_MAX_K && E <= PL_MAX_E;
 }
 
-// The same on blobs in the tiled layout (sub-item slots point into a tiled layer image). plan: null = the list is already
-// in the context (subs, nsub, pairs); else the gate/up kernel makes it and leaves it there for the down kernel.
-static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int T, void* stream, const PlanArgs* plan = nullptr) {
-    TiledArgs a{c->subs, c->nsub, pairs, c->xs, act32, c->act_split, ypair, c->err};
+// The same on blobs in the tiled layout (sub-item slots point into a tiled layer image). The work list: plan = the gate/up kernel
+// makes it and leaves it in the context for the down kernel; buckets = the router's; neither = it is in the context.
+static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int T, void* stream, const PlanArgs* plan = nullptr,
+                         const BucketArgs* buckets = nullptr) {
+    const TiledArgs a{c->subs, c->nsub, buckets ? buckets->pairs : pairs, c->xs, act32, c->act_split, ypair, c->err};
+    TiledArgs d = a;
+    d.xs = c->act_split;
+    PlanArgs pa = plan ? *plan : PlanArgs{};
+    pa.subs_out = c->subs; pa.nsub_out = c->nsub;
+    const BucketArgs ba = buckets ? *buckets : BucketArgs{};
     return by_fmt(fmt, [&]<int FMT>() {
         int rc;
-        if constexpr (FMT == FMT_SYM_F16) rc = plan ? tiled_launch_one<FMT, false, true>(c, a, T, stream, *plan) : tiled_launch_one<FMT, false>(c, a, T, stream);
-        else rc = tiled_launch_one<FMT, false>(c, a, T, stream);
-        if (rc != MOEXB_OK) return rc;
-        TiledArgs d = a;
-        d.xs = c->act_split;
-        return tiled_launch_one<FMT, true>(c, d, T, stream);
+        if (buckets) {
+            rc = tiled_launch_one<FMT, false, TL_BUCKETS>(c, a, T, stream, pa, ba);
+            return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, ba);
+        }
+        if constexpr (FMT == FMT_SYM_F16) rc = plan ? tiled_launch_one<FMT, false, TL_PLAN>(c, a, T, stream, pa, ba) : tiled_launch_one<FMT, false, TL_LIST>(c, a, T, stream, pa, ba);
+        else rc = tiled_launch_one<FMT, false, TL_LIST>(c, a, T, stream, pa, ba);
+        return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, ba);
     });
 }
 
@@ -1069,11 +1079,11 @@ static int grouped_rows(moexb_ctx* c, int fmt, const float* x, uint16_t* xs, int
     return MOEXB_OK;
 }
 
-// Experts of a large batch on the tensor-core grouped GEMM: the planner left the tiles in the context (subs, nsub), grouped_rows or
-// the token owners (expert parallelism) the activation rows.
-static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int parts, float* ypair, void* stream) {
+// Experts of a large batch on the tensor-core grouped GEMM: the tiles are in the context (subs, nsub) or in the buckets, and grouped_rows or
+// the token owners (expert parallelism) left the activation rows.
+static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int parts, float* ypair, void* stream, const BucketArgs* buckets = nullptr) {
     return by_fmt(fmt, [&]<int FMT>() {
-        GroupedArgs a{c->subs, c->nsub, pairs, c->xs, c->sx, c->act_split, c->sx_act, ypair, c->err, parts};
+        GroupedArgs a{buckets ? nullptr : c->subs, c->nsub, buckets ? *buckets : BucketArgs{}, buckets ? buckets->pairs : pairs, c->xs, c->sx, c->act_split, c->sx_act, ypair, c->err, parts};
         int rc = grouped_launch_one<FMT, false>(c, a, stream);
         if (rc != MOEXB_OK) return rc;
         a.xs = c->act_split; a.sx = c->sx_act; a.parts = 2;
@@ -1166,14 +1176,20 @@ extern "C" {
 // Router logits (into the context, [T][E + 1]) and the top-K selection in one launch; decode: also the K + 1 one-pair
 // sub-items of a single token.
 struct RouteEp { const EpDevice* dev; int row_bytes; unsigned phase; const unsigned* step; };
+struct RouteOut { bool buckets, shared; int* idx; float* w; };   // pairs into the buckets (with the shared expert's); the caller's copies
 template <typename WT>
-static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, int K, void* stream, bool decode, int tok0 = 0, const RouteEp* rep = nullptr) {
+static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
     // tok0: the T rows at xf are tokens tok0.. of the batch - their logits, ids and weights go to those rows of the workspace
     const int E = L->n_routed;
     const WT* W = static_cast<const WT*>(L->router);
     float* logits = c->logits + (size_t)tok0 * (E + 1);
     TopkOut o{c->idx + (size_t)tok0 * K, c->w + (size_t)tok0 * K, L->slot_table, decode ? c->slots : nullptr, decode ? c->wts : nullptr,
               decode ? c->subs : nullptr, decode ? c->pairs : nullptr, decode ? c->nsub : nullptr};
+    if (ro.buckets) {
+        o.bcnt = c->bcnt; o.bpairs = c->bpairs; o.bstride = c->max_tokens; o.e_lo = L->first_local; o.e_hi = L->first_local + L->n_local; o.npairs = T * K;
+        o.bshared = ro.shared;
+    }
+    o.idx2 = ro.idx; o.w2 = ro.w;
     if (rep) { o.ep = rep->dev; o.ep_row_bytes = rep->row_bytes; o.ep_phase = rep->phase; o.ep_step = rep->step; }
     auto run = [&]<int NJ>() -> int {
         // expert parallelism with few own tokens: one token per block row, so that each token's selection and dispatch stores are
@@ -1214,9 +1230,9 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, in
 }
 
 extern "C" {
-static int layer_route(moexb_ctx* c, moexb_layer* L, const float* xf, int T, int K, void* stream, bool decode, int tok0 = 0, const RouteEp* rep = nullptr) {
+static int layer_route(moexb_ctx* c, moexb_layer* L, const float* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
     PROF(c, MOEXB_PROF_ROUTER, stream);
-    return L->router_dtype == MOEXB_F32 ? route_launch<float>(c, L, xf, T, K, stream, decode, tok0, rep) : route_launch<__half>(c, L, xf, T, K, stream, decode, tok0, rep);
+    return L->router_dtype == MOEXB_F32 ? route_launch<float>(c, L, xf, T, K, stream, decode, ro, tok0, rep) : route_launch<__half>(c, L, xf, T, K, stream, decode, ro, tok0, rep);
 }
 
 // One layer. xin: the layer input as f32 [T][H]. flags as moexb_layer_forward. pre_normed: the context already holds
@@ -1248,7 +1264,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
         if (rc != MOEXB_OK) return rc;
     }
     const bool decode = T == 1 && all_local && shared && !partial && !prefill;
-    int rc = layer_route(c, L, xf, T, K, stream, decode);
+    const bool buckets = tiled && !decode && c->bpairs;
+    int rc = layer_route(c, L, xf, T, K, stream, decode, RouteOut{buckets, buckets && shared, idx_out, w_out});
     if (rc != MOEXB_OK) return rc;
     int ranks = K;                  // rows of ypair per token that the final reduction adds
     const float* extra = nullptr;   // + the shared expert's rows
@@ -1271,9 +1288,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
     } else {
         const int parts = (x_bf16 && !block) ? 1 : 2;
         const int maxp = prefill ? grouped_maxp(L->fmt) : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
-        const bool in_kernel = tiled && !prefill && plan_in_kernel(c, L->fmt, T, K, E);
-        const PlanArgs plan{c->idx, c->w, T, K, E, L->slot_table, L->first_local, L->first_local + L->n_local, shared ? c->logits + E : nullptr, ld, sh0, sh1, maxp, c->subs, c->pairs, c->nsub, nullptr, nullptr, 0u};
-        if (!in_kernel) {
+        const BucketArgs bk{c->bcnt, c->bpairs, c->max_tokens, E, shared ? sh0 : 0, shared ? sh1 : 0, maxp, L->slot_table};
+        if (!buckets) {
             PROF(c, MOEXB_PROF_GROUP, stream);
             // room in shared memory for the routed pairs (12 bytes each), so that the list is written out in full lines
             constexpr int PLAN_STAGE_MAX = 196608;
@@ -1292,8 +1308,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
             rc = grouped_rows(c, L->fmt, xf, c->xs, T, parts, stream);
             if (rc != MOEXB_OK) return rc;
         }
-        rc = prefill ? grouped_experts(c, L->fmt, c->pairs, parts, c->ypair, stream)
-           : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, in_kernel ? &plan : nullptr)
+        rc = prefill ? grouped_experts(c, L->fmt, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
+           : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr)
            : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream)
                        : pairs_launch(c, L->fmt, c->items, c->nitems, min(E, T * K) + 1, c->pairs, xf, c->act, c->ypair, stream);
         if (rc != MOEXB_OK) return rc;
@@ -1304,12 +1320,10 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
         const float* xres = (block && !partial) ? xin : nullptr;
         float* xn_next = next_norm ? c->xn : nullptr;
         const int* held = (!all_local && ranks == K) ? c->idx : nullptr;
-        if (f16) CUDA_TRY(launch_dep(reduce_residual_norm_k<true>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local));
-        else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, prefill ? (uint16_t*)nullptr : c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local));
+        if (f16) CUDA_TRY(launch_dep(reduce_residual_norm_k<true>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local, buckets ? c->bcnt : (int*)nullptr, E));
+        else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, prefill ? (uint16_t*)nullptr : c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local, buckets ? c->bcnt : (int*)nullptr, E));
         LAUNCHED("reduce_residual_norm");
     }
-    if (idx_out) CUDA_TRY(cudaMemcpyAsync(idx_out, c->idx, (size_t)T * K * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    if (w_out) CUDA_TRY(cudaMemcpyAsync(w_out, c->w, (size_t)T * K * sizeof(float), cudaMemcpyDeviceToDevice, st));
     return MOEXB_OK;
 }
 
@@ -1361,8 +1375,8 @@ int moexb_ep_residual_norm(moexb_ctx* c, moexb_layer* next, const float* x, cons
     float* xn = next ? c->xn : nullptr;
     PROF(c, MOEXB_PROF_COMBINE, stream);
     const float* no_extra = nullptr; const int* no_idx = nullptr;
-    if (f16) CUDA_TRY(launch_dep(reduce_residual_norm_k<true>, T, 256, 0, S(stream), total, no_extra, x, out, 1, xn, c->xs, 1e-6f, 0, 0, no_idx, 0, 0));
-    else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, S(stream), total, no_extra, x, out, 1, xn, c->xs, 1e-6f, 0, 0, no_idx, 0, 0));
+    if (f16) CUDA_TRY(launch_dep(reduce_residual_norm_k<true>, T, 256, 0, S(stream), total, no_extra, x, out, 1, xn, c->xs, 1e-6f, 0, 0, no_idx, 0, 0, (int*)nullptr, 0));
+    else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, S(stream), total, no_extra, x, out, 1, xn, c->xs, 1e-6f, 0, 0, no_idx, 0, 0, (int*)nullptr, 0));
     LAUNCHED("ep_residual_norm");
     return MOEXB_OK;
 }
@@ -1719,7 +1733,7 @@ int moexb_ep_dispatch(moexb_ep* e, moexb_layer* L, int l, const void* X, int x_d
     }
     // the routing kernel sends each token to the peers as soon as its experts are selected and raises the tokens' flags
     const RouteEp rep{e->dev, parts * EH * 2, (unsigned)(l + 1), e->step};
-    return layer_route(c, L, xn_own, n_own, K, stream, false, t0, &rep);
+    return layer_route(c, L, xn_own, n_own, K, stream, false, RouteOut{}, t0, &rep);
 }
 
 int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
@@ -1731,7 +1745,7 @@ int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
     const bool tiled = L->layout == MOEXB_LAYOUT_TILED, prefill = e->prefill;
     const int maxp = prefill ? grouped_maxp(L->fmt) : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
     const unsigned* flags = reinterpret_cast<const unsigned*>(e->peers.base[e->g.rank] + e->lay.flag_a);
-    const bool in_kernel = tiled && !prefill && plan_in_kernel(c, L->fmt, T, K, E, true);
+    const bool in_kernel = tiled && !prefill && plan_in_kernel(L->fmt, T, K, E);
     // the dispatch flags of all tokens are waited for by whoever makes the work list: the gate/up CTAs, or the planning kernel
     const PlanArgs plan{c->idx, c->w, T, K, E, L->slot_table, L->first_local, L->first_local + L->n_local, c->logits + E, E + 1, t0, t1, maxp, c->subs, c->pairs, c->nsub, flags, e->step, (unsigned)(l + 1)};
     if (!in_kernel) {

@@ -145,6 +145,9 @@ struct TopkOut {
     // weights to every rank, the activation row (ep_row_bytes at [token] of the exchange buffer's row area) to the ranks that
     // hold one of the selected experts - and the block then raises the tokens' dispatch flags
     const EpDevice* ep = nullptr; int ep_row_bytes = 0; unsigned ep_phase = 0; const unsigned* ep_step = nullptr;
+    // the pairs into the experts' buckets (BucketArgs): experts [e_lo, e_hi) are held here; npairs = T * K
+    int* bcnt = nullptr; moexb_pair* bpairs = nullptr; int bstride = 0, e_lo = 0, e_hi = 0, npairs = 0; bool bshared = false;
+    int* idx2 = nullptr; float* w2 = nullptr;   // a second copy of ids and weights (the caller's buffers)
 };
 __device__ __forceinline__ unsigned f2key(float v) { const unsigned u = __float_as_uint(v); return (u & 0x80000000u) ? ~u : (u | 0x80000000u); }
 __device__ __forceinline__ float key2f(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
@@ -161,7 +164,7 @@ __device__ __forceinline__ void topk_token(const float* __restrict__ l, int t, i
         if (j < nj) { const float a = CG ? __ldcg(l + lane + 32 * j) : l[lane + 32 * j]; v[j] = a != a ? -INFINITY : a; }
         m = fmaxf(m, v[j]);
     }
-    const float gate_logit = (o.slots_out && lane == K) ? (CG ? __ldcg(l + E) : l[E]) : 0.f;
+    const float gate_logit = ((o.slots_out || o.bshared) && lane == K) ? (CG ? __ldcg(l + E) : l[E]) : 0.f;
 #pragma unroll
     for (int off = 16; off; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
     unsigned key[NJ];
@@ -208,9 +211,14 @@ __device__ __forceinline__ void topk_token(const float* __restrict__ l, int t, i
         const float wk = norm ? mine / total : mine;
         o.idx[(size_t)t * K + lane] = mine_i;
         o.w[(size_t)t * K + lane] = wk;
+        if (o.bpairs && mine_i >= o.e_lo && mine_i < o.e_hi)
+            o.bpairs[(size_t)mine_i * o.bstride + atomicAdd(o.bcnt + mine_i, 1)] = {t, t * K + lane, wk};
+        if (o.idx2) o.idx2[(size_t)t * K + lane] = mine_i;
+        if (o.w2) o.w2[(size_t)t * K + lane] = wk;
         if (o.slots_out) { o.slots_out[(size_t)t * (K + 1) + lane] = o.slot_table[mine_i]; o.wts_out[(size_t)t * (K + 1) + lane] = wk; }
         if (o.dsubs) { o.dsubs[lane] = {o.slot_table[mine_i], lane, 1}; o.dpairs[lane] = {0, lane, wk}; }  // one token: expert k = sub-item k
     }
+    if (o.bshared && lane == K) o.bpairs[(size_t)E * o.bstride + t] = {t, o.npairs + t, 1.f / (1.f + expf(-gate_logit))};
     if (o.slots_out && lane == K) {
         const float gate = 1.f / (1.f + expf(-gate_logit));
         o.slots_out[(size_t)t * (K + 1) + K] = o.slot_table[E];

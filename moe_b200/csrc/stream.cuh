@@ -461,10 +461,11 @@ template <bool F16>
 __global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __restrict__ ypair, const float* __restrict__ extra, const float* __restrict__ x,
                                                               float* __restrict__ out, int K, float* __restrict__ xn_next,
                                                               uint16_t* __restrict__ xs_next, float eps, int ex0, int ex1,
-                                                              const int* __restrict__ idx, int e_lo, int e_hi) {
+                                                              const int* __restrict__ idx, int e_lo, int e_hi, int* __restrict__ cnt, int E) {
     pdl_wait();
     pdl_trigger();
     const size_t t = blockIdx.x;
+    if (cnt && t == 0 && (int)threadIdx.x < E) cnt[threadIdx.x] = 0;   // the layer's bucket counts: its expert kernels are done
     if ((int)t < ex0 || (int)t >= ex1) extra = nullptr;  // extra rows exist only for tokens [ex0, ex1)
     // idx given: only the ranks whose expert lies in [e_lo, e_hi) were computed here (expert parallelism); skip the others
     unsigned have = 0xffffffffu;
@@ -682,6 +683,72 @@ __global__ void __launch_bounds__(1024) group_pairs_k(const int* __restrict__ id
             if (rank == 0) atomicAdd(&at[e], (int)__popc(m));
         }
     }
+}
+
+// ---- the work list as buckets (no planning launch) ------------------------------------------------------------------------------
+//
+// Where every expert of a layer is routed by this GPU's own kernels, the warp that selects a token's experts puts its pairs straight
+// into the experts' buckets (topk_token), and a kernel that walks sub-items derives them from the 256 counts: a scan by one warp,
+// then a binary search per sub-item. A planning kernel between the two cost 11 us a layer (23 tokens: 83 us a layer with it, 75
+// without), and the list made from ids and weights inside the gate/up kernel 1.4 us more than this (4 tokens x 40 layers 1163, now
+// 1108 us).
+// The order of an expert's pairs is not pinned; a pair's result does not depend on its place. The combine kernel, which runs when
+// nothing reads the counts any more, clears them.
+constexpr int BK_MAX_E = 256, BK_LOCAL = 64;
+struct BucketArgs {
+    const int* cnt;                   // [E] pairs of each expert
+    const moexb_pair* pairs;          // [E + 1][stride]; the last bucket is the shared expert's, place t = token t
+    int stride, E, sh0, sh1, maxp;    // the shared expert takes the tokens [sh0, sh1); sub-items of at most maxp pairs
+    const uint8_t* const* slot_table; // E + 1 blob pointers
+};
+struct BucketSmem {
+    const uint8_t* slot[BK_MAX_E + 1];
+    int wide[BK_MAX_E + 2], narrow[BK_MAX_E + 2];   // sub-items of more than maxp / 2 pairs, and of fewer, before expert e
+    int cnt[BK_MAX_E + 1];
+    moexb_pair_item local[BK_LOCAL];                // a CTA's own range of sub-items
+};
+// What does not depend on the router: the blob pointers. A CTA barrier must follow.
+__device__ __forceinline__ void bucket_prepare(BucketSmem& L, const BucketArgs& a) {
+    for (int i = threadIdx.x; i <= a.E; i += blockDim.x) L.slot[i] = a.slot_table[i];
+}
+// By one warp, after the wait for the router. A CTA barrier must follow.
+__device__ __forceinline__ void bucket_scan(BucketSmem& L, const BucketArgs& a, int lane) {
+    const int Ts = L.slot[a.E] ? a.sh1 - a.sh0 : 0, maxp = a.maxp;
+    const unsigned rcp = 0xFFFFFFFFu / maxp + 1;   // c / maxp = the high half of c * rcp, exact for the counts (below 65536)
+    auto wide = [=](int c) { const int full = __umulhi(c, rcp); return full + (c - full * maxp > maxp / 2); };
+    auto narrow = [=](int c) { const int r = c - (int)__umulhi(c, rcp) * maxp; return (int)(r > 0 && r <= maxp / 2); };
+    int c[8] = {}, sw = 0, sn = 0;
+    if (8 * lane < a.E) {
+        const int4 p = __ldcg(reinterpret_cast<const int4*>(a.cnt) + 2 * lane), q = __ldcg(reinterpret_cast<const int4*>(a.cnt) + 2 * lane + 1);
+        c[0] = p.x; c[1] = p.y; c[2] = p.z; c[3] = p.w; c[4] = q.x; c[5] = q.y; c[6] = q.z; c[7] = q.w;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) { sw += wide(c[j]); sn += narrow(c[j]); }
+    int iw = sw, in = sn;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int uw = __shfl_up_sync(0xffffffffu, iw, o), un = __shfl_up_sync(0xffffffffu, in, o);
+        if (lane >= o) { iw += uw; in += un; }
+    }
+    int bw = iw - sw, bn = in - sn;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int e = 8 * lane + j;
+        if (e < a.E) { L.wide[e] = bw; L.narrow[e] = bn; L.cnt[e] = c[j]; }
+        bw += wide(c[j]); bn += narrow(c[j]);
+    }
+    if (lane == 31) { L.wide[a.E] = bw; L.narrow[a.E] = bn; L.cnt[a.E] = Ts; L.wide[a.E + 1] = bw + wide(Ts); L.narrow[a.E + 1] = bn + narrow(Ts); }
+}
+// Sub-item i: the wide ones of all experts first.
+__device__ __forceinline__ moexb_pair_item bucket_sub(const BucketSmem& L, const BucketArgs& a, int i) {
+    const int nw = L.wide[a.E + 1];
+    const bool w = i < nw;
+    const int* pre = w ? L.wide : L.narrow;
+    const int at = w ? i : i - nw;
+    int lo = 0, hi = a.E;   // the last e with pre[e] <= at
+    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (pre[mid] <= at) lo = mid; else hi = mid - 1; }
+    const int c = L.cnt[lo], j = w ? at - pre[lo] : L.wide[lo + 1] - L.wide[lo];
+    return {L.slot[lo], lo * a.stride + (lo == a.E ? a.sh0 : 0) + j * a.maxp, min(a.maxp, c - j * a.maxp)};
 }
 
 // Self-test of the bounded waits (moexb_ctx_selftest_timeout): one warp waits on an mbarrier that expects 16 bytes which

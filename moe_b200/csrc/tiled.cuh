@@ -230,11 +230,14 @@ struct TiledArgs {
 // DOWN = true : row tile = 16 down rows, 1 slice (K = 512); ypair = w * (down . act).
 // NB = 8-column blocks of activations per sub-item (1: up to 4 pairs, 2: up to 8 pairs - the weights of an expert with 5-8
 // pairs are then unpacked once instead of twice); CPS = CTAs per SM the launch is sized for.
-// PLAN (gate/up only): the CTA makes the work list itself (plan_in_cta) from pa instead of reading a.subs / a.pairs / a.nsub.
-template <int FMT, bool DOWN, int NW, int D, int NB = 1, int CPS = 2, bool PLAN = false>
-__global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a, const PlanArgs pa) {
+// SRC: where the work list comes from - TL_LIST: a.subs / a.pairs / a.nsub; TL_PLAN (gate/up only): the CTA makes it itself
+// (plan_in_cta) from pa; TL_BUCKETS (gate/up only): the router's buckets (ba).
+enum : int { TL_LIST = 0, TL_PLAN = 1, TL_BUCKETS = 2 };
+template <int FMT, bool DOWN, int NW, int D, int NB = 1, int CPS = 2, int SRC = TL_LIST>
+__global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a, const PlanArgs pa, const BucketArgs ba) {
+    constexpr bool PLAN = SRC == TL_PLAN, BUCKETS = SRC == TL_BUCKETS;
     static_assert(NB == 1 || FMT != FMT_ZP, "two column blocks are built for the symmetric formats only");
-    static_assert(!PLAN || !DOWN, "the down kernel reads the list the gate/up kernel left in global memory");
+    static_assert(SRC == TL_LIST || !DOWN, "the down kernel reads the list the gate/up kernel left in global memory");
     constexpr int GB = tl_group_bytes<FMT>(), SB = tl_slice_bytes<FMT>();
     constexpr int KS = DOWN ? 1 : 4;                       // slices per row tile
     constexpr int RPS = (DOWN ? 128 : 64) / NW;            // rounds per sub-item
@@ -245,7 +248,8 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* bsm = smem + NW * D * SB;                                 // 8 * NB activation columns
     uint64_t* bars = reinterpret_cast<uint64_t*>(bsm + 8 * NB * BCOL); // full[NW][D]
-    PlanSmem& P = *reinterpret_cast<PlanSmem*>(bars + NW * D + 8);      // PLAN only (the launch adds the room)
+    PlanSmem& P = *reinterpret_cast<PlanSmem*>(bars + NW * D + 8);      // PLAN, BUCKETS: the launch adds the room
+    BucketSmem& L = *reinterpret_cast<BucketSmem*>(bars + NW * D + 8);
     static_assert(!PLAN || sizeof(PlanTmp) <= NW * D * SB, "the planning scratch fits where the ring will be");
     // zero point: the sum of the activations over each 32-input chunk, per column: [K slice][group][chunk][8 columns]
     __shared__ __align__(16) float csum[Z ? KS * 8 * 2 * 8 : 4];
@@ -253,6 +257,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     if (threadIdx.x < NW * D) mbar_init(smem_u32(bars + threadIdx.x), 1);
     if (threadIdx.x == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if constexpr (PLAN) plan_prepare(P, *reinterpret_cast<PlanTmp*>(smem), pa);
+    if constexpr (BUCKETS) bucket_prepare(L, ba);
     __syncthreads();
     // Gate/up: the sub-items come from the kernel before this one. Down: they are older (the gate/up kernel read them
     // too), so the weight copies start while gate/up still runs; only the activation columns wait for it.
@@ -272,14 +277,28 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
         pdl_trigger();
         // the planning scratch was written through the generic proxy where the bulk copies (async proxy) are about to land
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    } else if constexpr (BUCKETS) {
+        pdl_wait();
+        if (warp == 0) bucket_scan(L, ba, lane);
+        __syncthreads();
+        if (blockIdx.x == 0) {   // the list for the down kernel, which may read it as soon as every CTA here has triggered
+            const int nw = L.wide[ba.E + 1], n = nw + L.narrow[ba.E + 1];
+            for (int i = threadIdx.x; i < n; i += NW * 32) pa.subs_out[i] = bucket_sub(L, ba, i);
+            if (threadIdx.x < 2) pa.nsub_out[threadIdx.x] = threadIdx.x ? nw : n;
+            __threadfence();
+            __syncthreads();
+        }
+        pdl_trigger();
     } else if (!DOWN) { pdl_wait(); pdl_trigger(); }
+    int first_sub = 0;   // BUCKETS: of this CTA's range
     // the work list: the CTA's own (PLAN) or the one in global memory
     auto sub_at = [&](int i) -> moexb_pair_item {
         if constexpr (PLAN) { const PlanSub su = P.subs[i]; return {P.slot[su.e], su.start, su.count}; }
+        else if constexpr (BUCKETS) return i < first_sub + BK_LOCAL ? L.local[i - first_sub] : bucket_sub(L, ba, i);
         else return a.subs[i];
     };
     auto pair_at = [&](int i) -> moexb_pair { if constexpr (PLAN) return P.pair_at(i); else return a.pairs[i]; };
-    const int nsub0 = PLAN ? P.nsub[0] : a.nsub[0], nsub1 = PLAN ? P.nsub[1] : a.nsub[1];
+    const int nsub0 = PLAN ? P.nsub[0] : BUCKETS ? L.wide[ba.E + 1] + L.narrow[ba.E + 1] : a.nsub[0], nsub1 = PLAN ? P.nsub[1] : BUCKETS ? L.wide[ba.E + 1] : a.nsub[1];
     // This CTA's contiguous range of rounds: an equal share of the cost, a round of a wide sub-item (more than 4 pairs,
     // they come first in subs[]) counting CW and any other CN.
     constexpr int CN = 10, CW = NB == 2 ? 13 : 10;   // measured: a wide round takes 1.3 times a narrow one in both kernels
@@ -288,6 +307,12 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     auto round_at = [&](long long x) { return (int)(x < RW * CW ? x / CW : RW + (x - RW * CW) / CN); };
     const int r0 = round_at(C * blockIdx.x / gridDim.x), r1 = round_at(C * (blockIdx.x + 1) / gridDim.x);
     const int Q = (r1 - r0) * KS;  // slices this warp will consume
+    if constexpr (BUCKETS) {
+        first_sub = r0 / RPS;
+        const int i = first_sub + threadIdx.x;
+        if (threadIdx.x < BK_LOCAL && r1 > r0 && i <= (r1 - 1) / RPS) L.local[threadIdx.x] = bucket_sub(L, ba, i);
+        __syncthreads();
+    }
     uint8_t* ring = smem + warp * D * SB;
     uint64_t* full = bars + warp * D;
 
@@ -467,7 +492,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     }
 }
 
-template <int FMT, bool DOWN, int NW, int D, int NB = 1, bool PLAN = false>
-constexpr int tl_smem_bytes() { return NW * D * tl_slice_bytes<FMT>() + 8 * NB * st_bcol_bytes<DOWN>() + NW * D * 8 + 64 + (PLAN ? (int)sizeof(PlanSmem) + 16 : 0); }
+template <int FMT, bool DOWN, int NW, int D, int NB = 1, int SRC = TL_LIST>
+constexpr int tl_smem_bytes() { return NW * D * tl_slice_bytes<FMT>() + 8 * NB * st_bcol_bytes<DOWN>() + NW * D * 8 + 64 + (SRC == TL_PLAN ? (int)sizeof(PlanSmem) + 16 : SRC == TL_BUCKETS ? (int)sizeof(BucketSmem) + 16 : 0); }
 
 }  // namespace moexb
