@@ -1210,14 +1210,18 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, in
                 return MOEXB_OK;
             };
             // a small batch: 16 outputs x 8 tokens per block, to reach every SM; a prefill chunk goes to the register-tiled
-            // kernel (32 tokens x 16 outputs per block, FMA-bound)
+            // kernel (64 tokens x 16 outputs per block, FMA-bound)
             auto gemm2 = [&]() -> int {
-                constexpr int SMEM = 2 * rg2_stage_bytes<WT>();
+                constexpr int SMEM = RG2_ST * rg2_stage_bytes<WT>();
                 static PerDeviceOnce once;
                 const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(route_gemm2_k<WT, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
                 if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "router kernel shared memory: %s", cudaGetErrorString(attr_err));
                 CUDA_TRY(launch_dep(route_gemm2_k<WT, NJ>, dim3((E + 1 + RG2_TN - 1) / RG2_TN, (T + RG2_TM - 1) / RG2_TM), 256, SMEM, S(stream),
-                                    W, xf, logits, E, K, 1, T, c->route_done, o));
+                                    W, xf, logits, E, K, 1, T, c->route_done, o, rep ? 1 : 0));
+                if (!rep) {
+                    LAUNCHED("route");
+                    CUDA_TRY(launch_dep(router_topk_k<8, NJ>, (T + 7) / 8, 256, 0, S(stream), (const float*)logits, E, K, 1, E + 1, T, o));
+                }
                 return MOEXB_OK;
             };
             const int rc = T >= 256 ? gemm2() : gemm.template operator()<2, 8>();

@@ -357,88 +357,117 @@ __global__ void __launch_bounds__(WARPS * 32) route_gemm_k(const WT* __restrict_
     ep_raise_dispatch_flags(o, r0, min(TR, T - r0));
 }
 
-// The same for a prefill chunk, register-tiled. A block of 8 warps owns 32 tokens x 16 outputs; warp (wm, wn) the 8 tokens
-// 8*wm.. and the 8 outputs 8*wn.., every lane the same 4 of each 128 inputs as in gemv_rows_k, so a lane holds 64 partial
-// sums and each (token, output) sum is formed in the pinned order. Token rows and weight rows come through shared memory in
-// chunks of 256 inputs (cp.async, two stages; two blocks per SM): per 128 inputs a warp reads 16 x 16 bytes per lane and does 256 fused
-// multiply-adds, which makes the kernel FMA-bound where route_gemm_k is bound by re-reading the weights from L2. The last
-// block of a token tile selects the experts of its 32 tokens. grid (ceil((E + 1) / 16), ceil(T / 32)); I = 2048.
-constexpr int RG2_TM = 32, RG2_TN = 16, RG2_KC = 256;
+// The sums of n accumulators over the 32 lanes of a warp, n / 32 of them left in each lane (lane l: accumulators l * n / 32 ..): at
+// every step a lane keeps half of what it has and hands the other half to its partner. The additions are those of warp_sum's
+// butterfly, so every sum has the same bits, with 124 shuffles for 128 accumulators instead of 640.
+template <int N, int M = 16>
+__device__ __forceinline__ void warp_sums(float* a, int lane) {
+    const bool up = lane & M;
+#pragma unroll
+    for (int k = 0; k < N / 2; k++) {
+        const float keep = up ? a[k + N / 2] : a[k], give = up ? a[k] : a[k + N / 2];
+        a[k] = keep + __shfl_xor_sync(0xffffffffu, give, M);
+    }
+    if constexpr (M > 1) warp_sums<N / 2, M / 2>(a, lane);
+}
+
+// The logits of a prefill chunk, register-tiled. A block of 8 warps owns 64 tokens x 16 outputs; warp (wm, wn) the 16 tokens
+// 16*wm.. and the 8 outputs 8*wn.., every lane the same 4 of each 128 inputs as in gemv_rows_k, so a lane holds 128 partial
+// sums and each (token, output) sum is formed in the pinned order. Token and weight rows come through shared memory 128 inputs at a
+// time (cp.async, four stages, one block per SM): per 128 inputs a warp reads 24 x 16 bytes per lane for 512 fused multiply-adds, so
+// that the shared-memory reads stay below the multiply-adds; with half as many partial sums (32 tokens a block) they were equal.
+// 2048 tokens: 77 us (125 with 32 tokens a block, 124 with two outputs per register pair and the two-wide multiply-add).
+// The block of the last outputs, when it has only one (E + 1 = 257), takes it warp by warp.
+// select (expert parallelism): the last block of a token tile selects the experts of its tokens; otherwise a kernel of its own does,
+// with a warp per token on all SMs instead of eight tokens per warp on the last one. grid (ceil((E + 1) / 16), ceil(T / 64)); I = 2048.
+constexpr int RG2_TM = 64, RG2_TN = 16, RG2_KC = 128, RG2_ST = 4;
 template <typename WT> constexpr int rg2_stage_bytes() { return RG2_TM * RG2_KC * 4 + RG2_TN * RG2_KC * (int)sizeof(WT); }
 template <typename WT, int NJ>
-__global__ void __launch_bounds__(256, 2) route_gemm2_k(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int E, int K,
-                                                     int norm, int T, int* __restrict__ done, const TopkOut o) {
+__global__ void __launch_bounds__(256, 1) route_gemm2_k(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int E, int K,
+                                                     int norm, int T, int* __restrict__ done, const TopkOut o, int select) {
     constexpr int I = EH, NCH = I / RG2_KC, STAGE = rg2_stage_bytes<WT>();
-    extern __shared__ __align__(16) uint8_t rsm[];   // 2 stages x ([32 tokens][512] f32 | [16 outputs][512] WT)
+    extern __shared__ __align__(16) uint8_t rsm[];   // stages of [64 tokens][128] f32 | [16 outputs][128] WT
     const int O = E + 1, r0 = blockIdx.y * RG2_TM, o0 = blockIdx.x * RG2_TN;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp >> 1, wn = warp & 1;
-    auto fill_w = [&](int ch) {
-        uint8_t* ws = rsm + (ch & 1) * STAGE + RG2_TM * RG2_KC * 4;
-        constexpr int PER_ROW = RG2_KC * (int)sizeof(WT) / 16;   // 16-byte pieces per row chunk
-        for (int i = tid; i < RG2_TN * PER_ROW; i += 256) {
-            const int r = i / PER_ROW, c = i % PER_ROW;
-            cp_async16(smem_u32(ws + (size_t)i * 16), reinterpret_cast<const uint8_t*>(W + (size_t)min(o0 + r, O - 1) * I + ch * RG2_KC) + c * 16);
+    if (O - o0 == 1) {
+        pdl_wait();
+        pdl_trigger();
+        const WT* wr = W + (size_t)o0 * I;
+        for (int r = r0 + warp; r < min(r0 + RG2_TM, T); r += 8) {
+            float acc = 0.f;
+#pragma unroll 8
+            for (int c = 0; c < I / 128; c++) {
+                const float4 w = ld_w4(wr, (size_t)128 * c + 4 * lane), v = __ldg(reinterpret_cast<const float4*>(x + (size_t)r * I + 128 * c + 4 * lane));
+                acc = fmaf(w.x, v.x, acc); acc = fmaf(w.y, v.y, acc); acc = fmaf(w.z, v.z, acc); acc = fmaf(w.w, v.w, acc);
+            }
+            acc = warp_sum(acc);
+            if (lane == 0) y[(size_t)r * O + o0] = acc;
         }
-    };
-    auto fill_x = [&](int ch) {
-        uint8_t* xs = rsm + (ch & 1) * STAGE;
-        constexpr int PER_ROW = RG2_KC * 4 / 16;
-        for (int i = tid; i < RG2_TM * PER_ROW; i += 256) {
-            const int r = i / PER_ROW, c = i % PER_ROW;
-            cp_async16(smem_u32(xs + (size_t)i * 16), reinterpret_cast<const uint8_t*>(x + (size_t)min(r0 + r, T - 1) * I + ch * RG2_KC) + c * 16);
-        }
-    };
-    fill_w(0);   // weights do not depend on the kernel before this one
-    pdl_wait();
-    pdl_trigger();
-    fill_x(0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    float acc[8][8];
+    } else {
+        // thread: 16-byte piece tid % 32 of token rows tid / 32 + 8i; for the weights piece and row by PW pieces a row
+        constexpr int PW = RG2_KC * (int)sizeof(WT) / 16;
+        const float* xp[8]; const WT* wp[RG2_TN * PW / 256];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+        for (int i = 0; i < 8; i++) xp[i] = x + (size_t)min(r0 + (tid >> 5) + 8 * i, T - 1) * I + 4 * (tid & 31);
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-    for (int ch = 0; ch < NCH; ch++) {
-        if (ch + 1 < NCH) { fill_w(ch + 1); fill_x(ch + 1); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        const float* xs = reinterpret_cast<const float*>(rsm + (ch & 1) * STAGE) + (size_t)(8 * wm) * RG2_KC;
-        const WT* ws = reinterpret_cast<const WT*>(rsm + (ch & 1) * STAGE + RG2_TM * RG2_KC * 4) + (size_t)(8 * wn) * RG2_KC;
+        for (int i = 0; i < RG2_TN * PW / 256; i++) { const int u = tid + 256 * i; wp[i] = W + (size_t)min(o0 + u / PW, O - 1) * I + (u % PW) * (16 / (int)sizeof(WT)); }
+        auto fill_w = [&](int ch) {
+            const uint32_t ws = smem_u32(rsm + (ch % RG2_ST) * STAGE + RG2_TM * RG2_KC * 4) + 16 * tid;
 #pragma unroll
-        for (int c = 0; c < RG2_KC / 128; c++) {
-            float4 wv[8];
+            for (int i = 0; i < RG2_TN * PW / 256; i++) cp_async16(ws + 4096 * i, wp[i] + ch * RG2_KC);
+        };
+        auto fill_x = [&](int ch) {
+            const uint32_t xs = smem_u32(rsm + (ch % RG2_ST) * STAGE) + 16 * tid;
+#pragma unroll
+            for (int i = 0; i < 8; i++) cp_async16(xs + 4096 * i, xp[i] + ch * RG2_KC);
+        };
+        for (int ch = 0; ch < RG2_ST - 1; ch++) fill_w(ch);   // weights do not depend on the kernel before this one
+        pdl_wait();
+        pdl_trigger();
+        for (int ch = 0; ch < RG2_ST - 1; ch++) { fill_x(ch); asm volatile("cp.async.commit_group;" ::: "memory"); }
+        float acc[128];
+#pragma unroll
+        for (int i = 0; i < 128; i++) acc[i] = 0.f;
+#pragma unroll 1
+        for (int ch = 0; ch < NCH; ch++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(RG2_ST - 2) : "memory");
+            __syncthreads();   // chunk ch is in, and every warp is done with the stage that is filled next
+            if (ch + RG2_ST - 1 < NCH) { fill_w(ch + RG2_ST - 1); fill_x(ch + RG2_ST - 1); }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            const float* xs = reinterpret_cast<const float*>(rsm + (ch % RG2_ST) * STAGE) + (size_t)(16 * wm) * RG2_KC + 4 * lane;
+            const WT* ws = reinterpret_cast<const WT*>(rsm + (ch % RG2_ST) * STAGE + RG2_TM * RG2_KC * 4) + (size_t)(8 * wn) * RG2_KC + 4 * lane;
+            float4 wv[8], v[2];
+            v[0] = *reinterpret_cast<const float4*>(xs);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                if constexpr (sizeof(WT) == 4) wv[j] = *reinterpret_cast<const float4*>(ws + (size_t)j * RG2_KC + 128 * c + 4 * lane);
+                if constexpr (sizeof(WT) == 4) wv[j] = *reinterpret_cast<const float4*>(ws + (size_t)j * RG2_KC);
                 else {
-                    const uint2 h = *reinterpret_cast<const uint2*>(ws + (size_t)j * RG2_KC + 128 * c + 4 * lane);
+                    const uint2 h = *reinterpret_cast<const uint2*>(ws + (size_t)j * RG2_KC);
                     const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), q = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
                     wv[j] = make_float4(p.x, p.y, q.x, q.y);
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const float4 v = *reinterpret_cast<const float4*>(xs + (size_t)i * RG2_KC + 128 * c + 4 * lane);
+            for (int i = 0; i < 16; i++) {
+                if (i + 1 < 16) v[(i + 1) & 1] = *reinterpret_cast<const float4*>(xs + (size_t)(i + 1) * RG2_KC);
+                const float4 u = v[i & 1];
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    float a = acc[i][j];
-                    a = fmaf(wv[j].x, v.x, a); a = fmaf(wv[j].y, v.y, a); a = fmaf(wv[j].z, v.z, a); a = fmaf(wv[j].w, v.w, a);
-                    acc[i][j] = a;
-                }
+                for (int j = 0; j < 8; j++) acc[8 * i + j] = fmaf(wv[j].x, u.x, acc[8 * i + j]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[8 * i + j] = fmaf(wv[j].y, u.y, acc[8 * i + j]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[8 * i + j] = fmaf(wv[j].z, u.z, acc[8 * i + j]);
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[8 * i + j] = fmaf(wv[j].w, u.w, acc[8 * i + j]);
             }
         }
-        __syncthreads();   // the stage is refilled by the copies of chunk ch + 2
+        warp_sums<128>(acc, lane);
+        const int r = r0 + 16 * wm + (lane >> 1), oo = o0 + 8 * wn + 4 * (lane & 1);
+        if (r < T)
+#pragma unroll
+            for (int k = 0; k < 4; k++) if (oo + k < O) y[(size_t)r * O + oo + k] = acc[k];
     }
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float sum = warp_sum(acc[i][j]);
-            const int r = r0 + 8 * wm + i, oo = o0 + 8 * wn + j;
-            if (lane == 0 && r < T && oo < O) y[(size_t)r * O + oo] = sum;
-        }
-    if (!last_block_done(done + blockIdx.y, gridDim.x)) return;
+    if (!select || !last_block_done(done + blockIdx.y, gridDim.x)) return;
     for (int r = warp; r < RG2_TM && r0 + r < T; r += 8) topk_token<NJ, true>(y + (size_t)(r0 + r) * O, r0 + r, E, K, norm, lane, o);
     ep_raise_dispatch_flags(o, r0, min(RG2_TM, T - r0));
 }
