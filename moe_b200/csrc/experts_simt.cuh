@@ -228,40 +228,6 @@ __global__ void __launch_bounds__(WARPS * 32) shared_down_k(const uint8_t* __res
 
 // ---- glue of the layer-level calls ------------------------------------------------------------------------------------
 
-__global__ void bf16_to_f32_k(const __nv_bfloat16* __restrict__ in, float* __restrict__ out, size_t n) {
-    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    if (i < n) {
-        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(in + i));
-        out[i] = v.x; out[i + 1] = v.y;
-    }
-}
-
-// y = x / sqrt(mean(x^2) + eps), unit weight (kernels.cuh:48-64 with w = 0). One block of 256 per row; D % 4 == 0.
-// The sum of squares has a pinned order (thread i takes elements 4i..4i+3, 1024+4i.., with fused multiply-adds; a
-// xor-butterfly per warp; the 8 warp sums added in order) and the square root and divisions are IEEE, so the CPU
-// oracle reproduces the normalised row bit for bit and a chained stack routes identically on both sides.
-__global__ void __launch_bounds__(256) rmsnorm_rows_k(const float* __restrict__ x, float* __restrict__ y, int D, float eps) {
-    __shared__ float part[8];
-    const float* xr = x + (size_t)blockIdx.x * D;
-    float ss = 0.f;
-    for (int i = threadIdx.x * 4; i < D; i += 1024) {
-        const float4 v = *reinterpret_cast<const float4*>(xr + i);
-        ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
-    }
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) tot += part[i];
-    const float r = 1.f / sqrtf(tot / (float)D + eps);
-    for (int i = threadIdx.x * 4; i < D; i += 1024) {
-        float4 v = *reinterpret_cast<const float4*>(xr + i);
-        v.x *= r; v.y *= r; v.z *= r; v.w *= r;
-        *reinterpret_cast<float4*>(y + (size_t)blockIdx.x * D + i) = v;
-    }
-}
-
 // out = x + moe (the residual add the reference folds into the next layer's RMSNorm, moex.cu:1082)
 __global__ void residual_add_k(const float* __restrict__ x, const float* __restrict__ moe, float* __restrict__ out, size_t n) {
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;

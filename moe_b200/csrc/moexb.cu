@@ -266,7 +266,7 @@ static int decode_launch(moexb_ctx* prof, int fmt, const uint8_t* const* slots, 
 static std::mutex g_default_lock;
 static moexb_ctx* g_default_ctx[MAX_DEVICES] = {};
 static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, void* stream);
-static int split_launch(moexb_ctx* c, const float* x, int rows, bool f16, void* stream, const SidePlan* plan = nullptr);
+static int split_launch(moexb_ctx* c, const float* x, int rows, void* stream, const SidePlan& plan);
 
 extern "C" {
 
@@ -294,7 +294,7 @@ int moexb_experts_forward(int fmt, const uint8_t* const* slots, const float* w, 
     cudaStream_t st = S(stream);
     SidePlan plan{};
     plan.slots = slots; plan.w = w; plan.K = K; plan.nh = nh; plan.subs = c->subs; plan.pairs = c->pairs; plan.nsub = c->nsub;
-    int rc = split_launch(c, x, 1, false, stream, &plan);
+    int rc = split_launch(c, x, 1, stream, plan);
     if (rc != MOEXB_OK) return rc;
     if (nh) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)K * EH * sizeof(float), st));   // rows of the experts beyond *nh stay zero
     rc = stream_experts(c, fmt, c->pairs, act, c->ypair, stream);
@@ -1070,15 +1070,6 @@ static int grouped_min_tokens(const moexb_ctx* c, int fmt) { return c->prefill_m
 // Pairs per tile of the grouped GEMM.
 static int grouped_maxp(int fmt) { return fmt == FMT_ZP ? gg_nmax<FMT_ZP>() : gg_nmax<FMT_SYM_F16>(); }
 
-// The activations as the grouped GEMM's rows, into the context. parts = 1 when x holds exact bf16 values, else 2.
-static int grouped_rows(moexb_ctx* c, int fmt, const float* x, uint16_t* xs, int rows, int parts, void* stream) {
-    PROF(c, MOEXB_PROF_OTHER, stream);
-    if (fmt == FMT_ZP) grouped_rows_k<true><<<rows, 256, 0, S(stream)>>>(x, xs, c->sx, parts);
-    else grouped_rows_k<false><<<rows, 256, 0, S(stream)>>>(x, xs, nullptr, parts);
-    LAUNCHED("grouped_rows");
-    return MOEXB_OK;
-}
-
 // Experts of a large batch on the tensor-core grouped GEMM: the tiles are in the context (subs, nsub) or in the buckets, and grouped_rows or
 // the token owners (expert parallelism) left the activation rows.
 static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int parts, float* ypair, void* stream, const BucketArgs* buckets = nullptr) {
@@ -1091,13 +1082,33 @@ static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int p
     });
 }
 
-// f16: the consumer is the tiled kernel of a symmetric format (fp16 operands); otherwise bf16. plan: made on the side by one more block.
-static int split_launch(moexb_ctx* c, const float* x, int rows, bool f16, void* stream, const SidePlan* plan) {
+// The bf16 split of f32 rows into the context; plan: made on the side by one more block.
+static int split_launch(moexb_ctx* c, const float* x, int rows, void* stream, const SidePlan& plan) {
     PROF(c, MOEXB_PROF_OTHER, stream);
-    const SidePlan p = plan ? *plan : SidePlan{};
-    CUDA_TRY(launch_dep(f16 ? split_rows_k<true> : split_rows_k<false>, rows + (plan ? 1 : 0), 256, 0, S(stream), x, c->xs, rows, p));
+    CUDA_TRY(launch_dep(split_rows_k, rows + 1, 256, 0, S(stream), x, c->xs, rows, plan));
     LAUNCHED("split_rows");
     return MOEXB_OK;
+}
+
+// What a layer makes of its input rows (layer_rows_k): xf = bf16 rows widened, xn = their rmsnorm (norm), xs = the split of either.
+static int layer_rows(moexb_ctx* c, const void* X, int x_dtype, int rows, float* xf, bool norm, float* xn, int mode, uint16_t* xs, int parts, void* stream) {
+    PROF(c, MOEXB_PROF_OTHER, stream);
+    auto run = [&]<typename XT, bool NORM, int MODE>() -> int {
+        CUDA_TRY(launch_dep(layer_rows_k<XT, NORM, MODE>, rows, 256, 0, S(stream), static_cast<const XT*>(X), xf, xn, xs, c->sx, parts, 1e-6f));
+        LAUNCHED("layer_rows");
+        return MOEXB_OK;
+    };
+    auto by_mode = [&]<typename XT, bool NORM>() -> int {
+        switch (mode) {
+            case ROWS_F16: return run.template operator()<XT, NORM, ROWS_F16>();
+            case ROWS_BF16: return run.template operator()<XT, NORM, ROWS_BF16>();
+            case ROWS_GEMM: return run.template operator()<XT, NORM, ROWS_GEMM>();
+            case ROWS_GEMM_Z: return run.template operator()<XT, NORM, ROWS_GEMM_Z>();
+        }
+        return run.template operator()<XT, NORM, ROWS_NONE>();
+    };
+    if (x_dtype == MOEXB_BF16) return norm ? by_mode.template operator()<__nv_bfloat16, true>() : by_mode.template operator()<__nv_bfloat16, false>();
+    return norm ? by_mode.template operator()<float, true>() : by_mode.template operator()<float, false>();
 }
 
 extern "C" int moexb_pairs_forward_tc(moexb_ctx* c, int fmt, const moexb_pair_item* items, int n_items, const moexb_pair* pairs,
@@ -1110,7 +1121,7 @@ extern "C" int moexb_pairs_forward_tc(moexb_ctx* c, int fmt, const moexb_pair_it
     if (n_items == 0) return MOEXB_OK;
     SidePlan plan{};
     plan.items = items; plan.n_items = n_items; plan.maxp = ST_MAXP; plan.subs = c->subs; plan.nsub = c->nsub;
-    int rc = split_launch(c, X, T, false, stream, &plan);
+    int rc = split_launch(c, X, T, stream, plan);
     if (rc != MOEXB_OK) return rc;
     return stream_experts(c, fmt, pairs, act, ypair, stream);
 }
@@ -1176,9 +1187,13 @@ extern "C" {
 // Router logits (into the context, [T][E + 1]) and the top-K selection in one launch; decode: also the K + 1 one-pair
 // sub-items of a single token.
 struct RouteEp { const EpDevice* dev; int row_bytes; unsigned phase; const unsigned* step; };
-struct RouteOut { bool buckets, shared; int* idx; float* w; };   // pairs into the buckets (with the shared expert's); the caller's copies
+// pairs into the buckets (with the shared expert's); the caller's copies of ids and weights; split: the rows of x (x_dtype) are split by
+// the routing kernel (ROWS_F16, ROWS_BF16; only where route_splits)
+struct RouteOut { bool buckets = false, shared = false; int* idx = nullptr; float* w = nullptr; int x_dtype = MOEXB_F32, split = ROWS_NONE; };
+static bool route_splits(int T) { return T < 8; }
 template <typename WT>
-static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
+static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
+    const float* xf = static_cast<const float*>(x);
     // tok0: the T rows at xf are tokens tok0.. of the batch - their logits, ids and weights go to those rows of the workspace
     const int E = L->n_routed;
     const WT* W = static_cast<const WT*>(L->router);
@@ -1196,7 +1211,11 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, in
         // done by a block of their own instead of one block sending a whole tile of 8
         if (T < 8 || (rep && T <= 16)) {
             constexpr int WARPS = 8;
-            CUDA_TRY(launch_dep(route_gemv_k<WT, WARPS, NJ>, dim3((E + 1 + WARPS - 1) / WARPS, T), WARPS * 32, 0, S(stream), W, xf, logits, EH, E, K, 1, c->route_done, o));
+            const dim3 grid((E + 1 + WARPS - 1) / WARPS + (ro.split ? 1 : 0), T);
+            uint16_t* xs = ro.split ? c->xs : nullptr;
+            if (ro.x_dtype == MOEXB_BF16)
+                CUDA_TRY(launch_dep(route_gemv_k<WT, __nv_bfloat16, WARPS, NJ>, grid, WARPS * 32, 0, S(stream), W, static_cast<const __nv_bfloat16*>(x), logits, EH, E, K, 1, c->route_done, o, xs, ro.split));
+            else CUDA_TRY(launch_dep(route_gemv_k<WT, float, WARPS, NJ>, grid, WARPS * 32, 0, S(stream), W, xf, logits, EH, E, K, 1, c->route_done, o, xs, ro.split));
         } else {
             // 16 outputs per block spread a small batch over more SMs; a prefill chunk has blocks to spare and re-reads
             // the router weights less with 32 outputs per block
@@ -1234,18 +1253,18 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const float* xf, int T, in
 }
 
 extern "C" {
-static int layer_route(moexb_ctx* c, moexb_layer* L, const float* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
+static int layer_route(moexb_ctx* c, moexb_layer* L, const void* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
     PROF(c, MOEXB_PROF_ROUTER, stream);
     return L->router_dtype == MOEXB_F32 ? route_launch<float>(c, L, xf, T, K, stream, decode, ro, tok0, rep) : route_launch<__half>(c, L, xf, T, K, stream, decode, ro, tok0, rep);
 }
 
-// One layer. xin: the layer input as f32 [T][H]. flags as moexb_layer_forward. pre_normed: the context already holds
-// rmsnorm(xin) and its bf16 split (left there by the previous layer of a stack); next_norm: leave rmsnorm(out) and its
+// One layer. X: the layer input [T][H] of x_dtype. flags as moexb_layer_forward. pre_normed: the context already holds
+// rmsnorm(X) and its split (left there by the previous layer of a stack); next_norm: leave rmsnorm(out) and its
 // split in the context for the next layer.
-static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int K, float* out, int* idx_out, float* w_out, int flags,
-                      void* stream, bool pre_normed, bool next_norm, int sh0 = 0, int sh1 = -1, bool x_bf16 = false) {
+static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, int T, int K, float* out, int* idx_out, float* w_out, int flags,
+                      void* stream, bool pre_normed, bool next_norm, int sh0 = 0, int sh1 = -1) {
     if (sh1 < 0) sh1 = T;
-    const bool shared = !(flags & 1) && sh1 > sh0, block = flags & 2, partial = flags & 4;
+    const bool shared = !(flags & 1) && sh1 > sh0, block = flags & 2, partial = flags & 4, bf16 = x_dtype == MOEXB_BF16;
     const bool all_local = L->n_local == L->n_routed;
     const int E = L->n_routed, ld = E + 1;
     cudaStream_t st = S(stream);
@@ -1254,22 +1273,27 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
     // large batches go to the tcgen05 grouped GEMM; the rest to the streaming kernels
     const bool prefill = tiled && T >= grouped_min_tokens(c, L->fmt);
     const bool f16 = tiled && L->fmt != FMT_ZP && !prefill;  // element type of the split activations the streaming kernels read
-    const float* xf = xin;  // what the router and the experts see
+    const int parts = prefill && bf16 && !block ? 1 : 2;
+    const int mode = !streaming ? ROWS_NONE : prefill ? (L->fmt == FMT_ZP ? ROWS_GEMM_Z : ROWS_GEMM) : f16 ? ROWS_F16 : ROWS_BF16;
+    // xin: the input as f32 (for the residual and the fp32 kernels); xr: what the router sees, of xr_dtype
+    const float* xin = bf16 ? c->xf : static_cast<const float*>(X);
+    const void* xr = xin;
+    RouteOut ro;
+    int rc = MOEXB_OK;
     if (block) {
-        xf = c->xn;
-        if (!pre_normed) {
-            PROF(c, MOEXB_PROF_OTHER, stream);
-            if (f16) rmsnorm_split_k<true><<<T, 256, 0, st>>>(xin, c->xn, c->xs, 1e-6f);
-            else rmsnorm_split_k<false><<<T, 256, 0, st>>>(xin, c->xn, prefill ? nullptr : c->xs, 1e-6f);
-            LAUNCHED("rmsnorm_split");
-        }
-    } else if (streaming && !prefill) {
-        const int rc = split_launch(c, xf, T, f16, stream);
-        if (rc != MOEXB_OK) return rc;
-    }
+        xr = c->xn;
+        if (!pre_normed || prefill) {   // (the previous layer leaves no rows for the grouped GEMM)
+            rc = layer_rows(c, X, x_dtype, T, c->xf, true, c->xn, mode, c->xs, parts, stream);
+        } else if (bf16) rc = layer_rows(c, X, x_dtype, T, c->xf, false, nullptr, ROWS_NONE, nullptr, 2, stream);
+    } else if (streaming && !prefill && route_splits(T)) {
+        xr = X; ro.x_dtype = x_dtype; ro.split = mode;
+    } else if (mode != ROWS_NONE || bf16) rc = layer_rows(c, X, x_dtype, T, c->xf, false, nullptr, mode, c->xs, parts, stream);
+    if (rc != MOEXB_OK) return rc;
+    const float* xf = block ? c->xn : xin;   // what the router and the experts see, as f32
     const bool decode = T == 1 && all_local && shared && !partial && !prefill;
     const bool buckets = tiled && !decode && c->bpairs;
-    int rc = layer_route(c, L, xf, T, K, stream, decode, RouteOut{buckets, buckets && shared, idx_out, w_out});
+    ro.buckets = buckets; ro.shared = buckets && shared; ro.idx = idx_out; ro.w = w_out;
+    rc = layer_route(c, L, xr, T, K, stream, decode, ro);
     if (rc != MOEXB_OK) return rc;
     int ranks = K;                  // rows of ypair per token that the final reduction adds
     const float* extra = nullptr;   // + the shared expert's rows
@@ -1282,7 +1306,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
             PROF(c, MOEXB_PROF_COMBINE, stream);
             residual_add_k<<<(unsigned)((EH / 4 + 255) / 256), 256, 0, st>>>(xin, c->moe, out, EH);
             LAUNCHED("residual_add");
-            if (next_norm) { rmsnorm_split_k<false><<<1, 256, 0, st>>>(out, c->xn, c->xs, 1e-6f); LAUNCHED("rmsnorm_split"); }
+            if (next_norm) { rc = layer_rows(c, out, MOEXB_F32, 1, nullptr, true, c->xn, ROWS_BF16, c->xs, 2, stream); if (rc != MOEXB_OK) return rc; }
         }
         ranks = 0;
     } else if (decode) {
@@ -1290,7 +1314,6 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
         if (rc != MOEXB_OK) return rc;
         ranks = K + 1;
     } else {
-        const int parts = (x_bf16 && !block) ? 1 : 2;
         const int maxp = prefill ? grouped_maxp(L->fmt) : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
         const BucketArgs bk{c->bcnt, c->bpairs, c->max_tokens, E, shared ? sh0 : 0, shared ? sh1 : 0, maxp, L->slot_table};
         if (!buckets) {
@@ -1307,10 +1330,6 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
             // pairs of experts that are not held here are never written: the SIMT reduction path needs zeros there, the fused
             // reduction skips them by expert id
             if (!all_local && !streaming) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)T * K * EH * sizeof(float), st));
-        }
-        if (prefill) {
-            rc = grouped_rows(c, L->fmt, xf, c->xs, T, parts, stream);
-            if (rc != MOEXB_OK) return rc;
         }
         rc = prefill ? grouped_experts(c, L->fmt, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
            : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr)
@@ -1331,18 +1350,6 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const float* xin, int T, int
     return MOEXB_OK;
 }
 
-// The layer input as f32: bf16 inputs are widened (exactly) into the context.
-static int layer_input(moexb_ctx* c, const void* X, int x_dtype, int T, void* stream, const float** xin) {
-    if (x_dtype == MOEXB_BF16) {
-        PROF(c, MOEXB_PROF_OTHER, stream);
-        const size_t n = (size_t)T * EH;
-        bf16_to_f32_k<<<(unsigned)((n / 2 + 255) / 256), 256, 0, S(stream)>>>(static_cast<const __nv_bfloat16*>(X), c->xf, n);
-        LAUNCHED("bf16_to_f32");
-        *xin = c->xf;
-    } else *xin = static_cast<const float*>(X);
-    return MOEXB_OK;
-}
-
 int moexb_layer_forward(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, int T, int K, float* out, int* idx_out,
                         float* w_out, int flags, void* stream) {
     REQUIRE(c && L && X && out, "layer_forward: null pointer");
@@ -1351,10 +1358,7 @@ int moexb_layer_forward(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype
     REQUIRE(K > 0 && K <= c->top_k, "layer_forward: K=%d exceeds the context's top_k=%d", K, c->top_k);
     REQUIRE(x_dtype == MOEXB_F32 || x_dtype == MOEXB_BF16, "layer_forward: x_dtype=%d", x_dtype);
     REQUIRE((flags & 1) || L->loaded[L->n_routed], "layer_forward: the shared expert of this layer was never loaded (upload it, or pass flags bit 0 to leave it out)");
-    const float* xin;
-    int rc = layer_input(c, X, x_dtype, T, stream, &xin);
-    if (rc != MOEXB_OK) return rc;
-    return layer_impl(c, L, xin, T, K, out, idx_out, w_out, flags, stream, false, false, 0, -1, x_dtype == MOEXB_BF16);
+    return layer_impl(c, L, X, x_dtype, T, K, out, idx_out, w_out, flags, stream, false, false);
 }
 
 int moexb_layer_forward_ep(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, int T, int K, float* out, int* idx_out,
@@ -1366,10 +1370,7 @@ int moexb_layer_forward_ep(moexb_ctx* c, moexb_layer* L, const void* X, int x_dt
     REQUIRE(x_dtype == MOEXB_F32 || x_dtype == MOEXB_BF16, "layer_forward_ep: x_dtype=%d", x_dtype);
     REQUIRE(shared_t0 >= 0 && shared_t0 <= shared_t1 && shared_t1 <= T, "layer_forward_ep: shared token range [%d, %d) outside 0..%d", shared_t0, shared_t1, T);
     REQUIRE(shared_t0 == shared_t1 || L->loaded[L->n_routed], "layer_forward_ep: the shared expert of this layer was never loaded");
-    const float* xin;
-    int rc = layer_input(c, X, x_dtype, T, stream, &xin);
-    if (rc != MOEXB_OK) return rc;
-    return layer_impl(c, L, xin, T, K, out, idx_out, w_out, 2 | 4, stream, pre_normed != 0, false, shared_t0, shared_t1);
+    return layer_impl(c, L, X, x_dtype, T, K, out, idx_out, w_out, 2 | 4, stream, pre_normed != 0, false, shared_t0, shared_t1);
 }
 
 int moexb_ep_residual_norm(moexb_ctx* c, moexb_layer* next, const float* x, const float* total, float* out, int T, void* stream) {
@@ -1488,12 +1489,13 @@ int moexb_stack_create(moexb_ctx* c, moexb_layer* const* layers, int n_layers, i
     const long long before = g_launches.load();
     e = cudaStreamBeginCapture(s->cap, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) { moexb_stack_destroy(s); return fail(MOEXB_ERR_CUDA, "stack_create: begin capture: %s", cudaGetErrorString(e)); }
-    const float* xin = nullptr;
-    int rc = layer_input(c, s->x_in, x_dtype, T, s->cap, &xin);
+    const void* xin = s->x_in;
+    int rc = MOEXB_OK;
     for (int l = 0; l < n_layers && rc == MOEXB_OK; l++) {
         // layer l leaves rmsnorm(x_{l+1}) and its split in the context, so layer l+1 starts at its router
-        if (residual) rc = layer_impl(c, layers[l], xin, T, K, s->buf[l & 1], nullptr, nullptr, 2, s->cap, l > 0, l + 1 < n_layers);
-        else rc = layer_impl(c, layers[l], xin, T, K, s->buf[l & 1], nullptr, nullptr, 0, s->cap, false, false, 0, -1, l == 0 && x_dtype == MOEXB_BF16);
+        const int dt = l ? MOEXB_F32 : x_dtype;
+        if (residual) rc = layer_impl(c, layers[l], xin, dt, T, K, s->buf[l & 1], nullptr, nullptr, 2, s->cap, l > 0, l + 1 < n_layers);
+        else rc = layer_impl(c, layers[l], xin, dt, T, K, s->buf[l & 1], nullptr, nullptr, 0, s->cap, false, false);
         xin = s->buf[l & 1];
     }
     e = cudaStreamEndCapture(s->cap, &s->graph);
@@ -1704,36 +1706,24 @@ int moexb_ep_dispatch(moexb_ep* e, moexb_layer* L, int l, const void* X, int x_d
     // activation columns per token: the grouped GEMM takes one when the layer input is exactly bf16, else hi + lo
     const int parts = prefill && x_dtype == MOEXB_BF16 && !residual && l == 0 ? 1 : 2;
     e->prefill = prefill; e->parts = parts;
+    const int mode = prefill ? ROWS_GEMM : f16 ? ROWS_F16 : ROWS_BF16;
     float* xn_own = c->xn + (size_t)t0 * EH;
     if (l == 0) {
-        // the own rows of the input as fp32: into the residual rows (blocks) or straight into the layer input (plain layers)
+        // the own rows of the input as fp32 into the residual rows (blocks) or straight into the layer input (plain layers), with the
+        // norm and the split in the same pass
         float* dst = residual ? e->x : xn_own;
         const size_t n = (size_t)n_own * EH;
-        PROF(c, MOEXB_PROF_OTHER, stream);
-        if (x_dtype == MOEXB_BF16) {
-            bf16_to_f32_k<<<(unsigned)((n / 2 + 255) / 256), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(X) + (size_t)t0 * EH, dst, n);
-            LAUNCHED("bf16_to_f32");
-        } else CUDA_TRY(cudaMemcpyAsync(dst, static_cast<const float*>(X) + (size_t)t0 * EH, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
-        if (residual && !prefill) {
-            if (f16) rmsnorm_split_k<true><<<n_own, 256, 0, st>>>(e->x, xn_own, c->xs + (size_t)t0 * 2 * EH, 1e-6f);
-            else rmsnorm_split_k<false><<<n_own, 256, 0, st>>>(e->x, xn_own, c->xs + (size_t)t0 * 2 * EH, 1e-6f);
-            LAUNCHED("rmsnorm_split");
-        } else if (residual) {
-            rmsnorm_rows_k<<<n_own, 256, 0, st>>>(e->x, xn_own, EH, 1e-6f);
-            LAUNCHED("rmsnorm_rows");
-        } else if (!prefill) {
-            if (f16) split_rows_k<true><<<n_own, 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * 2 * EH, n_own, SidePlan{});
-            else split_rows_k<false><<<n_own, 256, 0, st>>>(xn_own, c->xs + (size_t)t0 * 2 * EH, n_own, SidePlan{});
-            LAUNCHED("split_rows");
-        }
+        const uint8_t* own = static_cast<const uint8_t*>(X) + (size_t)t0 * EH * (x_dtype == MOEXB_BF16 ? 2 : 4);
+        if (x_dtype == MOEXB_F32) CUDA_TRY(cudaMemcpyAsync(dst, own, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        rc = layer_rows(c, own, x_dtype, n_own, dst, residual != 0, xn_own, mode, c->xs + (size_t)t0 * parts * EH, parts, stream);
+        if (rc != MOEXB_OK) return rc;
     } else {
         rc = ep_combine(e, f16, residual != 0, (unsigned)l, nullptr, true, !prefill, stream);
         if (rc != MOEXB_OK) return rc;
-    }
-    if (prefill) {
-        PROF(c, MOEXB_PROF_OTHER, stream);
-        rc = grouped_rows(c, L->fmt, xn_own, c->xs + (size_t)t0 * parts * EH, n_own, parts, stream);
-        if (rc != MOEXB_OK) return rc;
+        if (prefill) {
+            rc = layer_rows(c, xn_own, MOEXB_F32, n_own, nullptr, false, nullptr, mode, c->xs + (size_t)t0 * parts * EH, parts, stream);
+            if (rc != MOEXB_OK) return rc;
+        }
     }
     // the routing kernel sends each token to the peers as soon as its experts are selected and raises the tokens' flags
     const RouteEp rep{e->dev, parts * EH * 2, (unsigned)(l + 1), e->step};

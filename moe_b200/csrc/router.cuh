@@ -1,6 +1,7 @@
 // Router kernels: logits in a pinned fp32 summation order, softmax + top-K selection, pair grouping by expert.
 #pragma once
 #include "common.cuh"
+#include "rows.cuh"
 
 namespace moexb {
 
@@ -302,12 +303,15 @@ __device__ __forceinline__ bool last_block_done(int* cnt, int expected) {
 // Router logits and top-K selection of a few tokens in one launch: gemv_rows_k's grid (ceil(O / WARPS) blocks per
 // token, O = E + 1), and the last block of a token to finish selects that token's experts - no second launch, no wait:
 // the block that comes last simply does the extra work. done[t] must be zero before the first launch.
-template <typename WT, int WARPS, int NJ>
-__global__ void __launch_bounds__(WARPS * 32) route_gemv_k(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int I,
-                                                           int E, int K, int norm, int* __restrict__ done, const TopkOut o) {
+// x: f32 or bf16 rows. xs (a layer without a norm before it): one block more per token splits the token's row for the experts,
+// instead of a launch before this one (mode: ROWS_F16 or ROWS_BF16).
+template <typename WT, typename XT, int WARPS, int NJ>
+__global__ void __launch_bounds__(WARPS * 32) route_gemv_k(const WT* __restrict__ W, const XT* __restrict__ x, float* __restrict__ y, int I,
+                                                           int E, int K, int norm, int* __restrict__ done, const TopkOut o, uint16_t* __restrict__ xs, int mode) {
+    static_assert(WARPS == 8, "256 threads split a row");
     const int O = E + 1, t = blockIdx.y;
     const int out = blockIdx.x * WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const float* xr = x + (size_t)t * I;
+    const XT* xr = x + (size_t)t * I;
     const WT* wr = W + (size_t)min(out, O - 1) * I;
     float acc = 0.f;
     constexpr int U = 16;
@@ -315,12 +319,23 @@ __global__ void __launch_bounds__(WARPS * 32) route_gemv_k(const WT* __restrict_
         float4 v[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (c0 + u < I / 128) v[u] = __ldg(reinterpret_cast<const float4*>(xr + 128 * (c0 + u) + 4 * lane));
+            if (c0 + u < I / 128) v[u] = ld_x4(xr + 128 * (c0 + u) + 4 * lane);
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (c0 + u < I / 128) { acc = fmaf(w[u].x, v[u].x, acc); acc = fmaf(w[u].y, v[u].y, acc); acc = fmaf(w[u].z, v[u].z, acc); acc = fmaf(w[u].w, v[u].w, acc); }
     };
-    {
+    if (xs && blockIdx.x == gridDim.x - 1) {
+        pdl_wait();
+        pdl_trigger();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int k0 = 1024 * h + 4 * threadIdx.x;
+            const float4 p = ld_x4(xr + k0);
+            const float f[4] = {p.x, p.y, p.z, p.w};
+            if (mode == ROWS_F16) store_split4<ROWS_F16>(f, k0, xs + (size_t)t * 2 * EH, EH);
+            else store_split4<ROWS_BF16>(f, k0, xs + (size_t)t * 2 * EH, EH);
+        }
+    } else {
         float4 w[U];
 #pragma unroll
         for (int u = 0; u < U; u++)

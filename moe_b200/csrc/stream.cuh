@@ -20,6 +20,7 @@
 // of both MMAs of a word are one 16-byte load per lane (see split_pos).
 #pragma once
 #include "common.cuh"
+#include "rows.cuh"
 
 namespace moexb {
 
@@ -38,12 +39,6 @@ template <int FMT, int NW> constexpr int st_slot_bytes() { return st_pieces<NW>(
 // activation columns in shared memory: 8 columns of K bf16, column stride K*2 + 64 bytes (conflict-free 16-byte reads)
 template <bool DOWN> constexpr int st_bcol_bytes() { return (DOWN ? EI : EH) * 2 + 64; }
 template <int FMT, bool DOWN, int NW, int STAGES> constexpr int st_smem_bytes() { return STAGES * st_slot_bytes<FMT, NW>() + 8 * st_bcol_bytes<DOWN>() + 256 + 8; }
-
-// Position of input k inside a permuted activation row (see the header comment).
-__host__ __device__ constexpr int split_pos(int k) {
-    const int G = k >> 6, kl = k & 63, t = kl >> 4, w = (kl >> 3) & 1, e = kl & 7;
-    return G * 64 + w * 32 + t * 8 + (((e & 3) << 1) | (e >> 2));
-}
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -101,18 +96,6 @@ __device__ __forceinline__ void dq_word_h(uint32_t q, uint32_t (&P)[4]) {
         asm("lop3.b32 %0, %1, 0x00F000F0, 0x64806480, 0x6A;" : "=r"(r1) : "r"(x));
         asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(P[2 * j]) : "r"(r0), "r"(0x64086408u));
         asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(P[2 * j + 1]) : "r"(r1), "r"(0x2C002C00u), "r"(0xD480D480u));
-    }
-}
-
-// hi + lo halves of v as 16-bit patterns: fp16 (22 significand bits together) or bf16 (16 bits, full fp32 range)
-template <bool F16>
-__device__ __forceinline__ void split_hi_lo(float v, uint16_t& hi, uint16_t& lo) {
-    if constexpr (F16) {
-        const __half h = __float2half_rn(v), l = __float2half_rn(v - __half2float(h));
-        hi = __half_as_ushort(h); lo = __half_as_ushort(l);
-    } else {
-        const __nv_bfloat16 h = __float2bfloat16_rn(v), l = __float2bfloat16_rn(v - __bfloat162float(h));
-        hi = __bfloat16_as_ushort(h); lo = __bfloat16_as_ushort(l);
     }
 }
 
@@ -382,9 +365,8 @@ __device__ __forceinline__ void side_plan(const SidePlan& p) {
     if (threadIdx.x == 0) *p.nsub = done;
 }
 
-// x [rows][H] fp32 -> xs [rows][2][H] 16-bit: hi and lo halves (see split_hi_lo), both in the permuted order of split_pos. Block r takes
+// x [rows][H] fp32 -> xs [rows][2][H] bf16: hi and lo halves (see split_hi_lo), both in the permuted order of split_pos. Block r takes
 // row r, a thread 8 consecutive inputs, whose places are 8 consecutive ones too; block `rows`, when the launch has one, plans.
-template <bool F16>
 __global__ void __launch_bounds__(256) split_rows_k(const float* __restrict__ x, uint16_t* __restrict__ xs, int rows, const SidePlan plan) {
     pdl_wait();
     pdl_trigger();
@@ -394,7 +376,7 @@ __global__ void __launch_bounds__(256) split_rows_k(const float* __restrict__ x,
     const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
     uint16_t hi[8], lo[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) split_hi_lo<F16>(v[i], hi[i], lo[i]);
+    for (int i = 0; i < 8; i++) split_hi_lo<false>(v[i], hi[i], lo[i]);
     uint16_t* dst = xs + (size_t)r * 2 * EH + split_pos(k);
     auto put = [&](uint16_t* d, const uint16_t (&w)[8]) {   // places in the order of inputs 0, 4, 1, 5, 2, 6, 3, 7
         *reinterpret_cast<uint4*>(d) = make_uint4(w[0] | (uint32_t)w[4] << 16, w[1] | (uint32_t)w[5] << 16, w[2] | (uint32_t)w[6] << 16, w[3] | (uint32_t)w[7] << 16);
@@ -403,7 +385,8 @@ __global__ void __launch_bounds__(256) split_rows_k(const float* __restrict__ x,
 }
 
 // One row of D = 2048 floats held 8 per thread (thread i: elements 4i..4i+3 and 1024+4i..1024+4i+3): the sum of squares
-// in the pinned order of rmsnorm_rows_k, then the normalised row as fp32 (for the router) and as bf16 hi + lo in the
+// in a pinned order (fused multiply-adds in element order, a xor-butterfly per warp, the 8 warp sums in order; IEEE root and division, so
+// that the CPU oracle reproduces the row bit for bit and a chained stack routes identically on both sides), then the normalised row as fp32 (for the router) and as bf16 hi + lo in the
 // permuted order (for the streaming kernels).
 // lo_off: distance (elements) from the hi row to the lo row of the split.
 // 1 / sqrt(mean(v^2) + eps) of the row, the sum of squares in the pinned order (all 256 threads of the block call it).
@@ -420,23 +403,15 @@ __device__ __forceinline__ float row_rms_scale(const float (&v)[8], float eps) {
     for (int i = 0; i < 8; i++) tot += part[i];
     return 1.f / sqrtf(tot / (float)EH + eps);
 }
-// The row times r as fp32 into xn and, when xs is given, as 16-bit hi + lo in the permuted order into xs (hi) and xs + lo_off (lo).
+// The row times r as fp32 into xn and, when xs is given, split into xs (hi) and xs + lo_off (lo).
 template <bool F16>
 __device__ __forceinline__ void scaled_split_row(const float (&v)[8], float r, float* __restrict__ xn, uint16_t* __restrict__ xs, int lo_off = EH) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int k0 = 1024 * h + 4 * threadIdx.x;
-        float4 o = make_float4(v[4 * h] * r, v[4 * h + 1] * r, v[4 * h + 2] * r, v[4 * h + 3] * r);
-        *reinterpret_cast<float4*>(xn + k0) = o;
-        if (!xs) continue;
-        const float f[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            uint16_t hi, lo;
-            split_hi_lo<F16>(f[i], hi, lo);
-            const int pos = split_pos(k0 + i);
-            xs[pos] = hi; xs[lo_off + pos] = lo;
-        }
+        const float f[4] = {v[4 * h] * r, v[4 * h + 1] * r, v[4 * h + 2] * r, v[4 * h + 3] * r};
+        *reinterpret_cast<float4*>(xn + k0) = make_float4(f[0], f[1], f[2], f[3]);
+        if (xs) store_split4<F16 ? ROWS_F16 : ROWS_BF16>(f, k0, xs, lo_off);
     }
 }
 template <bool F16>
@@ -444,14 +419,40 @@ __device__ __forceinline__ void norm_split_row(const float (&v)[8], float* __res
     scaled_split_row<F16>(v, row_rms_scale(v, eps), xn, xs, lo_off);
 }
 
-// xn[t] = rmsnorm(x[t]) and its bf16 split, one block of 256 per row (H = 2048).
-template <bool F16>
-__global__ void __launch_bounds__(256) rmsnorm_split_k(const float* __restrict__ x, float* __restrict__ xn, uint16_t* __restrict__ xs, float eps) {
+// What a layer makes of its input rows before the router and the experts, in one pass: bf16 rows widened to xf (when given), the
+// rmsnorm of the row into xn (NORM), and the row that the experts see, split (MODE) into xs; parts = 1 leaves out the lo half. sx: sums
+// of what the split row holds per 32 inputs. One block of 256 per row.
+template <typename XT, bool NORM, int MODE>
+__global__ void __launch_bounds__(256) layer_rows_k(const XT* __restrict__ x, float* __restrict__ xf, float* __restrict__ xn, uint16_t* __restrict__ xs,
+                                                    float* __restrict__ sx, int parts, float eps) {
+    pdl_wait();
+    pdl_trigger();
     const size_t t = blockIdx.x;
     float v[8];
-    const float4 a = *reinterpret_cast<const float4*>(x + t * EH + 4 * threadIdx.x), b = *reinterpret_cast<const float4*>(x + t * EH + 1024 + 4 * threadIdx.x);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    norm_split_row<F16>(v, xn + t * EH, xs ? xs + t * 2 * EH : nullptr, eps);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int k0 = 1024 * h + 4 * threadIdx.x;
+        const float4 p = ld_x4(x + t * EH + k0);
+        v[4 * h] = p.x; v[4 * h + 1] = p.y; v[4 * h + 2] = p.z; v[4 * h + 3] = p.w;
+        if (sizeof(XT) == 2 && xf) *reinterpret_cast<float4*>(xf + t * EH + k0) = p;
+    }
+    const float r = NORM ? row_rms_scale(v, eps) : 1.f;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int k0 = 1024 * h + 4 * threadIdx.x;
+        float f[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) f[i] = NORM ? v[4 * h + i] * r : v[4 * h + i];
+        if (NORM) *reinterpret_cast<float4*>(xn + t * EH + k0) = make_float4(f[0], f[1], f[2], f[3]);
+        if constexpr (MODE != ROWS_NONE) {
+            float sum = store_split4<MODE>(f, k0, xs + t * parts * EH, parts == 2 ? EH : 0);
+            if constexpr (MODE == ROWS_GEMM_Z) {   // a chunk of 32 inputs is 8 threads
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if ((threadIdx.x & 7) == 0) sx[t * (EH / 32) + (k0 >> 5)] = sum;
+            }
+        }
+    }
 }
 
 // The end of a layer in one pass over the token's row: moe[t] = sum_{r<K} ypair[t*K+r] in rank order (+ extra[t]: the
