@@ -54,6 +54,15 @@ static bool pdl_enabled() {
     static const bool on = [] { const char* e = getenv("MOEXB_PDL"); return !(e && e[0] == '0'); }();
     return on;
 }
+// The kernels of a prefill-size batch fill every SM for tens of microseconds, and blocks of the next one that wait inside take the
+// place of blocks that could run: such a batch is launched the plain way (2048 tokens: 444 us with programmatic launches, 419 without;
+// up to a few hundred tokens it is the other way round).
+static thread_local bool t_plain_launches = false;
+struct PlainLaunches {
+    const bool before = t_plain_launches;
+    explicit PlainLaunches(bool on) { t_plain_launches = on; }
+    ~PlainLaunches() { t_plain_launches = before; }
+};
 template <typename... P, typename... A>
 static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -61,7 +70,7 @@ static cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.attrs = at; cfg.numAttrs = pdl_enabled() && !t_plain_launches ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 // Function attributes (the opt-in to more than 48 KB of dynamic shared memory, occupancy figures) belong to one device, so
@@ -1272,6 +1281,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     const bool streaming = tiled || c->path == 0;
     // large batches go to the tcgen05 grouped GEMM; the rest to the streaming kernels
     const bool prefill = tiled && T >= grouped_min_tokens(c, L->fmt);
+    const PlainLaunches plain(prefill);
     const bool f16 = tiled && L->fmt != FMT_ZP && !prefill;  // element type of the split activations the streaming kernels read
     const int parts = prefill && bf16 && !block ? 1 : 2;
     const int mode = !streaming ? ROWS_NONE : prefill ? (L->fmt == FMT_ZP ? ROWS_GEMM_Z : ROWS_GEMM) : f16 ? ROWS_F16 : ROWS_BF16;
