@@ -188,6 +188,7 @@ struct moexb_layer {
     void* router = nullptr;                 // [n_routed + 1][H]
     const uint8_t** slot_table = nullptr;   // device, n_routed + 1 pointers
     std::vector<const uint8_t*> slot_host;
+    GroupedMaps map_gate_up{}, map_down{};  // the image as the grouped GEMM's copies see it (tiled layout)
     // per expert id (index n_routed = the shared expert): weights were put there by an upload, a synthetic fill or a file load.
     // The image starts zeroed, so an expert that was never loaded contributes zeros; the shared expert runs for every token,
     // so the layer-level calls refuse to run it unloaded instead of silently adding nothing.
@@ -524,6 +525,36 @@ int moexb_synth_experts(moexb_ctx* ctx, int fmt, unsigned seed, int layer, int e
     return synth_launch(fmt, seed, layer, e0, n, dst, ctx->table_s, ctx->table_d, stream);
 }
 
+}  // extern "C"
+// One tensor map over the image of n_blobs tiled blobs, [slice / 4][K slice][8 bytes]: boxes of `elems` x 8 bytes of 16 slices - the same K
+// slice of 16 row tiles (gate/up), or 16 slices in a row (down). The encoder is a driver call, looked up through the runtime.
+static int image_map(CUtensorMap* map, const uint8_t* image, int slice_bytes, size_t n_blobs, int elems, bool down) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = nullptr; cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? (Encode)f : nullptr;
+    }();
+    if (!encode) return fail(MOEXB_ERR_CUDA, "layer_create: the driver has no tensor map encoder");
+    const cuuint64_t dims[3] = {(cuuint64_t)slice_bytes / 8, 4, (cuuint64_t)n_blobs * (TL_SLICES / 4)}, strides[2] = {(cuuint64_t)slice_bytes, (cuuint64_t)slice_bytes * 4};
+    const cuuint32_t box[3] = {(cuuint32_t)elems, down ? 4u : 1u, down ? 4u : 16u}, step[3] = {1, 1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<uint8_t*>(image), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? (int)MOEXB_OK : fail(MOEXB_ERR_CUDA, "layer_create: tensor map: error %d", (int)r);
+}
+static int layer_maps(moexb_layer* L) {
+    return by_fmt(L->fmt, [&]<int FMT>() {
+        int rc = MOEXB_OK;
+        for (int down = 0; down < 2 && rc == MOEXB_OK; down++) {
+            GroupedMaps& m = down ? L->map_down : L->map_gate_up;
+            rc = image_map(&m.w, L->image, tl_slice_bytes<FMT>(), L->n_local + 1, GG_CH * tl_group_bytes<FMT>() / 8, down);
+            if (rc == MOEXB_OK && FMT == FMT_ZP) rc = image_map(&m.dd, L->image, tl_slice_bytes<FMT>(), L->n_local + 1, 16, down);
+        }
+        return rc;
+    });
+}
+
+extern "C" {
 int moexb_layer_create(moexb_ctx* ctx, int fmt, int n_routed, int first_local, int n_local, int router_dtype, int layout, moexb_layer** out) {
     REQUIRE(ctx && out, "layer_create: null pointer");
     REQUIRE(fmt_ok(fmt), "layer_create: unknown expert format %d", fmt);
@@ -548,6 +579,10 @@ int moexb_layer_create(moexb_ctx* ctx, int fmt, int n_routed, int first_local, i
         e = cudaMemcpy(L->slot_table, L->slot_host.data(), L->slot_host.size() * sizeof(void*), cudaMemcpyHostToDevice);
     }
     if (e != cudaSuccess) { moexb_layer_destroy(L); return fail(MOEXB_ERR_NOMEM, "layer_create: %s", cudaGetErrorString(e)); }
+    if (layout == MOEXB_LAYOUT_TILED) {
+        const int rc = layer_maps(L);
+        if (rc != MOEXB_OK) { moexb_layer_destroy(L); return rc; }
+    }
     *out = L;
     return MOEXB_OK;
 }
@@ -1062,13 +1097,13 @@ static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* 
 // ---- prefill: grouped GEMM on tcgen05 ----------------------------------------------------------------------------------------
 
 template <int FMT, bool DOWN>
-static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, void* stream) {
+static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, const GroupedMaps& maps, void* stream) {
     constexpr int SMEM = gg_smem_bytes<FMT>();
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(grouped_k<FMT, DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "grouped GEMM shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
-    CUDA_TRY(launch_dep(grouped_k<FMT, DOWN>, c->sms, GG_THREADS, SMEM, S(stream), a));
+    CUDA_TRY(launch_dep(grouped_k<FMT, DOWN>, c->sms, GG_THREADS, SMEM, S(stream), a, maps));
     LAUNCHED(DOWN ? "grouped_down" : "grouped_gate_up");
     return MOEXB_OK;
 }
@@ -1081,13 +1116,13 @@ static int grouped_maxp(int fmt) { return fmt == FMT_ZP ? gg_nmax<FMT_ZP>() : gg
 
 // Experts of a large batch on the tensor-core grouped GEMM: the tiles are in the context (subs, nsub) or in the buckets, and grouped_rows or
 // the token owners (expert parallelism) left the activation rows.
-static int grouped_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, int parts, float* ypair, void* stream, const BucketArgs* buckets = nullptr) {
-    return by_fmt(fmt, [&]<int FMT>() {
-        GroupedArgs a{buckets ? nullptr : c->subs, c->nsub, buckets ? *buckets : BucketArgs{}, buckets ? buckets->pairs : pairs, c->xs, c->sx, c->act_split, c->sx_act, ypair, c->err, parts};
-        int rc = grouped_launch_one<FMT, false>(c, a, stream);
+static int grouped_experts(moexb_ctx* c, const moexb_layer* L, const moexb_pair* pairs, int parts, float* ypair, void* stream, const BucketArgs* buckets = nullptr) {
+    return by_fmt(L->fmt, [&]<int FMT>() {
+        GroupedArgs a{L->image, buckets ? nullptr : c->subs, c->nsub, buckets ? *buckets : BucketArgs{}, buckets ? buckets->pairs : pairs, c->xs, c->sx, c->act_split, c->sx_act, ypair, c->err, parts};
+        int rc = grouped_launch_one<FMT, false>(c, a, L->map_gate_up, stream);
         if (rc != MOEXB_OK) return rc;
         a.xs = c->act_split; a.sx = c->sx_act; a.parts = 2;
-        return grouped_launch_one<FMT, true>(c, a, stream);
+        return grouped_launch_one<FMT, true>(c, a, L->map_down, stream);
     });
 }
 
@@ -1341,7 +1376,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
             // reduction skips them by expert id
             if (!all_local && !streaming) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)T * K * EH * sizeof(float), st));
         }
-        rc = prefill ? grouped_experts(c, L->fmt, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
+        rc = prefill ? grouped_experts(c, L, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
            : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr)
            : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream)
                        : pairs_launch(c, L->fmt, c->items, c->nitems, min(E, T * K) + 1, c->pairs, xf, c->act, c->ypair, stream);
@@ -1763,7 +1798,7 @@ int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
                             flags, (const unsigned*)e->step, (unsigned)(l + 1), e->g.world, e->g.rank, c->err));
         LAUNCHED("group_plan");
     }
-    rc = prefill ? grouped_experts(c, L->fmt, c->pairs, e->parts, c->ypair, stream)
+    rc = prefill ? grouped_experts(c, L, c->pairs, e->parts, c->ypair, stream)
        : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, in_kernel ? &plan : nullptr)
                : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream);
     if (rc != MOEXB_OK) return rc;
