@@ -186,8 +186,8 @@ int moexb_ctx_destroy(moexb_ctx* ctx);
  * 256-byte row pieces (default), 1 = the fp32 SIMT kernels (the restatement of the reference's pairs_forward /
  * experts_forward, kept for cross-checks). TILED layers always use the tiled streaming kernels. */
 int moexb_ctx_set_path(moexb_ctx* ctx, int path);
-/* Batches of at least this many tokens run the experts on the tcgen05 grouped GEMM (TILED layers, symmetric formats);
- * smaller ones on the streaming kernels. Default 256. */
+/* Batches of at least this many tokens run the experts on the tcgen05 grouped GEMM (TILED layers; zero-point blobs from a
+ * third of it on); smaller ones on the streaming kernels. Default 256. */
 int moexb_ctx_set_prefill_min_tokens(moexb_ctx* ctx, int tokens);
 /* Pairs of one expert that a pass of the tiled streaming kernels takes (batches of 8 to prefill_min_tokens - 1 tokens,
  * symmetric formats): 8 (default; an expert with 5-8 pairs is unpacked once) or 4. Smaller batches and zero-point blobs
