@@ -20,7 +20,7 @@
 //       rank order (the products and the order of the down kernel + reduce_residual_norm_k) -> xnew[H] in global memory.
 //                                                                                              -- grid barrier --
 //   P5  every CTA: the new row from L2 (8 KB), rmsnorm and split for the next layer, all in shared memory.
-// The grid barrier is a monotonic counter in global memory (zeroed by the host before the launch): one thread per CTA adds
+// The grid barrier is a monotonic counter in global memory (zero at the launch): one thread per CTA adds
 // 1 and polls until the counter reaches (barriers so far) x grid. Every poll loop is bounded; a time-out sets the error
 // word and an abort flag that all other loops watch, and the CTAs leave after waiting (bounded) for their copies in flight.
 // The arithmetic of a slice is that of stream_tiled_k (exact fp16 nibbles, hi + lo activations, mma.sync, fp32 group
@@ -50,7 +50,7 @@ struct DecodeStackArgs {
     float* wts;              // [K + 1] routing weights of the selected experts, then the shared expert's gate
     int* idx_out;            // optional [n_layers][K]
     float* w_out;            // optional [n_layers][K]
-    unsigned* sync;          // [0] barrier counter, [1] abort flag; zero before the launch
+    unsigned* sync;          // [0] barrier counter, [1] abort flag, [2] CTAs that have left; zero before the first launch, left zero
     int* err;
 };
 
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_k(const DecodeStac
             *reinterpret_cast<float4*>(xres + 1024 * h + 4 * tid) = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
     }
     __syncthreads();
-    norm_split_row<F16>(v, xn, reinterpret_cast<uint16_t*>(xcol), 1e-6f, DS_XCOL / 2);
+    norm_split_row<F16, true>(v, xn, reinterpret_cast<uint16_t*>(xcol), 1e-6f, DS_XCOL / 2);
     __syncthreads();
     // [K slice][group][chunk][hi, lo]: thread = (column, K slice, group, chunk); read by P3 after later block barriers
     auto x_sums = [&]() {
@@ -505,22 +505,32 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_stack_k(const DecodeStac
             v[4 * h] = acc.x; v[4 * h + 1] = acc.y; v[4 * h + 2] = acc.z; v[4 * h + 3] = acc.w;
         }
         __syncthreads();   // part[] of norm_split_row and xn / xcol are free: every warp is past P1 and P3 of this layer
-        if (l + 1 < a.n_layers) norm_split_row<F16>(v, xn, reinterpret_cast<uint16_t*>(xcol), 1e-6f, DS_XCOL / 2);
+        if (l + 1 < a.n_layers) norm_split_row<F16, true>(v, xn, reinterpret_cast<uint16_t*>(xcol), 1e-6f, DS_XCOL / 2);
         asm volatile("cp.async.wait_all;" ::: "memory");   // the next layer's router rows and slot table
         __syncthreads();
         if (l + 1 < a.n_layers) x_sums();
     }
+    // The last CTA to leave clears the counters for the next launch (nobody polls them any more), which saves the host a memset.
+    auto left = [&]() {
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            if (atomicAdd(a.sync + 2, 1u) == (unsigned)grid - 1) { a.sync[0] = 0; a.sync[1] = 0; a.sync[2] = 0; }
+        }
+    };
     // leave: no copy may still be in flight into this CTA's shared memory
     if (!ok) {
         for (int s = consumed; s < issued; s++)
             if (slice_src(s)) wait_slice(s);
         if (sh_inflight) mbar_wait(smem_u32(&shbar), sh_phase, a.err, DS_ERR_COPY);
+        left();
         return;
     }
     if (b == 0) {
 #pragma unroll
         for (int h = 0; h < 2; h++) *reinterpret_cast<float4*>(a.x_out + 1024 * h + 4 * tid) = *reinterpret_cast<const float4*>(xres + 1024 * h + 4 * tid);
     }
+    left();
 }
 
 // Self-test of the grid barrier's time-out: a grid of ONE CTA arrives at a barrier that expects two arrivals.

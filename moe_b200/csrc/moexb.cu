@@ -1464,7 +1464,7 @@ int moexb_stack_destroy(moexb_stack* s) {
 
 }  // extern "C"
 template <int FMT, typename WT, bool XBF>
-static int decode_stack_launch(moexb_stack* s, void* stream) {
+static int decode_stack_launch(moexb_stack* s, const void* X, float* out, void* stream) {
     moexb_ctx* c = s->ctx;
     constexpr int SMEM = ds_smem_bytes<FMT>();
     static PerDeviceOnce once;
@@ -1476,17 +1476,16 @@ static int decode_stack_launch(moexb_stack* s, void* stream) {
         return e;
     });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "decode stack kernel: %s", cudaGetErrorString(attr_err));
-    CUDA_TRY(cudaMemsetAsync(s->dsync, 0, 2 * sizeof(unsigned), S(stream)));
-    DecodeStackArgs a{s->dlayers, s->n_layers, s->n_routed, s->K, s->x_in, s->buf[0], c->logits, c->act_split, c->ypair, c->wts, nullptr, nullptr, s->dsync, c->err};
+    DecodeStackArgs a{s->dlayers, s->n_layers, s->n_routed, s->K, X, out, c->logits, c->act_split, c->ypair, c->wts, nullptr, nullptr, s->dsync, c->err};
     void* args[] = {&a};
     // cooperative: every CTA is resident, which the grid barrier inside relies on
     CUDA_TRY(cudaLaunchCooperativeKernel((void*)decode_stack_k<FMT, WT, XBF>, dim3(c->sms), dim3(DS_THREADS), args, SMEM, S(stream)));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return MOEXB_OK;
 }
-static int decode_stack_run(moexb_stack* s, void* stream) {
+static int decode_stack_run(moexb_stack* s, const void* X, float* out, void* stream) {
     auto by_x = [&]<int FMT, typename WT>() {
-        return s->x_dtype == MOEXB_BF16 ? decode_stack_launch<FMT, WT, true>(s, stream) : decode_stack_launch<FMT, WT, false>(s, stream);
+        return s->x_dtype == MOEXB_BF16 ? decode_stack_launch<FMT, WT, true>(s, X, out, stream) : decode_stack_launch<FMT, WT, false>(s, X, out, stream);
     };
     auto by_w = [&]<int FMT>() {
         return s->router_dtype == MOEXB_F32 ? by_x.template operator()<FMT, float>() : by_x.template operator()<FMT, __half>();
@@ -1525,7 +1524,8 @@ int moexb_stack_create(moexb_ctx* c, moexb_layer* const* layers, int n_layers, i
         std::vector<DecodeLayer> h(n_layers);
         for (int l = 0; l < n_layers; l++) h[l] = {layers[l]->router, layers[l]->slot_table};
         e = cudaMalloc((void**)&s->dlayers, n_layers * sizeof(DecodeLayer));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&s->dsync, 2 * sizeof(unsigned));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&s->dsync, 3 * sizeof(unsigned));
+        if (e == cudaSuccess) e = cudaMemset(s->dsync, 0, 3 * sizeof(unsigned));
         if (e == cudaSuccess) e = cudaMemcpy(s->dlayers, h.data(), n_layers * sizeof(DecodeLayer), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) { moexb_stack_destroy(s); return fail(MOEXB_ERR_NOMEM, "stack_create: %s", cudaGetErrorString(e)); }
         s->fused = true; s->fmt = layers[0]->fmt; s->router_dtype = layers[0]->router_dtype; s->n_routed = layers[0]->n_routed;
@@ -1561,8 +1561,10 @@ int moexb_stack_kernel_count(moexb_stack* s) { return s ? s->kernels : 0; }
 int moexb_stack_run(moexb_stack* s, const void* X, float* out, void* stream) {
     REQUIRE(s && X && out, "stack_run: null pointer");
     const size_t n = (size_t)s->T * EH;
+    // the one-token kernel reads and writes the caller's buffers itself where they allow 16-byte accesses
+    if (s->fused && !((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(out)) & 15)) return decode_stack_run(s, X, out, stream);
     CUDA_TRY(cudaMemcpyAsync(s->x_in, X, n * (s->x_dtype == MOEXB_BF16 ? 2 : 4), cudaMemcpyDeviceToDevice, S(stream)));
-    if (s->fused) { const int rc = decode_stack_run(s, stream); if (rc != MOEXB_OK) return rc; }
+    if (s->fused) { const int rc = decode_stack_run(s, s->x_in, s->buf[0], stream); if (rc != MOEXB_OK) return rc; }
     else {
         CUDA_TRY(cudaGraphLaunch(s->exec, S(stream)));
         g_launches.fetch_add(s->kernels, std::memory_order_relaxed);
@@ -1575,7 +1577,7 @@ int moexb_stack_run_host(moexb_stack* s, const void* X_host, float* out_host, vo
     REQUIRE(s && X_host && out_host, "stack_run_host: null pointer");
     const size_t n = (size_t)s->T * EH;
     CUDA_TRY(cudaMemcpyAsync(s->x_in, X_host, n * (s->x_dtype == MOEXB_BF16 ? 2 : 4), cudaMemcpyHostToDevice, S(stream)));
-    if (s->fused) { const int rc = decode_stack_run(s, stream); if (rc != MOEXB_OK) return rc; }
+    if (s->fused) { const int rc = decode_stack_run(s, s->x_in, s->buf[0], stream); if (rc != MOEXB_OK) return rc; }
     else {
         CUDA_TRY(cudaGraphLaunch(s->exec, S(stream)));
         g_launches.fetch_add(s->kernels, std::memory_order_relaxed);

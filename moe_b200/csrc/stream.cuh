@@ -404,19 +404,30 @@ __device__ __forceinline__ float row_rms_scale(const float (&v)[8], float eps) {
     return 1.f / sqrtf(tot / (float)EH + eps);
 }
 // The row times r as fp32 into xn and, when xs is given, split into xs (hi) and xs + lo_off (lo).
-template <bool F16>
+// SHARED: xs is shared memory, where 2-byte stores are cheaper than the exchange between threads (one token x 40 layers: 527 us, 538
+// with the exchange).
+template <bool F16, bool SHARED = false>
 __device__ __forceinline__ void scaled_split_row(const float (&v)[8], float r, float* __restrict__ xn, uint16_t* __restrict__ xs, int lo_off = EH) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int k0 = 1024 * h + 4 * threadIdx.x;
         const float f[4] = {v[4 * h] * r, v[4 * h + 1] * r, v[4 * h + 2] * r, v[4 * h + 3] * r};
         *reinterpret_cast<float4*>(xn + k0) = make_float4(f[0], f[1], f[2], f[3]);
-        if (xs) store_split4<F16 ? ROWS_F16 : ROWS_BF16>(f, k0, xs, lo_off);
+        if (!xs) continue;
+        if constexpr (SHARED) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                uint16_t hi, lo;
+                split_hi_lo<F16>(f[i], hi, lo);
+                const int pos = split_pos(k0 + i);
+                xs[pos] = hi; xs[lo_off + pos] = lo;
+            }
+        } else store_split4<F16 ? ROWS_F16 : ROWS_BF16>(f, k0, xs, lo_off);
     }
 }
-template <bool F16>
+template <bool F16, bool SHARED = false>
 __device__ __forceinline__ void norm_split_row(const float (&v)[8], float* __restrict__ xn, uint16_t* __restrict__ xs, float eps, int lo_off = EH) {
-    scaled_split_row<F16>(v, row_rms_scale(v, eps), xn, xs, lo_off);
+    scaled_split_row<F16, SHARED>(v, row_rms_scale(v, eps), xn, xs, lo_off);
 }
 
 // What a layer makes of its input rows before the router and the experts, in one pass: bf16 rows widened to xf (when given), the
