@@ -1,0 +1,60 @@
+"""The work list where its size changes the path: the grouping kernel over several passes of 1024 pairs, and layers whose experts are too
+many for the router's buckets (a planning launch instead). Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+import moe_b200 as m
+from oracle import oracle as o
+from parity import check_ffn
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("lib_built")]
+DEV = "cuda:0"
+ITEM_DT = np.dtype([("slot", "<u8"), ("start", "<i4"), ("count", "<i4")])
+PAIR_DT = np.dtype([("t", "<i4"), ("p", "<i4"), ("w", "<f4")])
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+
+
+@pytest.mark.parametrize("T", [128, 129, 300])
+def test_group_pairs_in_several_passes(T):
+    E, K = 64, 8
+    rng = np.random.default_rng(T)
+    idx = np.stack([rng.choice(E, size=K, replace=False) for _ in range(T)]).astype(np.int32)
+    w = rng.uniform(0, 1, (T, K)).astype(np.float32)
+    table = np.arange(1, E + 2, dtype=np.int64) * 4096
+    held = np.ones(E, np.uint8)
+    held[7:11] = 0
+    table[7:11] = 0
+    items, pairs, nitems = m.group_pairs(dev(idx), dev(w), T, K, E, dev(table))
+    ri, pt, pp, pw = o.group_pairs(idx, w, E, held)
+    gi = items.cpu().numpy().view(ITEM_DT); gp = pairs.cpu().numpy().view(PAIR_DT)
+    assert int(nitems.item()) == len(ri)
+    assert [(int(table[e]), s, c) for e, s, c in ri] == [(int(a), int(b), int(c)) for a, b, c in gi[:len(ri)]]
+    assert not gi["count"][len(ri):].any() and not gp["w"][len(pt):].any()
+    assert np.array_equal(gp["t"][:len(pt)], pt) and np.array_equal(gp["p"][:len(pt)], pp) and np.array_equal(gp["w"][:len(pt)], pw)
+
+
+def test_layer_with_more_experts_than_the_buckets_take():
+    E, K = 288, 8
+    c = m.Context(0, max_tokens=20, max_experts=E, top_k=K)
+    L = m.Layer(c, m.FMT_SYM_F16, E)
+    L.fill_synth(4, 0)
+    rng = np.random.default_rng(6)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    host = [m.synth_expert_host(m.FMT_SYM_F16, 4, 0, e) for e in range(E + 1)]
+    try:
+        for T, min_tokens in ((5, 256), (20, 256), (20, 1)):
+            c.set_prefill_min_tokens(min_tokens)
+            X = rng.standard_normal((T, 2048)).astype(np.float32)
+            idx = torch.empty(T, K, dtype=torch.int32, device=DEV)
+            out = L.forward(dev(X), T, K, idx=idx).cpu().numpy()
+            assert c.status() == 0
+            ref, ri, _, _ = o.layer_forward(m.FMT_SYM_F16, host, W, X, K)
+            assert np.array_equal(idx.cpu().numpy(), ri)
+            check_ffn(out, ref, m.FMT_SYM_F16, f"{E} experts, {T} tokens")
+    finally:
+        L.close(); c.close()
