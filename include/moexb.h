@@ -198,7 +198,8 @@ int moexb_ctx_set_pairs_per_pass(moexb_ctx* ctx, int pairs);
  * Read when a stack is created. */
 int moexb_ctx_set_fused_decode(moexb_ctx* ctx, int on);
 /* Waits for the device and reads the error word of the kernels: 0 = none; 1 / 2 = a consumer warp / the producer warp of a
- * streaming kernel gave up waiting on a pipeline barrier, 3 = the same in the tensor-core grouped GEMM, 5 / 6 = the one-token
+ * streaming kernel gave up waiting on a pipeline barrier, 3 = the same in the tensor-core grouped GEMM, 4 = the router met
+ * bucket counts that were not zero (calls on one context that overlapped on the GPU), 5 / 6 = the one-token
  * stack kernel gave up at a grid barrier / on a weight copy, 7 / 8 = an expert-parallel rank gave up waiting for a peer's
  * dispatch / combine flag (every device-side wait is bounded). The word is cleared. */
 int moexb_ctx_status(moexb_ctx* ctx, int* status);
@@ -209,6 +210,10 @@ int moexb_ctx_status(moexb_ctx* ctx, int* status);
  * word is cleared. The counterpart of the reference's wait_add_k giving up after timeout_ns and
  * raising its abort word (kernels.cuh:1055-1089). */
 int moexb_ctx_selftest_timeout(moexb_ctx* ctx, int which, int polls, int* status);
+
+/* The next layer-level call on the context that runs the experts returns MOEXB_ERR_CUDA after its router was enqueued, as if a
+ * launch had failed there. What later calls on the context give must not depend on it. */
+int moexb_ctx_selftest_fail(moexb_ctx* ctx);
 
 /* Allocates the image of one layer: n_routed experts (ids 0..n_routed-1) and the shared expert (id n_routed), each a
  * blob of format fmt, plus the router [n_routed+1][H] (row n_routed = the shared expert's gate vector).

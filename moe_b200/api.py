@@ -197,6 +197,10 @@ class Context:
         check(lib().moexb_ctx_selftest_timeout(self.h, which, polls, C.byref(st)))
         return st.value
 
+    def selftest_fail(self):
+        """moexb_ctx_selftest_fail: the next layer call returns an error after its router was enqueued."""
+        check(lib().moexb_ctx_selftest_fail(self.h))
+
     def pairs_forward_tc(self, fmt, items, n_items, pairs, X, T, npairs, act, ypair):
         """reference pairs_forward_tc (kernels.cuh:955) on the streaming kernels."""
         check(lib().moexb_pairs_forward_tc(self.h, fmt, _ptr(items), n_items, _ptr(pairs), _ptr(X), T, npairs, _ptr(act), _ptr(ypair), _stream()))

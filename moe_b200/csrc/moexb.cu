@@ -149,6 +149,8 @@ struct moexb_ctx {
     int *nsub = nullptr, *err = nullptr;
     float *sx = nullptr, *sx_act = nullptr;             // grouped GEMM, zero point: activation sums per 32-input chunk, of the tokens and of act
     int* bcnt = nullptr; moexb_pair* bpairs = nullptr;  // the work list as buckets (null when they would be too large)
+    bool buckets_dirty = false;                         // a call failed between its router and its combine: bcnt may not be zero
+    bool selftest_fail = false;                         // the next layer call fails there (moexb_ctx_selftest_fail)
     int* route_done = nullptr;                          // per token tile: blocks of the routing kernel that have finished (returns to zero)
     int sms = 0, path = 0;                              // path: 0 = streaming kernels, 1 = fp32 SIMT kernels
     int fused_decode = 1;                               // one-token residual stacks run as one cooperative launch
@@ -1190,6 +1192,12 @@ extern "C" int moexb_ctx_set_prefill_min_tokens(moexb_ctx* c, int tokens) {
     return MOEXB_OK;
 }
 
+extern "C" int moexb_ctx_selftest_fail(moexb_ctx* c) {
+    REQUIRE(c, "ctx_selftest_fail: null pointer");
+    c->selftest_fail = true;
+    return MOEXB_OK;
+}
+
 extern "C" int moexb_ctx_set_path(moexb_ctx* c, int path) {
     REQUIRE(c && (path == 0 || path == 1), "ctx_set_path: path must be 0 (streaming) or 1 (fp32 SIMT)");
     c->path = path;
@@ -1248,7 +1256,7 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
               decode ? c->subs : nullptr, decode ? c->pairs : nullptr, decode ? c->nsub : nullptr};
     if (ro.buckets) {
         o.bcnt = c->bcnt; o.bpairs = c->bpairs; o.bstride = c->max_tokens; o.e_lo = L->first_local; o.e_hi = L->first_local + L->n_local; o.npairs = T * K;
-        o.bshared = ro.shared;
+        o.bshared = ro.shared; o.err = c->err;
     }
     o.idx2 = ro.idx; o.w2 = ro.w;
     if (rep) { o.ep = rep->dev; o.ep_row_bytes = rep->row_bytes; o.ep_phase = rep->phase; o.ep_step = rep->step; }
@@ -1304,6 +1312,29 @@ static int layer_route(moexb_ctx* c, moexb_layer* L, const void* xf, int T, int 
     return L->router_dtype == MOEXB_F32 ? route_launch<float>(c, L, xf, T, K, stream, decode, ro, tok0, rep) : route_launch<__half>(c, L, xf, T, K, stream, decode, ro, tok0, rep);
 }
 
+// Zeroes the bucket counts on `st`. Under capture the graph does it when it runs, so what is in memory now stays marked.
+static int clear_buckets(moexb_ctx* c, cudaStream_t st) {
+    c->buckets_dirty = true;
+    CUDA_TRY(cudaMemsetAsync(c->bcnt, 0, (size_t)c->max_experts * sizeof(int), st));
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    c->buckets_dirty = cap != cudaStreamCaptureStatusNone;
+    return MOEXB_OK;
+}
+// The router adds to the bucket counts and the combine kernel clears them; a call that returns between the two clears them itself, so
+// that neither the next call nor the replay of a graph finds its pairs there. Where that fails too, the next call does it.
+struct BucketCounts {
+    moexb_ctx* c; cudaStream_t st; bool open = false;
+    ~BucketCounts() {
+        if (!open) return;
+        char why[sizeof(g_err)];
+        memcpy(why, g_err, sizeof(g_err));
+        cudaGetLastError();
+        clear_buckets(c, st);
+        memcpy(g_err, why, sizeof(g_err));   // what the caller is told stays the first failure
+    }
+};
+
 // One layer. X: the layer input [T][H] of x_dtype. flags as moexb_layer_forward. pre_normed: the context already holds
 // rmsnorm(X) and its split (left there by the previous layer of a stack); next_norm: leave rmsnorm(out) and its
 // split in the context for the next layer.
@@ -1340,8 +1371,11 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     const bool decode = T == 1 && all_local && shared && !partial && !prefill;
     const bool buckets = tiled && !decode && c->bpairs;
     ro.buckets = buckets; ro.shared = buckets && shared; ro.idx = idx_out; ro.w = w_out;
+    if (buckets && c->buckets_dirty) { rc = clear_buckets(c, st); if (rc != MOEXB_OK) return rc; }
+    BucketCounts counts{c, st, buckets};
     rc = layer_route(c, L, xr, T, K, stream, decode, ro);
     if (rc != MOEXB_OK) return rc;
+    if (c->selftest_fail) { c->selftest_fail = false; return fail(MOEXB_ERR_CUDA, "layer: the failure that a self-test asked for"); }
     int ranks = K;                  // rows of ypair per token that the final reduction adds
     const float* extra = nullptr;   // + the shared expert's rows
     if (partial && !streaming) return fail(MOEXB_ERR_UNSUPPORTED, "layer_forward: partial outputs need the streaming kernels");
@@ -1393,6 +1427,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
         if (f16) CUDA_TRY(launch_dep(reduce_residual_norm_k<true>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local, buckets ? c->bcnt : (int*)nullptr, E));
         else CUDA_TRY(launch_dep(reduce_residual_norm_k<false>, T, 256, 0, st, c->ypair, extra, xres, out, ranks, xn_next, prefill ? (uint16_t*)nullptr : c->xs, 1e-6f, sh0, sh1, held, L->first_local, L->first_local + L->n_local, buckets ? c->bcnt : (int*)nullptr, E));
         LAUNCHED("reduce_residual_norm");
+        counts.open = false;
     }
     return MOEXB_OK;
 }
@@ -1563,6 +1598,7 @@ int moexb_stack_run(moexb_stack* s, const void* X, float* out, void* stream) {
     const size_t n = (size_t)s->T * EH;
     // the one-token kernel reads and writes the caller's buffers itself where they allow 16-byte accesses
     if (s->fused && !((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(out)) & 15)) return decode_stack_run(s, X, out, stream);
+    if (s->ctx->buckets_dirty) { const int rc = clear_buckets(s->ctx, S(stream)); if (rc != MOEXB_OK) return rc; }
     CUDA_TRY(cudaMemcpyAsync(s->x_in, X, n * (s->x_dtype == MOEXB_BF16 ? 2 : 4), cudaMemcpyDeviceToDevice, S(stream)));
     if (s->fused) { const int rc = decode_stack_run(s, s->x_in, s->buf[0], stream); if (rc != MOEXB_OK) return rc; }
     else {
@@ -1576,6 +1612,7 @@ int moexb_stack_run(moexb_stack* s, const void* X, float* out, void* stream) {
 int moexb_stack_run_host(moexb_stack* s, const void* X_host, float* out_host, void* stream) {
     REQUIRE(s && X_host && out_host, "stack_run_host: null pointer");
     const size_t n = (size_t)s->T * EH;
+    if (s->ctx->buckets_dirty) { const int rc = clear_buckets(s->ctx, S(stream)); if (rc != MOEXB_OK) return rc; }
     CUDA_TRY(cudaMemcpyAsync(s->x_in, X_host, n * (s->x_dtype == MOEXB_BF16 ? 2 : 4), cudaMemcpyHostToDevice, S(stream)));
     if (s->fused) { const int rc = decode_stack_run(s, s->x_in, s->buf[0], stream); if (rc != MOEXB_OK) return rc; }
     else {

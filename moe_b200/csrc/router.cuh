@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_rows_k(const WT* __restrict__
 // logits count as -inf. Optional decode outputs: slots_out / wts_out [K+1] = the selected experts' blob pointers and
 // weights followed by the shared expert with weight sigmoid(logits[E]); dsubs / dpairs / dnsub = the same K+1 experts as
 // one-pair sub-items for the streaming kernels (T = 1).
+constexpr int BK_ERR_FULL = 4;
 struct TopkOut {
     int* idx; float* w;
     const uint8_t* const* slot_table; const uint8_t** slots_out; float* wts_out;
@@ -147,7 +148,7 @@ struct TopkOut {
     // hold one of the selected experts - and the block then raises the tokens' dispatch flags
     const EpDevice* ep = nullptr; int ep_row_bytes = 0; unsigned ep_phase = 0; const unsigned* ep_step = nullptr;
     // the pairs into the experts' buckets (BucketArgs): experts [e_lo, e_hi) are held here; npairs = T * K
-    int* bcnt = nullptr; moexb_pair* bpairs = nullptr; int bstride = 0, e_lo = 0, e_hi = 0, npairs = 0; bool bshared = false;
+    int* bcnt = nullptr; moexb_pair* bpairs = nullptr; int bstride = 0, e_lo = 0, e_hi = 0, npairs = 0; bool bshared = false; int* err = nullptr;
     int* idx2 = nullptr; float* w2 = nullptr;   // a second copy of ids and weights (the caller's buffers)
 };
 __device__ __forceinline__ unsigned f2key(float v) { const unsigned u = __float_as_uint(v); return (u & 0x80000000u) ? ~u : (u | 0x80000000u); }
@@ -212,8 +213,12 @@ __device__ __forceinline__ void topk_token(const float* __restrict__ l, int t, i
         const float wk = norm ? mine / total : mine;
         o.idx[(size_t)t * K + lane] = mine_i;
         o.w[(size_t)t * K + lane] = wk;
-        if (o.bpairs && mine_i >= o.e_lo && mine_i < o.e_hi)
-            o.bpairs[(size_t)mine_i * o.bstride + atomicAdd(o.bcnt + mine_i, 1)] = {t, t * K + lane, wk};
+        if (o.bpairs && mine_i >= o.e_lo && mine_i < o.e_hi) {
+            const int place = atomicAdd(o.bcnt + mine_i, 1);
+            // an expert takes each token once, so a place beyond the bucket means counts that were not zero when the call began
+            if (place < o.bstride) o.bpairs[(size_t)mine_i * o.bstride + place] = {t, t * K + lane, wk};
+            else atomicExch(o.err, BK_ERR_FULL);
+        }
         if (o.idx2) o.idx2[(size_t)t * K + lane] = mine_i;
         if (o.w2) o.w2[(size_t)t * K + lane] = wk;
         if (o.slots_out) { o.slots_out[(size_t)t * (K + 1) + lane] = o.slot_table[mine_i]; o.wts_out[(size_t)t * (K + 1) + lane] = wk; }

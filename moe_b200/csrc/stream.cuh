@@ -733,6 +733,8 @@ __device__ __forceinline__ void bucket_scan(BucketSmem& L, const BucketArgs& a, 
     if (8 * lane < a.E) {
         const int4 p = __ldcg(reinterpret_cast<const int4*>(a.cnt) + 2 * lane), q = __ldcg(reinterpret_cast<const int4*>(a.cnt) + 2 * lane + 1);
         c[0] = p.x; c[1] = p.y; c[2] = p.z; c[3] = p.w; c[4] = q.x; c[5] = q.y; c[6] = q.z; c[7] = q.w;
+#pragma unroll
+        for (int j = 0; j < 8; j++) c[j] = min(c[j], a.stride);   // (more than that: topk_token has set the error word)
     }
 #pragma unroll
     for (int j = 0; j < 8; j++) { sw += wide(c[j]); sn += narrow(c[j]); }

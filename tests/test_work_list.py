@@ -58,3 +58,32 @@ def test_layer_with_more_experts_than_the_buckets_take():
             check_ffn(out, ref, m.FMT_SYM_F16, f"{E} experts, {T} tokens")
     finally:
         L.close(); c.close()
+
+
+@pytest.mark.parametrize("fmt,T", [(m.FMT_SYM_F16, 5), (m.FMT_ZP, 24), (m.FMT_SYM_F16, 24)])
+def test_a_call_that_failed_after_its_router_leaves_nothing_behind(fmt, T):
+    """The pairs that the router of a failed call put into the buckets must not be there for the next call, nor for the replay of a
+    stack captured before. 64 places a bucket: the pairs of both calls fit."""
+    E, K = 32, 8
+    c = m.Context(0, max_tokens=64, max_experts=E, top_k=K)
+    L = m.Layer(c, fmt, E)
+    L.fill_synth(5, 0)
+    rng = np.random.default_rng(T)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    X = rng.standard_normal((T, 2048)).astype(np.float32)
+    stack = m.Stack(c, [L], T, K, m.F32, residual=False)
+    try:
+        before = stack.run(dev(X)).cpu().numpy()
+        for again in range(3):
+            c.selftest_fail()
+            with pytest.raises(m.MoexbError, match="self-test"):
+                L.forward(dev(rng.standard_normal((T, 2048)).astype(np.float32)), T, K)
+            if again == 1:
+                assert np.array_equal(stack.run(dev(X)).cpu().numpy(), before)
+        assert np.array_equal(L.forward(dev(X), T, K).cpu().numpy(), before)
+        assert c.status() == 0
+        ref, _, _, _ = o.layer_forward(fmt, [m.synth_expert_host(fmt, 5, 0, e) for e in range(E + 1)], W, X, K)
+        check_ffn(before, ref, fmt, f"{T} tokens before and after failed calls")
+    finally:
+        stack.close(); L.close(); c.close()
