@@ -1113,7 +1113,10 @@ static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, const GroupedM
 // Batches from this size on run on the grouped GEMM. Zero-point blobs from a third of the symmetric formats' size on: their streaming
 // kernels take twice the MMAs and four pairs a pass (96 tokens: 256 us a layer against 237, 240 tokens 491 against 274; the symmetric
 // formats 192 against 204 at 240 tokens, 232 against 219 at 320).
-static int grouped_min_tokens(const moexb_ctx* c, int fmt) { return fmt == FMT_ZP ? (c->prefill_min_tokens + 2) / 3 : c->prefill_min_tokens; }
+static int grouped_min_tokens(const moexb_ctx* c, int fmt) {
+    const int t = c->prefill_min_tokens;
+    return fmt == FMT_ZP ? t / 3 + (t % 3 != 0) : t;   // (any threshold up to the largest int)
+}
 
 // Pairs per tile of the grouped GEMM.
 static int grouped_maxp(int fmt) { return fmt == FMT_ZP ? gg_nmax<FMT_ZP>() : gg_nmax<FMT_SYM_F16>(); }

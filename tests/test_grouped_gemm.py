@@ -37,3 +37,29 @@ def test_grouped_gemm_edges(fmt, block):
                 check_ffn(got, xf + ref if block else ref, fmt, f"grouped GEMM T={T} {x.dtype} block={block}")
     finally:
         L.close(); c.close()
+
+
+@pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_ZP])
+def test_a_threshold_of_any_size_keeps_batches_on_the_streaming_kernels(fmt):
+    """Thresholds whose third, rounded up, would pass the largest int: the outputs are those of the streaming kernels bit for bit. (The
+    grouped GEMM adds the products of a group in another order, so its outputs differ somewhere; that is checked first.)"""
+    T = 40
+    c = m.Context(0, max_tokens=T, max_experts=E, top_k=K)
+    L = m.Layer(c, fmt, E)
+    L.fill_synth(3, 0)
+    rng = np.random.default_rng(7)
+    L.set_router((rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32))
+    X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(DEV)
+    try:
+        streaming = L.forward(X, T, K).clone()   # 40 tokens: below the default threshold of either format
+        c.set_prefill_min_tokens(1)
+        assert not torch.equal(L.forward(X, T, K), streaming)
+        for tokens in (2**31 - 1, 2**31 - 2, 2**31 - 3, 3 * T + 1):
+            c.set_prefill_min_tokens(tokens)
+            assert torch.equal(L.forward(X, T, K), streaming), tokens
+        for tokens in (3 * T, 3 * T - 2) if fmt == m.FMT_ZP else (T,):   # the smallest batch that the grouped GEMM takes
+            c.set_prefill_min_tokens(tokens)
+            assert not torch.equal(L.forward(X, T, K), streaming), tokens
+        assert c.status() == 0
+    finally:
+        L.close(); c.close()
