@@ -372,8 +372,14 @@ __global__ void __launch_bounds__(256) split_rows_k(const float* __restrict__ x,
     pdl_trigger();
     const int r = blockIdx.x, k = 8 * threadIdx.x;
     if (r == rows) { side_plan(plan); return; }
-    const float4 p = *reinterpret_cast<const float4*>(x + (size_t)r * EH + k), q = *reinterpret_cast<const float4*>(x + (size_t)r * EH + k + 4);
-    const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+    const float* src = x + (size_t)r * EH + k;
+    float v[8];
+    if (!(reinterpret_cast<uintptr_t>(x) & 15)) {
+        const float4 p = *reinterpret_cast<const float4*>(src), q = *reinterpret_cast<const float4*>(src + 4);
+        v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3] = p.w; v[4] = q.x; v[5] = q.y; v[6] = q.z; v[7] = q.w;
+    } else   // the caller's rows may begin at any float
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = src[i];
     uint16_t hi[8], lo[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) split_hi_lo<false>(v[i], hi[i], lo[i]);

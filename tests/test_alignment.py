@@ -1,0 +1,59 @@
+"""Activation rows that do not begin on a 16-byte boundary, as a view into a larger buffer gives them: the calls take them and give the
+results of aligned rows bit for bit. Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+import moe_b200 as m
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("lib_built")]
+DEV, E, K = "cuda:0", 32, 8
+
+
+def shifted(x, elements):
+    """The same values, `elements` places behind an aligned address."""
+    buf = torch.empty(x.numel() + elements, device=x.device, dtype=x.dtype)
+    view = buf[elements:].view(x.shape)
+    view.copy_(x)
+    assert view.data_ptr() % 16 == elements * x.element_size() % 16
+    return view
+
+
+@pytest.fixture(scope="module")
+def blobs():
+    """A context and a layer of every format in the reference layout."""
+    c = m.Context(0, max_tokens=16, max_experts=E, top_k=K)
+    layers = {}
+    for fmt in (m.FMT_SYM_F16, m.FMT_SYM_F32, m.FMT_ZP):
+        layers[fmt] = m.Layer(c, fmt, E, layout=m.LAYOUT_REFERENCE)
+        layers[fmt].fill_synth(6, 0)
+    yield c, layers
+    for L in layers.values():
+        L.close()
+    c.close()
+
+
+@pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_SYM_F32, m.FMT_ZP])
+def test_pairs_and_one_token_calls(blobs, fmt):
+    c, layers = blobs
+    L, T = layers[fmt], 5
+    g = torch.Generator(device=DEV).manual_seed(1)
+    X = torch.randn(T, 2048, device=DEV, generator=g)
+    idx = torch.rand(T, E, device=DEV, generator=g).topk(K, dim=1).indices.to(torch.int32).contiguous()
+    w = torch.rand(T, K, device=DEV, generator=g)
+    items, pairs, _ = m.group_pairs(idx, w, T, K, E, L.slot_table())
+    slots = torch.tensor([L.blob_ptr(int(e)) for e in idx[0]], dtype=torch.int64, device=DEV)
+
+    def both(x):
+        y = c.pairs_forward_tc(fmt, items, E, pairs, x, T, T * K, None, torch.zeros(T * K, 2048, device=DEV))
+        return y.cpu().numpy(), m.experts_forward(fmt, slots, w[0].contiguous(), K, x[0]).cpu().numpy()
+
+    c.make_default()
+    try:
+        want = both(X)
+        for elements in (1, 2, 3):
+            for a, b in zip(both(shifted(X, elements)), want):
+                assert np.array_equal(a, b), elements
+        assert c.status() == 0
+    finally:
+        c.make_default(False)
