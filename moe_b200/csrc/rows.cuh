@@ -58,8 +58,9 @@ __device__ __forceinline__ float store_split4(const float (&f)[4], int k0, uint1
     return sum;
 }
 __device__ __forceinline__ float4 ld_x4(const float* x) { return __ldg(reinterpret_cast<const float4*>(x)); }
+// (two 4-byte loads: bf16 rows of a caller are 4-byte aligned, no more)
 __device__ __forceinline__ float4 ld_x4(const __nv_bfloat16* x) {
-    const uint2 u = __ldg(reinterpret_cast<const uint2*>(x));
+    const uint2 u = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(x)), __ldg(reinterpret_cast<const uint32_t*>(x) + 1));
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xFFFF0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xFFFF0000u));
 }
 

@@ -57,3 +57,24 @@ def test_pairs_and_one_token_calls(blobs, fmt):
         assert c.status() == 0
     finally:
         c.make_default(False)
+
+
+@pytest.mark.parametrize("fmt,min_tokens", [(m.FMT_SYM_F16, 1 << 20), (m.FMT_ZP, 1 << 20), (m.FMT_SYM_F16, 1), (m.FMT_ZP, 1)])
+@pytest.mark.parametrize("flags", [0, 2])
+def test_bf16_rows_of_a_layer(fmt, min_tokens, flags):
+    """bf16 rows on a 4-byte boundary, through the routing kernel (fewer than 8 tokens) and the kernel that prepares the rows."""
+    c = m.Context(0, max_tokens=16, max_experts=E, top_k=K)
+    c.set_prefill_min_tokens(min_tokens)
+    L = m.Layer(c, fmt, E)
+    L.fill_synth(6, 0)
+    rng = np.random.default_rng(2)
+    L.set_router((rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32))
+    try:
+        for T in (1, 3, 16):
+            X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(DEV).to(torch.bfloat16)
+            want = L.forward(X, T, K, flags=flags).cpu().numpy()
+            for elements in (2, 4, 6):
+                assert np.array_equal(L.forward(shifted(X, elements), T, K, flags=flags).cpu().numpy(), want), (T, elements)
+        assert c.status() == 0
+    finally:
+        L.close(); c.close()
