@@ -304,7 +304,7 @@ int moexb_layer_load_st(moexb_layer* layer, const moexb_st* s, const char* prefi
 /* One MoE layer for T tokens: router logits -> top-K softmax (renormalised) -> routed experts -> rank-order combine ->
  * + sigmoid(gate) * shared expert. X [T][H] of x_dtype; out [T][H] f32. The sequence the reference runs at
  * moex.cu:1093-1107 (decode) and moex.cu:1414-1415, 1466-1617 (chunk). Optional outputs (may be null): idx_out [T][K],
- * w_out [T][K]. flags bit 0: skip the shared expert; bit 1: X is the layer input before RMSNorm, so normalise it first
+ * w_out [T][K]. X begins on a 16-byte boundary (f32) or on a 4-byte one (bf16), out on a 16-byte one. flags bit 0: skip the shared expert; bit 1: X is the layer input before RMSNorm, so normalise it first
  * (unit weight, eps 1e-6) and write out = X + moe(norm(X)) - the residual block the 40-layer stack chains. */
 int moexb_layer_forward(moexb_ctx* ctx, moexb_layer* layer, const void* X, int x_dtype, int T, int K, float* out,
                         int* idx_out, float* w_out, int flags, void* stream);
@@ -362,7 +362,7 @@ int moexb_ep_read_routing(moexb_ep* ep, int* idx_out, float* w_out, void* stream
  *   dispatch    l == 0: takes the own rows of X [T][H] (x_dtype; every rank passes the whole batch); l > 0: adds up layer
  *               l - 1 for the own tokens (waits for the peers' partial rows). Then normalises (residual != 0: the blocks
  *               x_{l+1} = x_l + moe_l(rmsnorm(x_l)); residual == 0: the plain layer moe(X), single layer only), routes the
- *               own tokens and sends ids, weights and activation rows.
+ *               own tokens and sends ids, weights and activation rows. X may begin on any 4-byte boundary.
  *   experts     waits for all ranks' dispatch of layer l, runs the pairs of the experts held here (and the shared expert for
  *               the own tokens) and sends the partial rows to the token owners.
  *   finish      adds up the last layer: out_own [own tokens][H] f32. */

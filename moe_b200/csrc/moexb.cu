@@ -1803,8 +1803,10 @@ int moexb_ep_dispatch(moexb_ep* e, moexb_layer* L, int l, const void* X, int x_d
         float* dst = residual ? e->x : xn_own;
         const size_t n = (size_t)n_own * EH;
         const uint8_t* own = static_cast<const uint8_t*>(X) + (size_t)t0 * EH * (x_dtype == MOEXB_BF16 ? 2 : 4);
-        if (x_dtype == MOEXB_F32) CUDA_TRY(cudaMemcpyAsync(dst, own, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
-        rc = layer_rows(c, own, x_dtype, n_own, dst, residual != 0, xn_own, mode, c->xs + (size_t)t0 * parts * EH, parts, stream);
+        const bool f32 = x_dtype == MOEXB_F32;
+        if (f32) CUDA_TRY(cudaMemcpyAsync(dst, own, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        // f32 rows are read from the copy: the caller's may begin at any float
+        rc = layer_rows(c, f32 ? static_cast<const void*>(dst) : own, x_dtype, n_own, dst, residual != 0, xn_own, mode, c->xs + (size_t)t0 * parts * EH, parts, stream);
         if (rc != MOEXB_OK) return rc;
     } else {
         rc = ep_combine(e, f16, residual != 0, (unsigned)l, nullptr, true, !prefill, stream);

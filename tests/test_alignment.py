@@ -78,3 +78,35 @@ def test_bf16_rows_of_a_layer(fmt, min_tokens, flags):
         assert c.status() == 0
     finally:
         L.close(); c.close()
+
+
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("min_tokens", [1 << 20, 1])
+def test_rows_of_an_expert_parallel_step(residual, min_tokens):
+    """f32 rows at any float and bf16 rows on a 4-byte boundary as the input of a step (one rank)."""
+    T = 9
+    c = m.Context(0, max_tokens=T, max_experts=E, top_k=K)
+    c.set_prefill_min_tokens(min_tokens)
+    L = m.Layer(c, m.FMT_SYM_F16, E)
+    L.fill_synth(6, 0)
+    rng = np.random.default_rng(3)
+    L.set_router((rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32))
+    buf = m.ExchangeBuffer(T, K, 1)
+    ep = m.EP(c, 0, 1, T, K, E, [buf.ptr])
+    try:
+        X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(DEV)
+        for x, places in ((X, (1, 2, 3)), (X.to(torch.bfloat16), (2, 4, 6))):
+            def step(rows):
+                ep.begin_step()
+                ep.dispatch(L, 0, rows, residual)
+                ep.experts(L, 0)
+                out = torch.empty(T, 2048, device=DEV)
+                ep.finish(1, out, residual)
+                return out.cpu().numpy()
+            want = step(x)
+            assert np.isfinite(want).all() and want.any()
+            for elements in places:
+                assert np.array_equal(step(shifted(x, elements)), want), (x.dtype, elements)
+        assert c.status() == 0
+    finally:
+        ep.close(); L.close(); c.close(); buf.close()
