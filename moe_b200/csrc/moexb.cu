@@ -210,9 +210,11 @@ template <typename WT>
 static int gemv_any(const WT* W, const float* x, float* y, int I, int O, void* stream, int rows) {
     REQUIRE(W && x && y, "gemv: null pointer");
     REQUIRE(I > 0 && I % 128 == 0 && O > 0 && rows > 0, "gemv: I=%d must be a positive multiple of 128, O=%d, rows=%d", I, O, rows);
-    // A warp per (row, output) re-reads the weights from L2 for every row, which up to 24 rows costs less than the tiles of the batched
-    // kernel, of which a small batch has too few to reach every SM (16 rows: 3 us against 19).
-    if (rows > 24) {
+    // A warp per (row, output) re-reads the weights from L2 for every row; the batched kernel's tiles read them once per 8 rows, but of
+    // them a small batch has too few to reach every SM. In a chain of calls (f16 / f32 weights, us): 8 rows 3.1 / 3.2 against 6.0 / 5.7,
+    // 14 rows 5.2 / 5.2 against 6.0 / 5.7, 16 rows 5.6 / 5.6 against 6.0 / 5.8, 20 rows 6.6 / 6.8 against 6.0 / 5.8; with weights that
+    // come from memory the lines cross at 16 (a chunk of 16 tokens over 2 layers: 187 us against 184).
+    if (rows >= 16) {
         constexpr int WARPS = 8, TO = 2, TR = 8;  // 16 outputs x 8 rows per block: 17 x 8 blocks for the 64-token router
         const int smem = TR * I * (int)sizeof(float);
         REQUIRE(smem <= 200 * 1024, "gemv: I=%d is too large for the batched kernel", I);

@@ -12,6 +12,13 @@ __device__ __forceinline__ float4 ld_w4(const __half* W, size_t k) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// Asks for a row of weights in L2. Weights that the kernel before this one may still write cannot be loaded before the wait for it, but
+// they can be brought this far: what is written meanwhile arrives in L2 too.
+template <typename WT>
+__device__ __forceinline__ void prefetch_row(const WT* w, int I, int lane) {
+    for (int b = 128 * lane; b < I * (int)sizeof(WT); b += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(w) + b));
+}
+
 // y[r][o] = W[o] . x[r]. One warp per (row r, output o): lane j accumulates elements 128c+4j .. 128c+4j+3 for
 // c = 0, 1, .. with fused multiply-adds in ascending order, then a xor-butterfly (16, 8, 4, 2, 1) adds the 32 partial
 // sums. The CPU oracle follows the same order, so the logits - and with them the selected experts - agree bit for bit.
@@ -25,30 +32,17 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_rows_k(const WT* __restrict__
     const WT* wr = W + (size_t)o * I;
     float acc = 0.f;
     constexpr int U = 16;  // loads of U steps are in flight before the first multiply-add; the summation order is unchanged
-    auto steps = [&](int c0, const float4 (&w)[U]) {
-        float4 v[U];
+    if (blockIdx.y == 0) prefetch_row(wr, I, lane);
+    pdl_wait();
+    pdl_trigger();
+    for (int c0 = 0; c0 < I / 128; c0 += U) {
+        float4 w[U], v[U];
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (c0 + u < I / 128) v[u] = __ldg(reinterpret_cast<const float4*>(xr + 128 * (c0 + u) + 4 * lane));
+            if (c0 + u < I / 128) { w[u] = ld_w4(wr, (size_t)128 * (c0 + u) + 4 * lane); v[u] = __ldg(reinterpret_cast<const float4*>(xr + 128 * (c0 + u) + 4 * lane)); }
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (c0 + u < I / 128) { acc = fmaf(w[u].x, v[u].x, acc); acc = fmaf(w[u].y, v[u].y, acc); acc = fmaf(w[u].z, v[u].z, acc); acc = fmaf(w[u].w, v[u].w, acc); }
-    };
-    {   // the weights of the first U steps do not depend on the kernel before this one: they are requested before the wait
-        float4 w[U];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-            if (u < I / 128) w[u] = ld_w4(wr, (size_t)128 * u + 4 * lane);
-        pdl_wait();
-        pdl_trigger();
-        steps(0, w);
-    }
-    for (int c0 = U; c0 < I / 128; c0 += U) {
-        float4 w[U];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-            if (c0 + u < I / 128) w[u] = ld_w4(wr, (size_t)128 * (c0 + u) + 4 * lane);
-        steps(c0, w);
     }
     acc = warp_sum(acc);
     if (lane == 0) y[(size_t)blockIdx.y * O + o] = acc;
@@ -57,7 +51,8 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_rows_k(const WT* __restrict__
 // One tile of the batched rows: a block stages TR activation rows in shared memory and its WARPS warps each own TO outputs, with the
 // weights of U steps requested at a time and the next U already in flight; a lane still holds elements 128c+4j..4j+3 of every dot
 // product, so every (row, output) sum is formed in exactly the order of gemv_rows_k and the kernels agree bit for bit.
-// Waits for the kernel before (pdl_wait); EARLY: only once its first weights, which that kernel must not write, are requested. Dynamic shared memory TR * I floats.
+// Waits for the kernel before (pdl_wait); EARLY: only once its first weights, which that kernel must not write, are requested.
+// Dynamic shared memory TR * I floats.
 template <typename WT, int WARPS, int TO, int TR, bool EARLY>
 __device__ __forceinline__ void gemm_tile(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int I, int O, int rows) {
     extern __shared__ __align__(16) float xsm[];  // [TR][I]
@@ -78,6 +73,9 @@ __device__ __forceinline__ void gemm_tile(const WT* __restrict__ W, const float*
                 if (c0 + u < I / 128) wn[i][u] = ld_w4(wr[i], (size_t)128 * (c0 + u) + 4 * lane);
     };
     if (EARLY) load_w(0);
+    else if (blockIdx.y == 0)
+#pragma unroll
+        for (int i = 0; i < TO; i++) prefetch_row(wr[i], I, lane);
     pdl_wait();
     pdl_trigger();
     if (!EARLY) load_w(0);

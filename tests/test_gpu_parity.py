@@ -84,6 +84,24 @@ def test_router_logits_bit_exact(rows, O):
     assert np.array_equal(m.gemv_f16(dev(W16), dev(x), rows=rows).cpu().numpy(), o.router_logits(W16, x, rows))
 
 
+@pytest.mark.parametrize("rows", [1, 15, 16, 33])
+def test_router_weights_written_by_the_kernel_before(rows):
+    """The weights of a pointer-level call may be the output of the kernel before it, here of a combine whose launch lets the next
+    kernel start early: every call sees the weights of its own turn."""
+    O = 4096
+    rng = np.random.default_rng(rows)
+    src = [dev(rng.standard_normal((O, 2048)).astype(np.float32)) for _ in range(2)]
+    x = dev(rng.standard_normal((rows, 2048)).astype(np.float32))
+    want = [m.gemv_f32(s, x, rows=rows).clone() for s in src]
+    W, y = torch.empty(O, 2048, device=DEV), torch.empty(8, rows, O, device=DEV)
+    torch.cuda.synchronize()
+    for i in range(8):
+        m.pairs_reduce(src[i & 1], None, W, 1, 2048, O)   # a copy of src into W
+        m.gemv_f32(W, x, y[i], rows=rows)
+    for i in range(8):
+        assert torch.equal(y[i], want[i & 1]), i
+
+
 @pytest.mark.parametrize("T,E,K,ld", [(1, 256, 8, 257), (7, 256, 8, 256), (64, 256, 8, 257), (3, 32, 4, 40), (2, 1024, 15, 1024)])
 def test_router_topk(T, E, K, ld):
     rng = np.random.default_rng(T + E)
