@@ -406,6 +406,9 @@ int moexb_stack_kernel_count(moexb_stack* stack);
 
 /* Kernels launched by this library in this process so far (graph replays count their kernel nodes). */
 long long moexb_launch_count(void);
+/* Expert kernels launched so far in this process of which an SM takes fewer CTAs than their grids are sized for: 0, or a kernel has
+ * outgrown the SM's shared memory or registers. */
+int moexb_short_residency(void);
 
 enum { MOEXB_PROF_ROUTER = 0, MOEXB_PROF_TOPK = 1, MOEXB_PROF_GROUP = 2, MOEXB_PROF_GATE_UP = 3, MOEXB_PROF_DOWN = 4,
        MOEXB_PROF_COMBINE = 5, MOEXB_PROF_OTHER = 6, MOEXB_PROF_TAGS = 7 };

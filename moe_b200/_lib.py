@@ -111,6 +111,7 @@ SIGNATURES = {
     "moexb_stack_run_host": (_i, [_vp, _vp, _vp, _vp]),
     "moexb_stack_kernel_count": (_i, [_vp]),
     "moexb_launch_count": (_ll, []),
+    "moexb_short_residency": (_i, []),
     "moexb_ctx_profile": (_i, [_vp, _i]),
     "moexb_ctx_profile_read": (_i, [_vp, _vp, _vp]),
 }

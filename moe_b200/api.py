@@ -476,3 +476,8 @@ class Stack:
 
 def launch_count():
     return lib().moexb_launch_count()
+
+
+def short_residency():
+    """moexb_short_residency: expert kernels of which an SM takes fewer CTAs than their grids are sized for (0 expected)."""
+    return lib().moexb_short_residency()

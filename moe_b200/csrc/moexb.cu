@@ -92,6 +92,16 @@ struct PerDeviceOnce {
         return err[dev];
     }
 };
+// The opt-in of a kernel to `smem` bytes of dynamic shared memory. Its grid is sized for `ctas` CTAs per SM: kernels of which fewer fit
+// are counted (moexb_short_residency); they run, but what does not fit waits for a second wave.
+std::atomic<int> g_short_residency{0};
+template <typename K>
+static cudaError_t opt_in(K* kernel, int threads, int smem, int ctas) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    int fit = 0;
+    if (e == cudaSuccess && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, smem) == cudaSuccess && fit < ctas) g_short_residency++;
+    return e;
+}
 inline bool fmt_ok(int fmt) { return fmt == FMT_SYM_F32 || fmt == FMT_SYM_F16 || fmt == FMT_ZP; }
 
 // Calls f.template operator()<FMT>() for the run-time format.
@@ -1018,7 +1028,7 @@ static int stream_launch_one(moexb_ctx* c, const StreamArgs& a, void* stream) {
     constexpr int NW = 4, CPS = 3, STAGES = DOWN ? 3 : 2;
     constexpr int SMEM = st_smem_bytes<FMT, DOWN, NW, STAGES>();
     static PerDeviceOnce once;
-    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(stream_k<FMT, DOWN, NW, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
+    const cudaError_t attr_err = once.run([] { return opt_in(stream_k<FMT, DOWN, NW, STAGES>, (NW + ST_NP) * 32, SMEM, CPS); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "stream kernel shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
     static_assert(SMEM * CPS <= 227 * 1024, "shared memory of the resident CTAs");
@@ -1043,9 +1053,9 @@ static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float*
 template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC>
 static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa, const BucketArgs& ba, void* stream) {
     constexpr int SMEM = tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC>();
-    static_assert(SMEM * CPS <= 227 * 1024, "shared memory of the resident CTAs");
+    static_assert(tl_fits<FMT, DOWN, NW, D, NB, CPS, SRC>(), "shared memory of the resident CTAs");
     static PerDeviceOnce once;
-    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
+    const cudaError_t attr_err = once.run([] { return opt_in(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, NW * 32, SMEM, CPS); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "tiled stream kernel shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
     CUDA_TRY(launch_dep(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, CPS * c->sms, NW * 32, SMEM, S(stream), a, pa, ba));
@@ -1104,7 +1114,7 @@ template <int FMT, bool DOWN>
 static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, const GroupedMaps& maps, void* stream) {
     constexpr int SMEM = gg_smem_bytes<FMT>();
     static PerDeviceOnce once;
-    const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(grouped_k<FMT, DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
+    const cudaError_t attr_err = once.run([] { return opt_in(grouped_k<FMT, DOWN>, GG_THREADS, SMEM, 1); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "grouped GEMM shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
     CUDA_TRY(launch_dep(grouped_k<FMT, DOWN>, c->sms, GG_THREADS, SMEM, S(stream), a, maps));
@@ -1401,7 +1411,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
         ranks = K + 1;
     } else {
         const int maxp = prefill ? grouped_maxp(L->fmt) : (tiled ? tiled_maxp(c, L->fmt, T) : ST_MAXP);
-        const BucketArgs bk{c->bcnt, c->bpairs, c->max_tokens, E, shared ? sh0 : 0, shared ? sh1 : 0, maxp, L->slot_table};
+        const BucketArgs bk{c->bcnt, c->bpairs, c->max_tokens, E, shared ? sh0 : 0, shared ? sh1 : 0, maxp, L->image - L->first_local * expert_bytes(L->fmt), L->slot_host[E]};
         if (!buckets) {
             PROF(c, MOEXB_PROF_GROUP, stream);
             // room in shared memory for the routed pairs (12 bytes each), so that the list is written out in full lines
@@ -1910,6 +1920,7 @@ int moexb_ep_stack_create(moexb_ep* e, moexb_layer* const* layers, int n_layers,
 // ---- instrumentation ------------------------------------------------------------------------------------------------------
 
 long long moexb_launch_count(void) { return g_launches.load(); }
+int moexb_short_residency(void) { return g_short_residency.load(); }
 
 int moexb_ctx_profile(moexb_ctx* c, int on) {
     REQUIRE(c, "ctx_profile: null context");

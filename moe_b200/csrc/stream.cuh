@@ -717,21 +717,18 @@ struct BucketArgs {
     const int* cnt;                   // [E] pairs of each expert
     const moexb_pair* pairs;          // [E + 1][stride]; the last bucket is the shared expert's, place t = token t
     int stride, E, sh0, sh1, maxp;    // the shared expert takes the tokens [sh0, sh1); sub-items of at most maxp pairs
-    const uint8_t* const* slot_table; // E + 1 blob pointers
+    const uint8_t *routed, *shared;   // expert 0's blob, were it held here (only held experts have pairs), and the shared expert's
 };
+// The blobs' places are computed, not kept: with a table of 257 pointers more the zero-point kernels do not fit twice on an SM (a layer of
+// 4, 40, 64 tokens: 51, 173, 205 us with the table, 43, 161, 191 without; f16 scales 64 tokens 102.8 and 102.9, f32 scales 103.0 and 103.1).
 struct BucketSmem {
-    const uint8_t* slot[BK_MAX_E + 1];
     int wide[BK_MAX_E + 2], narrow[BK_MAX_E + 2];   // sub-items of more than maxp / 2 pairs, and of fewer, before expert e
     int cnt[BK_MAX_E + 1];
     moexb_pair_item local[BK_LOCAL];                // a CTA's own range of sub-items
 };
-// What does not depend on the router: the blob pointers. A CTA barrier must follow.
-__device__ __forceinline__ void bucket_prepare(BucketSmem& L, const BucketArgs& a) {
-    for (int i = threadIdx.x; i <= a.E; i += blockDim.x) L.slot[i] = a.slot_table[i];
-}
 // By one warp, after the wait for the router. A CTA barrier must follow.
 __device__ __forceinline__ void bucket_scan(BucketSmem& L, const BucketArgs& a, int lane) {
-    const int Ts = L.slot[a.E] ? a.sh1 - a.sh0 : 0, maxp = a.maxp;
+    const int Ts = a.sh1 - a.sh0, maxp = a.maxp;
     const unsigned rcp = 0xFFFFFFFFu / maxp + 1;   // c / maxp = the high half of c * rcp, exact for the counts (below 65536)
     auto wide = [=](int c) { const int full = __umulhi(c, rcp); return full + (c - full * maxp > maxp / 2); };
     auto narrow = [=](int c) { const int r = c - (int)__umulhi(c, rcp) * maxp; return (int)(r > 0 && r <= maxp / 2); };
@@ -760,6 +757,7 @@ __device__ __forceinline__ void bucket_scan(BucketSmem& L, const BucketArgs& a, 
     if (lane == 31) { L.wide[a.E] = bw; L.narrow[a.E] = bn; L.cnt[a.E] = Ts; L.wide[a.E + 1] = bw + wide(Ts); L.narrow[a.E + 1] = bn + narrow(Ts); }
 }
 // Sub-item i: the wide ones of all experts first.
+template <int FMT>
 __device__ __forceinline__ moexb_pair_item bucket_sub(const BucketSmem& L, const BucketArgs& a, int i) {
     const int nw = L.wide[a.E + 1];
     const bool w = i < nw;
@@ -768,7 +766,7 @@ __device__ __forceinline__ moexb_pair_item bucket_sub(const BucketSmem& L, const
     int lo = 0, hi = a.E;   // the last e with pre[e] <= at
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (pre[mid] <= at) lo = mid; else hi = mid - 1; }
     const int c = L.cnt[lo], j = w ? at - pre[lo] : L.wide[lo + 1] - L.wide[lo];
-    return {L.slot[lo], lo * a.stride + (lo == a.E ? a.sh0 : 0) + j * a.maxp, min(a.maxp, c - j * a.maxp)};
+    return {lo == a.E ? a.shared : a.routed + (size_t)lo * expert_bytes(FMT), lo * a.stride + (lo == a.E ? a.sh0 : 0) + j * a.maxp, min(a.maxp, c - j * a.maxp)};
 }
 
 // Self-test of the bounded waits (moexb_ctx_selftest_timeout): one warp waits on an mbarrier that expects 16 bytes which

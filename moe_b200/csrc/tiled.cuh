@@ -209,6 +209,8 @@ __device__ __forceinline__ void plan_in_cta(PlanSmem& L, PlanTmp& P, const PlanA
     __syncthreads();   // also: the scratch is free for the first weight copies
 }
 
+// zero point: sums of the activations, [K slice][group][chunk][8 columns]
+template <int FMT, bool DOWN> constexpr int tl_csum_floats() { return FMT == FMT_ZP ? (DOWN ? 1 : 4) * 8 * 2 * 8 : 4; }
 struct TiledArgs {
     const moexb_pair_item* subs;  // sub-items: at most 4 * NB pairs each, slot = tiled blob
     const int* nsub;
@@ -252,12 +254,11 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     BucketSmem& L = *reinterpret_cast<BucketSmem*>(bars + NW * D + 8);
     static_assert(!PLAN || sizeof(PlanTmp) <= NW * D * SB, "the planning scratch fits where the ring will be");
     // zero point: the sum of the activations over each 32-input chunk, per column: [K slice][group][chunk][8 columns]
-    __shared__ __align__(16) float csum[Z ? KS * 8 * 2 * 8 : 4];
+    __shared__ __align__(16) float csum[tl_csum_floats<FMT, DOWN>()];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     if (threadIdx.x < NW * D) mbar_init(smem_u32(bars + threadIdx.x), 1);
     if (threadIdx.x == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if constexpr (PLAN) plan_prepare(P, *reinterpret_cast<PlanTmp*>(smem), pa);
-    if constexpr (BUCKETS) bucket_prepare(L, ba);
     __syncthreads();
     // Gate/up: the sub-items come from the kernel before this one. Down: they are older (the gate/up kernel read them
     // too), so the weight copies start while gate/up still runs; only the activation columns wait for it.
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
         __syncthreads();
         if (blockIdx.x == 0) {   // the list for the down kernel, which may read it as soon as every CTA here has triggered
             const int nw = L.wide[ba.E + 1], n = nw + L.narrow[ba.E + 1];
-            for (int i = threadIdx.x; i < n; i += NW * 32) pa.subs_out[i] = bucket_sub(L, ba, i);
+            for (int i = threadIdx.x; i < n; i += NW * 32) pa.subs_out[i] = bucket_sub<FMT>(L, ba, i);
             if (threadIdx.x < 2) pa.nsub_out[threadIdx.x] = threadIdx.x ? nw : n;
             __threadfence();
             __syncthreads();
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     // the work list: the CTA's own (PLAN) or the one in global memory
     auto sub_at = [&](int i) -> moexb_pair_item {
         if constexpr (PLAN) { const PlanSub su = P.subs[i]; return {P.slot[su.e], su.start, su.count}; }
-        else if constexpr (BUCKETS) return i < first_sub + BK_LOCAL ? L.local[i - first_sub] : bucket_sub(L, ba, i);
+        else if constexpr (BUCKETS) return i < first_sub + BK_LOCAL ? L.local[i - first_sub] : bucket_sub<FMT>(L, ba, i);
         else return a.subs[i];
     };
     auto pair_at = [&](int i) -> moexb_pair { if constexpr (PLAN) return P.pair_at(i); else return a.pairs[i]; };
@@ -310,7 +311,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     if constexpr (BUCKETS) {
         first_sub = r0 / RPS;
         const int i = first_sub + threadIdx.x;
-        if (threadIdx.x < BK_LOCAL && r1 > r0 && i <= (r1 - 1) / RPS) L.local[threadIdx.x] = bucket_sub(L, ba, i);
+        if (threadIdx.x < BK_LOCAL && r1 > r0 && i <= (r1 - 1) / RPS) L.local[threadIdx.x] = bucket_sub<FMT>(L, ba, i);
         __syncthreads();
     }
     uint8_t* ring = smem + warp * D * SB;
@@ -494,5 +495,8 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
 
 template <int FMT, bool DOWN, int NW, int D, int NB = 1, int SRC = TL_LIST>
 constexpr int tl_smem_bytes() { return NW * D * tl_slice_bytes<FMT>() + 8 * NB * st_bcol_bytes<DOWN>() + NW * D * 8 + 64 + (SRC == TL_PLAN ? (int)sizeof(PlanSmem) + 16 : SRC == TL_BUCKETS ? (int)sizeof(BucketSmem) + 16 : 0); }
+// Whether CPS CTAs fit on an SM: 228 KB of shared memory, of which a CTA also takes its static part and 1 KB of the system's.
+template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC>
+constexpr bool tl_fits() { return (tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC>() + tl_csum_floats<FMT, DOWN>() * 4 + 1024) * CPS <= 228 * 1024; }
 
 }  // namespace moexb

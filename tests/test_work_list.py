@@ -87,3 +87,24 @@ def test_a_call_that_failed_after_its_router_leaves_nothing_behind(fmt, T):
         check_ffn(before, ref, fmt, f"{T} tokens before and after failed calls")
     finally:
         stack.close(); L.close(); c.close()
+
+
+@pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_SYM_F32, m.FMT_ZP])
+@pytest.mark.parametrize("layout", [m.LAYOUT_TILED, m.LAYOUT_REFERENCE])
+def test_the_expert_kernels_are_resident_as_often_as_their_grids_assume(fmt, layout):
+    """Work list from the buckets, from a planning launch (288 experts) and one token's own; both widths of a pass; the grouped GEMM."""
+    K = 8
+    for E in (32, 288):
+        c = m.Context(0, max_tokens=16, max_experts=E, top_k=K)
+        L = m.Layer(c, fmt, E, layout=layout)
+        L.fill_synth(1, 0)
+        L.set_router(np.zeros((E + 1, 2048), np.float32))
+        try:
+            for T, pairs, min_tokens in ((1, 8, 256), (3, 8, 256), (16, 8, 256), (16, 4, 256), (16, 8, 1)):
+                c.set_pairs_per_pass(pairs)
+                c.set_prefill_min_tokens(min_tokens)
+                L.forward(torch.zeros(T, 2048, device=DEV), T, K)
+            assert c.status() == 0
+        finally:
+            L.close(); c.close()
+    assert m.short_residency() == 0
