@@ -53,12 +53,9 @@ __global__ void __launch_bounds__(WARPS * 32) gemv_rows_k(const WT* __restrict__
 // product, so every (row, output) sum is formed in exactly the order of gemv_rows_k and the kernels agree bit for bit.
 // Waits for the kernel before (pdl_wait); EARLY: only once its first weights, which that kernel must not write, are requested.
 // Dynamic shared memory TR * I floats.
-template <typename WT, int WARPS, int TO, int TR, bool EARLY>
+template <typename WT, int WARPS, int TO, int TR, int U, bool EARLY>
 __device__ __forceinline__ void gemm_tile(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int I, int O, int rows) {
     extern __shared__ __align__(16) float xsm[];  // [TR][I]
-    // steps per batch of weights: the small tile takes 8 (half of I = 2048) - the first batch, requested before the wait,
-    // arrives while the kernel before this one still runs (all 16 at once would spill)
-    constexpr int U = TO <= 2 ? 8 : 4;
     const int r0 = blockIdx.y * TR, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int o0 = (blockIdx.x * WARPS + warp) * TO;
     const WT* wr[TO];
@@ -123,10 +120,10 @@ __device__ __forceinline__ void gemm_tile(const WT* __restrict__ W, const float*
 
 // The same result for many rows (a batch or a prefill chunk).
 // grid (ceil(O / (WARPS*TO)), ceil(rows / TR)); dynamic shared memory TR * I floats.
-template <typename WT, int WARPS, int TO, int TR>
+template <typename WT, int WARPS, int TO, int TR, int U>
 __global__ void __launch_bounds__(WARPS * 32) gemm_rows_k(const WT* __restrict__ W, const float* __restrict__ x,
                                                           float* __restrict__ y, int I, int O, int rows) {
-    gemm_tile<WT, WARPS, TO, TR, false>(W, x, y, I, O, rows);
+    gemm_tile<WT, WARPS, TO, TR, U, false>(W, x, y, I, O, rows);
 }
 
 // Softmax over E logits and the K largest by one warp (kernels.cuh:373-406 does it with a block per token).
@@ -369,7 +366,8 @@ template <typename WT, int WARPS, int TO, int TR, int NJ>
 __global__ void __launch_bounds__(WARPS * 32) route_gemm_k(const WT* __restrict__ W, const float* __restrict__ x, float* __restrict__ y, int I,
                                                            int E, int K, int norm, int T, int* __restrict__ done, const TopkOut o) {
     const int O = E + 1, r0 = blockIdx.y * TR, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    gemm_tile<WT, WARPS, TO, TR, true>(W, x, y, I, O, T);
+    // weights of 8 steps (half of I = 2048) at a time: the first arrive while the kernel before this one still runs (16 would spill)
+    gemm_tile<WT, WARPS, TO, TR, 8, true>(W, x, y, I, O, T);
     if (!last_block_done(done + blockIdx.y, gridDim.x)) return;
     for (int r = warp; r < TR && r0 + r < T; r += WARPS) topk_token<NJ, true>(y + (size_t)(r0 + r) * O, r0 + r, E, K, norm, lane, o);
     ep_raise_dispatch_flags(o, r0, min(TR, T - r0));

@@ -84,6 +84,17 @@ def test_router_logits_bit_exact(rows, O):
     assert np.array_equal(m.gemv_f16(dev(W16), dev(x), rows=rows).cpu().numpy(), o.router_logits(W16, x, rows))
 
 
+@pytest.mark.parametrize("rows,O,I", [(15, 257, 2048), (16, 257, 2048), (64, 257, 2048), (65, 257, 2048), (300, 257, 2048), (1200, 5, 2048), (1200, 17, 384), (17, 2500, 128)])
+def test_router_logits_where_the_tiles_change(rows, O, I):
+    """Per-row kernel, tiles up to one per SM and beyond it, in remainders of 8 rows and 16 outputs, short rows: bit-exact as ever."""
+    rng = np.random.default_rng(rows + O)
+    W = (rng.standard_normal((O, I)) * 0.02).astype(np.float32)
+    x = rng.standard_normal((rows, I)).astype(np.float32)
+    assert np.array_equal(m.gemv_f32(dev(W), dev(x), rows=rows).cpu().numpy(), o.router_logits(W, x, rows))
+    W16 = W.astype(np.float16)
+    assert np.array_equal(m.gemv_f16(dev(W16), dev(x), rows=rows).cpu().numpy(), o.router_logits(W16, x, rows))
+
+
 @pytest.mark.parametrize("rows", [1, 15, 16, 33])
 def test_router_weights_written_by_the_kernel_before(rows):
     """The weights of a pointer-level call may be the output of the kernel before it, here of a combine whose launch lets the next
