@@ -302,7 +302,7 @@ static int decode_launch(moexb_ctx* prof, int fmt, const uint8_t* const* slots, 
 // The context whose workspace the pointer-level one-token entry point may use on each device (moexb_set_default_ctx).
 static std::mutex g_default_lock;
 static moexb_ctx* g_default_ctx[MAX_DEVICES] = {};
-static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, void* stream);
+static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int npairs, void* stream);
 static int split_launch(moexb_ctx* c, const float* x, int rows, void* stream, const SidePlan& plan);
 
 extern "C" {
@@ -334,7 +334,7 @@ int moexb_experts_forward(int fmt, const uint8_t* const* slots, const float* w, 
     int rc = split_launch(c, x, 1, stream, plan);
     if (rc != MOEXB_OK) return rc;
     if (nh) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)K * EH * sizeof(float), st));   // rows of the experts beyond *nh stay zero
-    rc = stream_experts(c, fmt, c->pairs, act, c->ypair, stream);
+    rc = stream_experts(c, fmt, c->pairs, act, c->ypair, K, stream);
     if (rc != MOEXB_OK) return rc;
     CUDA_TRY(launch_dep(pairs_reduce_k, dim3((EH / 4 + 255) / 256, 1), 256, 0, st, (const float*)c->ypair, (const float*)nullptr, out, K, EH, (const int*)nullptr));
     LAUNCHED("pairs_reduce");
@@ -1035,31 +1035,43 @@ int moexb_layer_load_st(moexb_layer* L, const moexb_st* s, const char* prefix, i
 
 // ---- streaming (tensor-core) expert path ------------------------------------------------------------------------------------
 
-template <int FMT, bool DOWN>
-static int stream_launch_one(moexb_ctx* c, const StreamArgs& a, void* stream) {
-    // three CTAs per SM: the 12 consumer warps, not the ring's depth, are what the loop is short of with two
-    constexpr int NW = 4, CPS = 3, STAGES = DOWN ? 3 : 2;
+template <int FMT, bool DOWN, int CPS>
+static int stream_launch_cfg(moexb_ctx* c, const StreamArgs& a, void* stream) {
+    constexpr int NW = ST_NW, STAGES = (DOWN ? 3 : 2) + (CPS == 2);
     constexpr int SMEM = st_smem_bytes<FMT, DOWN, NW, STAGES>();
     static PerDeviceOnce once;
     const cudaError_t attr_err = once.run([] { return opt_in(stream_k<FMT, DOWN, NW, STAGES>, (NW + ST_NP) * 32, SMEM, CPS); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "stream kernel shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
-    static_assert(SMEM * CPS <= 227 * 1024, "shared memory of the resident CTAs");
+    static_assert((SMEM + 1024) * CPS <= 228 * 1024, "shared memory of the resident CTAs");
     CUDA_TRY(launch_dep(stream_k<FMT, DOWN, NW, STAGES>, CPS * c->sms, (NW + ST_NP) * 32, SMEM, S(stream), a));
     LAUNCHED(DOWN ? "stream_down" : "stream_gate_up");
     return MOEXB_OK;
 }
+// CTAs per SM. Symmetric formats: three - the 12 consumer warps, not the ring's depth, are what the loop is short of with two. The
+// zero-point loop is bound by its arithmetic, so that three CTAs do in 3/2 of the time what two do, and two keep a stage more in
+// flight: they take it, except where a short list (a few rounds) fills the rounds of three CTAs better. npairs bounds the
+// sub-items. 1, 2, 3, 4, 5, 8, 64 tokens, three CTAs against two: 28, 36, 38, 52, 57, 73, 245 us and 24, 28, 43, 46, 58, 73, 239.
+template <int FMT, bool DOWN>
+static int stream_launch_one(moexb_ctx* c, const StreamArgs& a, int npairs, void* stream) {
+    if constexpr (FMT != FMT_ZP) return stream_launch_cfg<FMT, DOWN, 3>(c, a, stream);
+    else {
+        const long long tiles = (long long)npairs * st_tiles<DOWN>();
+        const long long rounds2 = (tiles + 2 * c->sms - 1) / (2 * c->sms), rounds3 = (tiles + 3 * c->sms - 1) / (3 * c->sms);
+        return rounds3 <= (DOWN ? 3 : 2) && 3 * rounds3 <= 2 * rounds2 ? stream_launch_cfg<FMT, DOWN, 3>(c, a, stream) : stream_launch_cfg<FMT, DOWN, 2>(c, a, stream);
+    }
+}
 
 // gate/up then down over the sub-items already planned in the context (subs, nsub);
 // xs = the split activations [token][2][H]; act32 optional.
-static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, void* stream) {
+static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int npairs, void* stream) {
     StreamArgs a{c->subs, c->nsub, pairs, reinterpret_cast<const __nv_bfloat16*>(c->xs), act32, reinterpret_cast<__nv_bfloat16*>(c->act_split), ypair, c->err};
     return by_fmt(fmt, [&]<int FMT>() {
-        int rc = stream_launch_one<FMT, false>(c, a, stream);
+        int rc = stream_launch_one<FMT, false>(c, a, npairs, stream);
         if (rc != MOEXB_OK) return rc;
         StreamArgs d = a;
         d.xs = reinterpret_cast<const __nv_bfloat16*>(c->act_split);
-        return stream_launch_one<FMT, true>(c, d, stream);
+        return stream_launch_one<FMT, true>(c, d, npairs, stream);
     });
 }
 
@@ -1199,7 +1211,7 @@ extern "C" int moexb_pairs_forward_tc(moexb_ctx* c, int fmt, const moexb_pair_it
     plan.items = items; plan.n_items = n_items; plan.maxp = ST_MAXP; plan.subs = c->subs; plan.nsub = c->nsub;
     int rc = split_launch(c, X, T, stream, plan);
     if (rc != MOEXB_OK) return rc;
-    return stream_experts(c, fmt, pairs, act, ypair, stream);
+    return stream_experts(c, fmt, pairs, act, ypair, npairs, stream);
 }
 
 extern "C" int moexb_ctx_set_fused_decode(moexb_ctx* c, int on) {
@@ -1419,7 +1431,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
         }
         ranks = 0;
     } else if (decode) {
-        rc = tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream) : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream);
+        rc = tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream) : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, K + 1, stream);
         if (rc != MOEXB_OK) return rc;
         ranks = K + 1;
     } else {
@@ -1442,7 +1454,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
         }
         rc = prefill ? grouped_experts(c, L, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
            : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr)
-           : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream)
+           : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T * (K + 1), stream)
                        : pairs_launch(c, L->fmt, c->items, c->nitems, min(E, T * K) + 1, c->pairs, xf, c->act, c->ypair, stream);
         if (rc != MOEXB_OK) return rc;
         if (shared) extra = c->ypair + (size_t)T * K * EH;
@@ -1871,7 +1883,7 @@ int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
     }
     rc = prefill ? grouped_experts(c, L, c->pairs, e->parts, c->ypair, stream)
        : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, in_kernel ? &plan : nullptr)
-               : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, stream);
+               : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T * (K + 1), stream);
     if (rc != MOEXB_OK) return rc;
     PROF(c, MOEXB_PROF_COMBINE, stream);
     CUDA_TRY(launch_dep(ep_partial_push_k, T, 256, 0, st, e->g, e->peers, e->lay, (const float*)c->ypair, (const unsigned*)e->step, (unsigned)(l + 1)));

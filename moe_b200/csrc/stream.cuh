@@ -27,13 +27,14 @@ namespace moexb {
 constexpr int ST_PIECE = 256;    // bytes of one row piece: 512 int4 weights
 constexpr int ST_STRIDE = 288;   // piece stride in shared memory (rows g..g+3 of a half-warp land on distinct banks)
 constexpr int ST_SC_PER_PIECE = 48;  // zero point: 16 x [sc, mn] + 2 x (d, dm) = 40 scale bytes per piece, kept 16-byte aligned
-constexpr int ST_NP = 2;         // producer warps
+constexpr int ST_NW = 4, ST_NP = 2;  // consumer and producer warps
 constexpr int ST_MAXP = 4;       // pairs per sub-item: 4 x (hi, lo) = the 8 columns of one MMA tile
 constexpr int ST_WAIT_LIMIT = 1 << 22;
 
 enum : int { ST_ERR_NONE = 0, ST_ERR_FULL_WAIT = 1, ST_ERR_EMPTY_WAIT = 2 };
 
 template <int FMT> constexpr int st_scale_bytes() { return FMT == FMT_SYM_F16 ? 16 : FMT == FMT_SYM_F32 ? 32 : ST_SC_PER_PIECE; }
+template <bool DOWN> constexpr int st_tiles() { return DOWN ? EH / (16 * ST_NW) : EI / (8 * ST_NW); }   // per sub-item
 template <int NW> constexpr int st_pieces() { return 16 * NW; }
 template <int FMT, int NW> constexpr int st_slot_bytes() { return st_pieces<NW>() * (ST_STRIDE + st_scale_bytes<FMT>()); }
 // activation columns in shared memory: 8 columns of K bf16, column stride K*2 + 64 bytes (conflict-free 16-byte reads)

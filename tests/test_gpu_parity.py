@@ -224,6 +224,21 @@ def test_pairs_forward_tc_streaming(ctx, experts, fmt):
     assert np.abs(a - b).max() <= 5e-3 * np.abs(b).max()
 
 
+@pytest.mark.parametrize("counts", [[1], [3, 1, 12, 8], [12, 12, 12, 4], [12] * 6])
+def test_pairs_forward_tc_zero_point_lists(ctx, experts, counts):
+    """Lists of 1, 24, 40 and 72 pairs: three CTAs of the zero-point kernels per SM or two, in one projection, in both or in none."""
+    host, devb = experts[m.FMT_ZP]
+    rng = np.random.default_rng(len(counts))
+    T = 12
+    X = rng.standard_normal((T, 2048)).astype(np.float32)
+    items, pairs, jobs, npairs = make_work(rng, devb, counts, T)
+    ref = o.run_pairs(m.FMT_ZP, [(host[i], t, p, w) for i, t, p, w in jobs], X, npairs)
+    yp = torch.zeros(npairs * 2048, device=DEV)
+    ctx.pairs_forward_tc(m.FMT_ZP, dev(items.view(np.uint8)), len(items), dev(pairs.view(np.uint8)), dev(X), T, npairs, None, yp)
+    assert ctx.status() == 0
+    check_ffn(yp.cpu().numpy().reshape(npairs, 2048), ref, m.FMT_ZP, f"{npairs} zero-point pairs")
+
+
 def test_pairs_reduce_and_gated_add():
     rng = np.random.default_rng(2)
     T, K, D = 5, 8, 2048
