@@ -239,6 +239,29 @@ def test_pairs_forward_tc_zero_point_lists(ctx, experts, counts):
     check_ffn(yp.cpu().numpy().reshape(npairs, 2048), ref, m.FMT_ZP, f"{npairs} zero-point pairs")
 
 
+@pytest.mark.parametrize("n_items", [256, 257, 300, 520])
+def test_pairs_forward_tc_plans_more_than_256_items(experts, n_items):
+    """The planning block walks the items 256 at a time: pairs on both sides of item 256, empty items between them and at the ends."""
+    fmt, T = m.FMT_SYM_F16, 12
+    host, devb = experts[fmt]
+    rng = np.random.default_rng(n_items)
+    X = rng.standard_normal((T, 2048)).astype(np.float32)
+    at = sorted({1, 2, 255, 256, n_items - 2} & set(range(n_items)))
+    few, pairs, jobs, npairs = make_work(rng, devb, [5, 9, 1, 12, 3][:len(at)], T)
+    items = np.zeros(n_items, ITEM_DT)
+    items["start"] = npairs
+    items[at] = few
+    c = m.Context(0, max_tokens=T, max_experts=544, top_k=8)
+    try:
+        ref = o.run_pairs(fmt, [(host[i], t, p, w) for i, t, p, w in jobs], X, npairs)
+        yp = torch.zeros(npairs * 2048, device=DEV)
+        c.pairs_forward_tc(fmt, dev(items.view(np.uint8)), n_items, dev(pairs.view(np.uint8)), dev(X), T, npairs, None, yp)
+        assert c.status() == 0
+        check_ffn(yp.cpu().numpy().reshape(npairs, 2048), ref, fmt, f"{n_items} items")
+    finally:
+        c.close()
+
+
 def test_pairs_reduce_and_gated_add():
     rng = np.random.default_rng(2)
     T, K, D = 5, 8, 2048
@@ -270,6 +293,24 @@ def test_shared_expert_add(experts, fmt):
     sh = o.run_pairs(fmt, [(host[2], list(range(T)), list(range(T)), [1.0] * T)], X, T)
     ref = base + sh / (1 + np.exp(-gl[:, None]))
     check_ffn(out.cpu().numpy(), ref, fmt, "shared expert")
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("T", [1, 3, 4, 5, 16])
+@pytest.mark.parametrize("gl_stride", [1, 257])
+def test_shared_expert_add_over_token_tiles(experts, fmt, T, gl_stride):
+    """Blocks of four tokens: full ones, ones that repeat their last row, and gate logits as a column of the router's rows."""
+    host, devb = experts[fmt]
+    rng = np.random.default_rng(T)
+    X = rng.standard_normal((T, 2048)).astype(np.float32); gl = rng.standard_normal((T, gl_stride)).astype(np.float32)
+    base = rng.standard_normal((T, 2048)).astype(np.float32)
+    out = torch.cat([dev(base), torch.full((4, 2048), 7.0, device=DEV)])   # rows past the last token are not touched
+    gl_d = dev(gl)
+    m.shared_expert_add(fmt, devb[2], gl_d.data_ptr() + 4 * (gl_stride - 1), gl_stride, dev(X), T, out)
+    sh = o.run_pairs(fmt, [(host[2], list(range(T)), list(range(T)), [1.0] * T)], X, T)
+    got = out.cpu().numpy()
+    check_ffn(got[:T], base + sh / (1 + np.exp(-gl[:, -1:])), fmt, f"shared expert, {T} tokens, gate stride {gl_stride}")
+    assert (got[T:] == 7.0).all()
 
 
 @pytest.mark.parametrize("T,E,K,holes", [(1, 256, 8, False), (4, 256, 8, False), (64, 256, 8, True), (33, 64, 4, True)])
