@@ -140,7 +140,7 @@ int moexb_pairs_reduce(const float* ypair, const float* ycpu, float* moe, int K,
 int moexb_gated_add_rows(float* out, const float* sh, const float* gl, int gl_stride, int D, int T, void* stream);
 
 /* Shared expert held as one int4 blob of the routed experts' shape: out[t] += sigmoid(gl[t*gl_stride]) *
- * down(silu(gate x_t) * up x_t) for t < T. scratch: >= T*(I + H + 3) + 4 floats, 16-byte aligned. Stands behind shared_expert_add
+ * down(silu(gate x_t) * up x_t) for t < T. scratch: >= T*I floats, 16-byte aligned. Stands behind shared_expert_add
  * (kernels.cuh:2018-2028) and shared_rows (moex.cu:1674-1682), whose dense int8/int6 weight matrices are replaced by
  * an expert blob. */
 int moexb_shared_expert_add(int fmt, const uint8_t* blob, const float* gl, int gl_stride, const float* X, int T,
@@ -149,7 +149,8 @@ int moexb_shared_expert_add(int fmt, const uint8_t* blob, const float* gl, int g
 /* Bucket the T*K (token, rank) pairs by expert id: items in ascending expert id, pairs in token order inside an
  * expert, p = t*K + rank, as the host loop at moex.cu:1466-1486 and route_export_k (kernels.cuh:1020-1054) do.
  * slot_table: E blob pointers (null = expert not held here: its pairs are dropped, which is how an expert-parallel
- * rank sees only its own experts). items: E entries; pairs: T*K entries; nitems: 1 int; counts: E ints of scratch. */
+ * rank sees only its own experts). items: E entries; pairs: T*K entries; nitems: 1 int; counts: not null, no
+ * longer written. items beyond *nitems and pairs beyond theirs come back empty. */
 int moexb_group_pairs(const int* idx, const float* w, int T, int K, int E, const uint8_t* const* slot_table,
                       moexb_pair_item* items, moexb_pair* pairs, int* nitems, int* counts, void* stream);
 

@@ -26,9 +26,14 @@ def _ptr(t):
     return int(t)
 
 
+# the raw handle of a device's current stream, without building a Stream object on every call, where this torch has it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    # the raw handle of the current stream of the current device, without building a Stream object on every call
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def expert_bytes(fmt):
@@ -91,7 +96,7 @@ def gated_add_rows(out, sh, gl, gl_stride, D, T):
 
 def shared_expert_add(fmt, blob, gl, gl_stride, X, T, out, scratch=None):
     if scratch is None:
-        scratch = torch.empty(T * (EI + EH + 3) + 4, device=X.device, dtype=torch.float32)
+        scratch = torch.empty(T * EI, device=X.device, dtype=torch.float32)
     check(lib().moexb_shared_expert_add(fmt, _ptr(blob), _ptr(gl), gl_stride, _ptr(X), T, _ptr(out), _ptr(scratch), _stream()))
     return out
 
@@ -101,10 +106,10 @@ def group_pairs(idx, w, T, K, E, slot_table):
     dev = idx.device
     items = torch.empty(E * _ITEM_BYTES, device=dev, dtype=torch.uint8)
     pairs = torch.empty(T * K * _PAIR_BYTES, device=dev, dtype=torch.uint8)
-    counts = torch.empty(1 + E, device=dev, dtype=torch.int32)   # the number of items, then scratch
-    p = counts.data_ptr()
-    check(lib().moexb_group_pairs(_ptr(idx), _ptr(w), T, K, E, _ptr(slot_table), items.data_ptr(), pairs.data_ptr(), p, p + 4, _stream()))
-    return items, pairs, counts[:1]
+    nitems = torch.empty(1, device=dev, dtype=torch.int32)
+    p = nitems.data_ptr()
+    check(lib().moexb_group_pairs(_ptr(idx), _ptr(w), T, K, E, _ptr(slot_table), items.data_ptr(), pairs.data_ptr(), p, p, _stream()))
+    return items, pairs, nitems
 
 
 def dequant(fmt, blob):

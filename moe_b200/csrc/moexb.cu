@@ -1147,9 +1147,11 @@ static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, const GroupedM
     return MOEXB_OK;
 }
 
-// Batches from this size on run on the grouped GEMM. Zero-point blobs from a third of the symmetric formats' size on: their streaming
-// kernels take twice the MMAs and four pairs a pass (96 tokens: 256 us a layer against 237, 240 tokens 491 against 274; the symmetric
-// formats 192 against 204 at 240 tokens, 232 against 219 at 320).
+// Batches from this size on run on the grouped GEMM; where the lines cross depends on how many experts the tokens share. Zero-point blobs
+// from a third of the symmetric formats' size on: their streaming kernels take twice the MMAs and four pairs a pass. us a layer,
+// streaming against grouped, of independent tokens and of a 12-layer stack whose tokens have grown alike:
+//   symmetric   192 tokens 160 / 204 and 162 / 181, 256 tokens 194 / 221 and 194 / 193, 336 tokens 237 / 226 and 231 / 209
+//   zero point   72 tokens 209 / 232 and 167 / 116,  88 tokens 230 / 235 and 185 / 115, 128 tokens 286 / 238 and 250 / 143
 static int grouped_min_tokens(const moexb_ctx* c, int fmt) {
     const int t = c->prefill_min_tokens;
     return fmt == FMT_ZP ? t / 3 + (t % 3 != 0) : t;   // (any threshold up to the largest int)
@@ -1158,7 +1160,7 @@ static int grouped_min_tokens(const moexb_ctx* c, int fmt) {
 // Pairs per tile of the grouped GEMM.
 static int grouped_maxp(int fmt) { return fmt == FMT_ZP ? gg_nmax<FMT_ZP>() : gg_nmax<FMT_SYM_F16>(); }
 
-// Experts of a large batch on the tensor-core grouped GEMM: the tiles are in the context (subs, nsub) or in the buckets, and grouped_rows or
+// Experts of a large batch on the tensor-core grouped GEMM: the tiles are in the context (subs, nsub) or in the buckets, and layer_rows or
 // the token owners (expert parallelism) left the activation rows.
 static int grouped_experts(moexb_ctx* c, const moexb_layer* L, const moexb_pair* pairs, int parts, float* ypair, void* stream, const BucketArgs* buckets = nullptr) {
     return by_fmt(L->fmt, [&]<int FMT>() {
@@ -1193,7 +1195,8 @@ static int layer_rows(moexb_ctx* c, const void* X, int x_dtype, int rows, float*
             case ROWS_GEMM: return run.template operator()<XT, NORM, ROWS_GEMM>();
             case ROWS_GEMM_Z: return run.template operator()<XT, NORM, ROWS_GEMM_Z>();
         }
-        return run.template operator()<XT, NORM, ROWS_NONE>();
+        if constexpr (NORM || sizeof(XT) == 2) return run.template operator()<XT, NORM, ROWS_NONE>();
+        else return (int)MOEXB_OK;   // f32 rows as they are
     };
     if (x_dtype == MOEXB_BF16) return norm ? by_mode.template operator()<__nv_bfloat16, true>() : by_mode.template operator()<__nv_bfloat16, false>();
     return norm ? by_mode.template operator()<float, true>() : by_mode.template operator()<float, false>();
@@ -1311,10 +1314,10 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
                 CUDA_TRY(launch_dep(route_gemv_k<WT, __nv_bfloat16, WARPS, NJ>, grid, WARPS * 32, 0, S(stream), W, static_cast<const __nv_bfloat16*>(x), logits, EH, E, K, 1, c->route_done, o, xs, ro.split));
             else CUDA_TRY(launch_dep(route_gemv_k<WT, float, WARPS, NJ>, grid, WARPS * 32, 0, S(stream), W, xf, logits, EH, E, K, 1, c->route_done, o, xs, ro.split));
         } else {
-            // 16 outputs per block spread a small batch over more SMs; a prefill chunk has blocks to spare and re-reads
-            // the router weights less with 32 outputs per block
-            auto gemm = [&]<int TO, int TR>() -> int {
-                constexpr int WARPS = 8, SMEM = TR * EH * (int)sizeof(float);
+            // a small batch: 16 outputs x 8 tokens per block, to reach every SM; a prefill chunk goes to the register-tiled
+            // kernel (64 tokens x 16 outputs per block, FMA-bound)
+            auto gemm = [&]() -> int {
+                constexpr int WARPS = 8, TO = 2, TR = 8, SMEM = TR * EH * (int)sizeof(float);
                 static PerDeviceOnce once;
                 const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(route_gemm_k<WT, WARPS, TO, TR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
                 if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "router kernel shared memory: %s", cudaGetErrorString(attr_err));
@@ -1322,8 +1325,6 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
                                     W, xf, logits, EH, E, K, 1, T, c->route_done, o));
                 return MOEXB_OK;
             };
-            // a small batch: 16 outputs x 8 tokens per block, to reach every SM; a prefill chunk goes to the register-tiled
-            // kernel (64 tokens x 16 outputs per block, FMA-bound)
             auto gemm2 = [&]() -> int {
                 constexpr int SMEM = RG2_ST * rg2_stage_bytes<WT>();
                 static PerDeviceOnce once;
@@ -1337,7 +1338,7 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
                 }
                 return MOEXB_OK;
             };
-            const int rc = T >= 256 ? gemm2() : gemm.template operator()<2, 8>();
+            const int rc = T >= 256 ? gemm2() : gemm();
             if (rc != MOEXB_OK) return rc;
         }
         LAUNCHED("route");

@@ -1,4 +1,4 @@
-// Streaming expert kernels for 1..64 tokens: the bandwidth-bound skinny GEMM of the decode-size path.
+// Streaming expert kernels on blobs in the reference layout, for any work list: the bandwidth-bound skinny GEMM of the decode-size path.
 //
 // One kernel template serves both projections (gate/up with the SwiGLU epilogue, down with the routing-weight epilogue).
 // A persistent CTA has two producer warps and NW consumer warps. The producers stream packed int4 rows and their scale bytes
