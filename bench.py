@@ -47,7 +47,7 @@ WORKLOADS = {
 SEED = 0
 # dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the roofline kernel, from the ncu captures
 # summarised under profiles/ (gate/up kernel on a 2-layer case of serve64; the one-token stack kernel; the grouped GEMM)
-TRAFFIC_RATIO = {"serve64": 1.01, "decode1": 1.015, "prefill2048": 1.06}
+TRAFFIC_RATIO = {"serve64": 1.01, "decode1": 1.015, "prefill2048": 1.13}
 
 
 def router_weights(layer):
@@ -416,7 +416,8 @@ def measure(env, workload, allreduce=False):
         return ix[(ix >= first) & (ix < first + count)]
     distinct = float(np.mean([len(torch.unique(local(idx[l]))) for l in range(NL)])) + 1  # + the shared expert
     # passes over expert weights: an expert with n tokens is streamed ceil(n / maxp) times (maxp pairs per sub-item)
-    maxp = 128 if T >= 256 else args.pairs_per_pass if (T >= 8 and fmt != m.FMT_ZP) else 4
+    grouped = T >= (86 if fmt == m.FMT_ZP else 256)   # the library's default threshold of the grouped GEMM, and its tiles
+    maxp = (48 if fmt == m.FMT_ZP else 80) if grouped else args.pairs_per_pass if (T >= 8 and fmt != m.FMT_ZP) else 4
     passes = float(np.mean([int(torch.ceil(torch.bincount(local(idx[l].flatten()).long(), minlength=E) / maxp).sum()) for l in range(NL)])) + (sh1 - sh0 + maxp - 1) // maxp
     eb = m.expert_bytes(fmt)
     qb_gu, qb_dn = 2 * EI * EH // 2, EH * EI // 2
@@ -462,8 +463,8 @@ def measure(env, workload, allreduce=False):
         flops_gu, flops_dn = 2.0 * npairs * EH * 2 * EI, 2.0 * npairs * EH * EI
         r.update({"bound": "tensor", "unit": "TFLOP/s", "achieved": flops_gu / (per_launch_us["gate_up"] * 1e-6) / 1e12, "peak": tensor_peak,
                   "algorithmic_flops_per_launch": flops_gu, "pairs_per_layer": npairs, "hbm_achieved_gbs": achieved, "hbm_frac": achieved / hbm_peak,
-                  "note": "weights enter the tensor core as an exact fp16 hi + lo pair: 2 MMAs per weight tile (gate/up), 4 (down), so the "
-                          "nominal-flop fraction cannot exceed 0.50 / 0.25 at full tensor-pipe activity"})
+                  "note": "weights enter the tensor core as exact 4-bit integers, one MMA pass per activation part: bf16 tokens are one part (gate/up), "
+                          "the down projection's activations two (hi + lo), so the nominal-flop fraction cannot exceed 1.0 / 0.5"})
         r["frac"] = r["achieved"] / r["peak"]
         r["down"].update({"achieved": flops_dn / (per_launch_us["down"] * 1e-6) / 1e12, "algorithmic_flops_per_launch": flops_dn})
         r["whole_layer"].update({"flops": 1.5 * flops_gu + 2.0 * T * (E + 1) * EH,
