@@ -224,13 +224,14 @@ static int gemv_any(const WT* W, const float* x, float* y, int I, int O, void* s
     // them a small batch has too few to reach every SM. In a chain of calls (f16 / f32 weights, us): 8 rows 3.1 / 3.2 against 6.0 / 5.7,
     // 14 rows 5.2 / 5.2 against 6.0 / 5.7, 16 rows 5.6 / 5.6 against 6.0 / 5.8, 20 rows 6.6 / 6.8 against 6.0 / 5.8; with weights that
     // come from memory the lines cross at 16 (a chunk of 16 tokens over 2 layers: 187 us against 184).
-    if (rows >= 16) {
+    constexpr int TR = 8, SMEM_MAX = 200 * 1024;
+    const int smem = I <= SMEM_MAX / (TR * (int)sizeof(float)) ? TR * I * (int)sizeof(float) : SMEM_MAX + 1;   // of a tile's rows
+    if (rows > 24 || (rows >= 16 && smem <= SMEM_MAX)) {   // (up to 24 rows of any length are taken)
         // Tiles of 16 outputs x 8 rows. Up to one tile per SM the warps are what is short: 8 of 2 outputs each (64 rows of 257 outputs
         // 6.2 / 5.9 us, 10.3 / 7.9 with 4 of 4). Beyond, the reads of the rows from shared memory, which a warp's outputs share (65 rows
         // 11.1 / 10.6 us with 8 of 2, 8.8 / 7.2 with 4 of 4; 256 rows 22.6 / 21.5 and 19.5 / 14.8; 2048 rows 163 / 155 and 102 / 89).
-        constexpr int TR = 8, TILE = 16;
-        const int smem = TR * I * (int)sizeof(float);
-        REQUIRE(smem <= 200 * 1024, "gemv: I=%d is too large for the batched kernel", I);
+        constexpr int TILE = 16;
+        REQUIRE(smem <= SMEM_MAX, "gemv: I=%d is too large for the batched kernel", I);
         const dim3 grid((O + TILE - 1) / TILE, (rows + TR - 1) / TR);
         int dev = 0, sms = 0;
         CUDA_TRY(cudaGetDevice(&dev));
@@ -238,7 +239,7 @@ static int gemv_any(const WT* W, const float* x, float* y, int I, int O, void* s
         auto tiles = [&]<int WARPS, int U>() -> int {
             constexpr auto kernel = gemm_rows_k<WT, WARPS, TILE / WARPS, TR, U>;
             static PerDeviceOnce once;
-            const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
+            const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX); });
             if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "gemv: shared memory attribute: %s", cudaGetErrorString(attr_err));
             CUDA_TRY(launch_dep(kernel, grid, WARPS * 32, smem, S(stream), W, x, y, I, O, rows));
             return MOEXB_OK;

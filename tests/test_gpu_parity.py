@@ -95,6 +95,17 @@ def test_router_logits_where_the_tiles_change(rows, O, I):
     assert np.array_equal(m.gemv_f16(dev(W16), dev(x), rows=rows).cpu().numpy(), o.router_logits(W16, x, rows))
 
 
+def test_router_rows_longer_than_a_tile_holds():
+    """Rows of 8192 inputs: up to 24 of them are taken, more are refused."""
+    rng = np.random.default_rng(1)
+    W = (rng.standard_normal((33, 8192)) * 0.02).astype(np.float32)
+    x = rng.standard_normal((25, 8192)).astype(np.float32)
+    for rows in (1, 16, 24):
+        assert np.array_equal(m.gemv_f32(dev(W), dev(x[:rows]), rows=rows).cpu().numpy(), o.router_logits(W, x[:rows], rows))
+    with pytest.raises(m.MoexbError, match="too large"):
+        m.gemv_f32(dev(W), dev(x), rows=25)
+
+
 @pytest.mark.parametrize("rows", [1, 15, 16, 33])
 def test_router_weights_written_by_the_kernel_before(rows):
     """The weights of a pointer-level call may be the output of the kernel before it, here of a combine whose launch lets the next
