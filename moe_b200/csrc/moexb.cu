@@ -1076,15 +1076,15 @@ static int stream_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float*
     });
 }
 
-template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC>
+template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC, bool KSP = false>
 static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa, const BucketArgs& ba, void* stream) {
-    constexpr int SMEM = tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC>();
-    static_assert(tl_fits<FMT, DOWN, NW, D, NB, CPS, SRC>(), "shared memory of the resident CTAs");
+    constexpr int SMEM = tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC, KSP>();
+    static_assert(tl_fits<FMT, DOWN, NW, D, NB, CPS, SRC, KSP>(), "shared memory of the resident CTAs");
     static PerDeviceOnce once;
-    const cudaError_t attr_err = once.run([] { return opt_in(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, NW * 32, SMEM, CPS); });
+    const cudaError_t attr_err = once.run([] { return opt_in(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC, KSP>, NW * 32, SMEM, CPS); });
     if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "tiled stream kernel shared memory: %s", cudaGetErrorString(attr_err));
     PROF(c, DOWN ? MOEXB_PROF_DOWN : MOEXB_PROF_GATE_UP, stream);
-    CUDA_TRY(launch_dep(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC>, CPS * c->sms, NW * 32, SMEM, S(stream), a, pa, ba));
+    CUDA_TRY(launch_dep(stream_tiled_k<FMT, DOWN, NW, D, NB, CPS, SRC, KSP>, CPS * c->sms, NW * 32, SMEM, S(stream), a, pa, ba));
     LAUNCHED(DOWN ? "stream_tiled_down" : "stream_tiled_gate_up");
     return MOEXB_OK;
 }
@@ -1097,6 +1097,15 @@ static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa
 template <int FMT, bool DOWN, int SRC>
 static int tiled_launch_one(moexb_ctx* c, const TiledArgs& a, int T, void* stream, const PlanArgs& pa, const BucketArgs& ba) {
     static_assert(SRC != TL_PLAN || FMT == FMT_SYM_F16, "the in-kernel work list fits beside the ring of the fp16-scale format only");
+    // The K slices of a row tile on four warps: one zero-point token (9 sub-items, a slice per warp: 26.0 -> 21.6 us a layer; symmetric
+    // formats 19.2 either way), and 8 to 15 tokens of the symmetric formats, where whole rounds are two or three per CTA and leave many
+    // CTAs with one less (8, 9, 11, 14 tokens 47.9, 50.1, 55.8, 58.3 -> 46.7, 49.2, 52.6, 58.0 us; stacks of 10 and 12 43.7, 48.1 -> 41.6, 44.2;
+    // 16 and 23 tokens 59.8, 71.5 -> 60.5, 72.1; zero point 9 and 14 tokens 71.4, 92.9 -> 73.1, 90.1).
+    if constexpr (!DOWN && FMT == FMT_ZP) { if (T == 1) return tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream); }
+    else if constexpr (!DOWN) {
+        if (T >= 8 && T < 16) return c->pairs_per_pass == 4 ? tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream)
+                                                            : tiled_launch_cfg<FMT, DOWN, 16, 2, 2, 1, SRC, true>(c, a, pa, ba, stream);
+    }
     if (T < 8) return tiled_launch_cfg<FMT, DOWN, 4, 4, 1, 2, SRC>(c, a, pa, ba, stream);
     if (FMT == FMT_ZP || c->pairs_per_pass == 4) return tiled_launch_cfg<FMT, DOWN, 8, 2, 1, 2, SRC>(c, a, pa, ba, stream);
     if constexpr (FMT == FMT_ZP) return MOEXB_OK;

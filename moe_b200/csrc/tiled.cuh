@@ -222,6 +222,12 @@ struct TiledArgs {
     int* err;
 };
 
+// Where the work list of a launch comes from (SRC below).
+enum : int { TL_LIST = 0, TL_PLAN = 1, TL_BUCKETS = 2 };
+// Ring, activation columns, barriers and work list; behind them the partial sums (KSP below).
+template <int FMT, bool DOWN, int NW, int D, int NB, int SRC>
+__host__ __device__ constexpr int tl_red_offset() { return NW * D * tl_slice_bytes<FMT>() + 8 * NB * st_bcol_bytes<DOWN>() + NW * D * 8 + 64 + (SRC == TL_PLAN ? (int)sizeof(PlanSmem) + 16 : SRC == TL_BUCKETS ? (int)sizeof(BucketSmem) + 16 : 0); }
+
 // Streaming expert kernel on the tiled layout. No producer warp: every warp is its own pipeline. A warp owns a ring of D
 // slice buffers; lane 0 issues one cp.async.bulk per slice (4-5 KB, one contiguous run of the blob) D slices ahead and
 // the warp waits on the slice's mbarrier before consuming it, so there is no cross-warp hand-off on the weight stream.
@@ -234,15 +240,17 @@ struct TiledArgs {
 // pairs are then unpacked once instead of twice); CPS = CTAs per SM the launch is sized for.
 // SRC: where the work list comes from - TL_LIST: a.subs / a.pairs / a.nsub; TL_PLAN (gate/up only): the CTA makes it itself
 // (plan_in_cta) from pa; TL_BUCKETS (gate/up only): the router's buckets (ba).
-enum : int { TL_LIST = 0, TL_PLAN = 1, TL_BUCKETS = 2 };
-template <int FMT, bool DOWN, int NW, int D, int NB = 1, int CPS = 2, int SRC = TL_LIST>
+// KSP (gate/up only): the four K slices of a row tile go to four warps, whose partial sums meet in shared memory: a round is NW / 4 row
+// tiles of one slice each. Finer rounds share a short list out better; on a long one the hand-over costs more than that (64 tokens 103.2 ->
+// 106.0 us a layer; where the line lies: tiled_launch_one).
+template <int FMT, bool DOWN, int NW, int D, int NB = 1, int CPS = 2, int SRC = TL_LIST, bool KSP = false>
 __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a, const PlanArgs pa, const BucketArgs ba) {
     constexpr bool PLAN = SRC == TL_PLAN, BUCKETS = SRC == TL_BUCKETS;
     static_assert(NB == 1 || FMT != FMT_ZP, "two column blocks are built for the symmetric formats only");
     static_assert(SRC == TL_LIST || !DOWN, "the down kernel reads the list the gate/up kernel left in global memory");
     constexpr int GB = tl_group_bytes<FMT>(), SB = tl_slice_bytes<FMT>();
     constexpr int KS = DOWN ? 1 : 4;                       // slices per row tile
-    constexpr int RPS = (DOWN ? 128 : 64) / NW;            // rounds per sub-item
+    static_assert(!KSP || !DOWN, "a down tile is one slice");
     constexpr int KB = DOWN ? EI : EH;
     constexpr int BCOL = st_bcol_bytes<DOWN>();
     constexpr bool Z = FMT == FMT_ZP;
@@ -252,6 +260,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     uint64_t* bars = reinterpret_cast<uint64_t*>(bsm + 8 * NB * BCOL); // full[NW][D]
     PlanSmem& P = *reinterpret_cast<PlanSmem*>(bars + NW * D + 8);      // PLAN, BUCKETS: the launch adds the room
     BucketSmem& L = *reinterpret_cast<BucketSmem*>(bars + NW * D + 8);
+    float2* red = reinterpret_cast<float2*>(smem + tl_red_offset<FMT, DOWN, NW, D, NB, SRC>());   // KSP: [round & 1][tile][slice - 1][block][lane]
     static_assert(!PLAN || sizeof(PlanTmp) <= NW * D * SB, "the planning scratch fits where the ring will be");
     // zero point: the sum of the activations over each 32-input chunk, per column: [K slice][group][chunk][8 columns]
     __shared__ __align__(16) float csum[tl_csum_floats<FMT, DOWN>()];
@@ -302,12 +311,16 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     const int nsub0 = PLAN ? P.nsub[0] : BUCKETS ? L.wide[ba.E + 1] + L.narrow[ba.E + 1] : a.nsub[0], nsub1 = PLAN ? P.nsub[1] : BUCKETS ? L.wide[ba.E + 1] : a.nsub[1];
     // This CTA's contiguous range of rounds: an equal share of the cost, a round of a wide sub-item (more than 4 pairs,
     // they come first in subs[]) counting CW and any other CN.
+    constexpr int TPS = DOWN ? 128 : 64;   // row tiles per sub-item
     constexpr int CN = 10, CW = NB == 2 ? 13 : 10;   // measured: a wide round takes 1.3 times a narrow one in both kernels
+    constexpr int KSW = KSP ? 1 : KS;                            // slices of a round per warp (of KS per row tile)
+    constexpr int TPR = KSP ? NW / KS : NW, RPS = TPS / TPR;     // row tiles per round, rounds per sub-item
+    const int in_round = KSP ? warp / KS : warp;                 // the warp's row tile of a round
     const long long RW = NB == 2 ? (long long)nsub1 * RPS : 0, R = (long long)nsub0 * RPS;
     const long long C = RW * CW + (R - RW) * CN;
     auto round_at = [&](long long x) { return (int)(x < RW * CW ? x / CW : RW + (x - RW * CW) / CN); };
     const int r0 = round_at(C * blockIdx.x / gridDim.x), r1 = round_at(C * (blockIdx.x + 1) / gridDim.x);
-    const int Q = (r1 - r0) * KS;  // slices this warp will consume
+    const int Q = (r1 - r0) * KSW;  // slices this warp will consume
     if constexpr (BUCKETS) {
         first_sub = r0 / RPS;
         const int i = first_sub + threadIdx.x;
@@ -319,8 +332,8 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
 
     // slice q of this warp: round r0 + q / KS, row tile rin*NW + warp, K slice q % KS
     auto issue = [&](int q) {
-        const int r = r0 + q / KS, sub = r / RPS, rin = r % RPS, wt = rin * NW + warp;
-        const uint8_t* src = sub_at(sub).slot + (size_t)(DOWN ? 256 + wt : wt * 4 + q % KS) * SB;
+        const int r = r0 + q / KSW, sub = r / RPS, rin = r % RPS, wt = rin * TPR + in_round;
+        const uint8_t* src = sub_at(sub).slot + (size_t)(DOWN ? 256 + wt : wt * 4 + (KSP ? warp % KS : q % KS)) * SB;
         const uint32_t bar = smem_u32(full + q % D);
         mbar_arrive_expect_tx(bar, SB);
         bulk_g2s(smem_u32(ring + (q % D) * SB), src, SB, bar);
@@ -348,7 +361,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     int failed = -1;   // the slice this warp gave up waiting for
     const uint8_t* bcol = bsm + g * BCOL + t * 16;  // the lane's activation column (pair slot g >> 1, part g & 1)
     for (int q = 0; q < Q; q++) {
-        const int r = r0 + q / KS, sub = r / RPS, rin = r % RPS, ks = q % KS;
+        const int r = r0 + q / KSW, sub = r / RPS, rin = r % RPS, ks = KSP ? warp % KS : q % KS;
         if (sub != cur_sub) {
             // new sub-item: the CTA's warps swap the activation columns together (their weight copies stay in flight)
             cur_sub = sub;
@@ -382,7 +395,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
             }
         }
         if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(full + q % D), (q / D) & 1, a.err, ST_ERR_FULL_WAIT))) { failed = q; break; }
-        if (ks == 0) { acc[0] = acc[1] = acc[2] = acc[3] = 0.f; acd[0] = acd[1] = acd[2] = acd[3] = 0.f; }
+        if (KSP || ks == 0) { acc[0] = acc[1] = acc[2] = acc[3] = 0.f; acd[0] = acd[1] = acd[2] = acd[3] = 0.f; }
         const uint8_t* sl = ring + (q % D) * SB;
         const uint8_t* bp = bcol + ks * 1024;  // 8 groups of 128 bytes per slice
         auto groups = [&]<bool WIDE>() {
@@ -457,9 +470,26 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             issue(q + D);
         }
-        if (ks == KS - 1) {
+        if (KSP || ks == KS - 1) {
             // epilogue: the lane's columns 2t (hi) and 2t+1 (lo) of column block b belong to pair slot 4b + t
-            const int wt = rin * NW + warp;
+            const int wt = rin * TPR + in_round;
+            if constexpr (KSP) {
+                float2* part = red + (size_t)((q & 1) * TPR + warp / KS) * (KS - 1) * NB * 32 + lane;
+                if (ks) {
+                    part[(ks - 1) * NB * 32] = make_float2(acc[0] + acc[1], acc[2] + acc[3]);
+                    if constexpr (NB == 2) part[((ks - 1) * NB + 1) * 32] = make_float2(acd[0] + acd[1], acd[2] + acd[3]);
+                }
+                // the tile's four warps; of two buffers the other one is free when all have come here again
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / KS), "n"(KS * 32) : "memory");
+                if (ks) continue;
+                auto add = [&](float (&x)[4], int b) {
+                    x[0] += x[1]; x[2] += x[3]; x[1] = x[3] = 0.f;
+#pragma unroll
+                    for (int k = 0; k < KS - 1; k++) { const float2 v = part[(k * NB + b) * 32]; x[0] += v.x; x[2] += v.y; }
+                };
+                add(acc, 0);
+                if constexpr (NB == 2) add(acd, 1);
+            }
 #pragma unroll
             for (int b = 0; b < NB; b++) {
                 if (4 * b + t >= n) break;
@@ -483,20 +513,21 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     }
     if (failed >= 0) {
         // A wait ran out. The other warps of the CTA carry on, so this warp still takes part in every CTA barrier they will
-        // reach (three per change of sub-item with zero-point blobs, else two), without computing; then it waits (bounded) for
+        // reach (three per change of sub-item with zero-point blobs, else two; KSP: one per round), without computing; then it waits (bounded) for
         // the copies it has requested - slices [failed, failed + D) - so that none is in flight when the CTA leaves.
-        for (int q = failed + 1; q < Q; q++) {
-            const int sub = (r0 + q / KS) / RPS;
+        for (int q = failed; q < Q; q++) {
+            const int sub = (r0 + q / KSW) / RPS;
             if (sub != cur_sub) { cur_sub = sub; __syncthreads(); __syncthreads(); if (Z) __syncthreads(); }
+            if (KSP) asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / KS), "n"(KS * 32) : "memory");   // of this round
         }
         for (int q = failed; q < min(Q, failed + D); q++) mbar_wait(smem_u32(full + q % D), (q / D) & 1, a.err, ST_ERR_FULL_WAIT);
     }
 }
 
-template <int FMT, bool DOWN, int NW, int D, int NB = 1, int SRC = TL_LIST>
-constexpr int tl_smem_bytes() { return NW * D * tl_slice_bytes<FMT>() + 8 * NB * st_bcol_bytes<DOWN>() + NW * D * 8 + 64 + (SRC == TL_PLAN ? (int)sizeof(PlanSmem) + 16 : SRC == TL_BUCKETS ? (int)sizeof(BucketSmem) + 16 : 0); }
+template <int FMT, bool DOWN, int NW, int D, int NB = 1, int SRC = TL_LIST, bool KSP = false>
+constexpr int tl_smem_bytes() { return tl_red_offset<FMT, DOWN, NW, D, NB, SRC>() + (KSP ? 2 * (NW / 4) * 3 * NB * 32 * 8 : 0); }
 // Whether CPS CTAs fit on an SM: 228 KB of shared memory, of which a CTA also takes its static part and 1 KB of the system's.
-template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC>
-constexpr bool tl_fits() { return (tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC>() + tl_csum_floats<FMT, DOWN>() * 4 + 1024) * CPS <= 228 * 1024; }
+template <int FMT, bool DOWN, int NW, int D, int NB, int CPS, int SRC, bool KSP = false>
+constexpr bool tl_fits() { return (tl_smem_bytes<FMT, DOWN, NW, D, NB, SRC, KSP>() + tl_csum_floats<FMT, DOWN>() * 4 + 1024) * CPS <= 228 * 1024; }
 
 }  // namespace moexb

@@ -108,3 +108,31 @@ def test_the_expert_kernels_are_resident_as_often_as_their_grids_assume(fmt, lay
         finally:
             L.close(); c.close()
     assert m.short_residency() == 0
+
+
+@pytest.mark.parametrize("fmt, tokens", [(m.FMT_ZP, (1,)), (m.FMT_SYM_F16, (8, 9, 15, 16)), (m.FMT_SYM_F32, (8, 15))])
+def test_k_slices_on_four_warps(fmt, tokens):
+    """Gate/up with the K slices of a row tile on four warps: few experts (CTAs without a round, ranges that begin inside a sub-item) and
+    many, narrow and wide sub-items. Against the oracle; 4 and 8 pairs a pass agree bit for bit."""
+    for E in (32, 96):
+        c = m.Context(0, max_tokens=16, max_experts=E, top_k=8)
+        L = m.Layer(c, fmt, E)
+        L.fill_synth(3, 0)
+        rng = np.random.default_rng(13)
+        W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+        L.set_router(W)
+        host = [m.synth_expert_host(fmt, 3, 0, e) for e in range(E + 1)]
+        try:
+            for T in tokens:
+                X = rng.standard_normal((T, 2048)).astype(np.float32)
+                ref, ids, _, _ = o.layer_forward(fmt, host, W, X, 8)
+                idx = torch.empty(T, 8, dtype=torch.int32, device=DEV)
+                outs = []
+                for p in (4, 8):
+                    c.set_pairs_per_pass(p)
+                    outs.append(L.forward(torch.from_numpy(X).to(DEV), T, 8, idx=idx).cpu().numpy())
+                assert c.status() == 0 and np.array_equal(idx.cpu().numpy(), ids)
+                assert np.array_equal(outs[0], outs[1])
+                check_ffn(outs[1], ref, fmt, f"K slices on four warps, T={T} E={E}")
+        finally:
+            L.close(); c.close()
