@@ -1124,10 +1124,11 @@ static bool plan_in_kernel(int fmt, int T, int K, int E) {
 // The same on blobs in the tiled layout (sub-item slots point into a tiled layer image). The work list: plan = the gate/up kernel
 // makes it and leaves it in the context for the down kernel; buckets = the router's; neither = it is in the context.
 static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int T, void* stream, const PlanArgs* plan = nullptr,
-                         const BucketArgs* buckets = nullptr) {
-    const TiledArgs a{c->subs, c->nsub, buckets ? buckets->pairs : pairs, c->xs, act32, c->act_split, ypair, c->err};
+                         const BucketArgs* buckets = nullptr, bool clear = false) {
+    const TiledArgs a{c->subs, c->nsub, buckets ? buckets->pairs : pairs, c->xs, act32, c->act_split, ypair, c->err, nullptr, 0};
     TiledArgs d = a;
     d.xs = c->act_split;
+    if (clear) { d.cnt = c->bcnt; d.n_cnt = buckets->E; }
     PlanArgs pa = plan ? *plan : PlanArgs{};
     pa.subs_out = c->subs; pa.nsub_out = c->nsub;
     const BucketArgs ba = buckets ? *buckets : BucketArgs{};
@@ -1297,9 +1298,13 @@ struct RouteEp { const EpDevice* dev; int row_bytes; unsigned phase; const unsig
 // pairs into the buckets (with the shared expert's); the caller's copies of ids and weights; split: the rows of x (x_dtype) are split by
 // the routing kernel (ROWS_F16, ROWS_BF16; only where route_splits)
 struct RouteOut { bool buckets = false, shared = false; int* idx = nullptr; float* w = nullptr; int x_dtype = MOEXB_F32, split = ROWS_NONE; };
+// A stack's layer whose router also makes its input: the end of the layer before (rows of ypair; residual rows x) into out and, split, into
+// the context (combine_route_k; 2 to 8 tokens, whose blocks are there at once, two per SM)
+struct RouteCombine { const float* x; float* out; bool f16; };
 static bool route_splits(int T) { return T < 8; }
 template <typename WT>
-static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
+static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr,
+                        const RouteCombine* rc = nullptr) {
     const float* xf = static_cast<const float*>(x);
     // tok0: the T rows at xf are tokens tok0.. of the batch - their logits, ids and weights go to those rows of the workspace
     const int E = L->n_routed;
@@ -1314,6 +1319,20 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
     o.idx2 = ro.idx; o.w2 = ro.w;
     if (rep) { o.ep = rep->dev; o.ep_row_bytes = rep->row_bytes; o.ep_phase = rep->phase; o.ep_step = rep->step; }
     auto run = [&]<int NJ>() -> int {
+        if (rc) {
+            auto combine = [&]<bool F16>() -> int {
+                constexpr auto kernel = combine_route_k<WT, NJ, F16>;
+                constexpr int SMEM = 8 * EH * (int)sizeof(WT);
+                static PerDeviceOnce once;
+                const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
+                if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "router kernel shared memory: %s", cudaGetErrorString(attr_err));
+                const float *ypair = c->ypair, *extra = c->ypair + (size_t)T * K * EH;
+                CUDA_TRY(launch_dep(kernel, dim3((E + 1 + 7) / 8 + 1, T), 256, SMEM, S(stream), W, logits, E, K, 1, c->route_done, o, ypair, extra, rc->x, rc->out, c->xs, 1e-6f));
+                LAUNCHED("combine_route");
+                return MOEXB_OK;
+            };
+            return rc->f16 ? combine.template operator()<true>() : combine.template operator()<false>();
+        }
         // expert parallelism with few own tokens: one token per block row, so that each token's selection and dispatch stores are
         // done by a block of their own instead of one block sending a whole tile of 8
         if (T < 8 || (rep && T <= 16)) {
@@ -1358,9 +1377,9 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
 }
 
 extern "C" {
-static int layer_route(moexb_ctx* c, moexb_layer* L, const void* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr) {
+static int layer_route(moexb_ctx* c, moexb_layer* L, const void* xf, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr, const RouteCombine* rc = nullptr) {
     PROF(c, MOEXB_PROF_ROUTER, stream);
-    return L->router_dtype == MOEXB_F32 ? route_launch<float>(c, L, xf, T, K, stream, decode, ro, tok0, rep) : route_launch<__half>(c, L, xf, T, K, stream, decode, ro, tok0, rep);
+    return L->router_dtype == MOEXB_F32 ? route_launch<float>(c, L, xf, T, K, stream, decode, ro, tok0, rep, rc) : route_launch<__half>(c, L, xf, T, K, stream, decode, ro, tok0, rep, rc);
 }
 
 // Zeroes the bucket counts on `st`. Under capture the graph does it when it runs, so what is in memory now stays marked.
@@ -1388,9 +1407,10 @@ struct BucketCounts {
 
 // One layer. X: the layer input [T][H] of x_dtype. flags as moexb_layer_forward. pre_normed: the context already holds
 // rmsnorm(X) and its split (left there by the previous layer of a stack); next_norm: leave rmsnorm(out) and its
-// split in the context for the next layer.
+// split in the context for the next layer. chain_x (a stack of 2 to 8 tokens): the layer before left its end to this one's router, whose
+// kernel makes X from chain_x, the residual rows of that layer; chain_next: this one leaves its end to the next one.
 static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, int T, int K, float* out, int* idx_out, float* w_out, int flags,
-                      void* stream, bool pre_normed, bool next_norm, int sh0 = 0, int sh1 = -1) {
+                      void* stream, bool pre_normed, bool next_norm, int sh0 = 0, int sh1 = -1, const float* chain_x = nullptr, bool chain_next = false) {
     if (sh1 < 0) sh1 = T;
     const bool shared = !(flags & 1) && sh1 > sh0, block = flags & 2, partial = flags & 4, bf16 = x_dtype == MOEXB_BF16;
     const bool all_local = L->n_local == L->n_routed;
@@ -1411,7 +1431,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     int rc = MOEXB_OK;
     if (block) {
         xr = c->xn;
-        if (!pre_normed || prefill) {   // (the previous layer leaves no rows for the grouped GEMM)
+        if (chain_x) {}
+        else if (!pre_normed || prefill) {   // (the previous layer leaves no rows for the grouped GEMM)
             rc = layer_rows(c, X, x_dtype, T, c->xf, true, c->xn, mode, c->xs, parts, stream);
         } else if (bf16) rc = layer_rows(c, X, x_dtype, T, c->xf, false, nullptr, ROWS_NONE, nullptr, 2, stream);
     } else if (streaming && !prefill && route_splits(T)) {
@@ -1424,7 +1445,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     ro.buckets = buckets; ro.shared = buckets && shared; ro.idx = idx_out; ro.w = w_out;
     if (buckets && c->buckets_dirty) { rc = clear_buckets(c, st); if (rc != MOEXB_OK) return rc; }
     BucketCounts counts{c, st, buckets};
-    rc = layer_route(c, L, xr, T, K, stream, decode, ro);
+    const RouteCombine from_prev{chain_x, const_cast<float*>(xin), f16};
+    rc = layer_route(c, L, xr, T, K, stream, decode, ro, 0, nullptr, chain_x ? &from_prev : nullptr);
     if (rc != MOEXB_OK) return rc;
     if (c->selftest_fail) { c->selftest_fail = false; return fail(MOEXB_ERR_CUDA, "layer: the failure that a self-test asked for"); }
     int ranks = K;                  // rows of ypair per token that the final reduction adds
@@ -1464,12 +1486,13 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
             if (!all_local && !streaming) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)T * K * EH * sizeof(float), st));
         }
         rc = prefill ? grouped_experts(c, L, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
-           : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr)
+           : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr, chain_next)
            : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T * (K + 1), stream)
                        : pairs_launch(c, L->fmt, c->items, c->nitems, min(E, T * K) + 1, c->pairs, xf, c->act, c->ypair, stream);
         if (rc != MOEXB_OK) return rc;
         if (shared) extra = c->ypair + (size_t)T * K * EH;
     }
+    if (chain_next) { counts.open = false; return MOEXB_OK; }
     if (ranks) {
         PROF(c, MOEXB_PROF_COMBINE, stream);
         const float* xres = (block && !partial) ? xin : nullptr;
@@ -1622,13 +1645,19 @@ int moexb_stack_create(moexb_ctx* c, moexb_layer* const* layers, int n_layers, i
     const long long before = g_launches.load();
     e = cudaStreamBeginCapture(s->cap, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) { moexb_stack_destroy(s); return fail(MOEXB_ERR_CUDA, "stack_create: begin capture: %s", cudaGetErrorString(e)); }
+    // 2 to 8 tokens: a layer's end and the next one's routing are one kernel, where every layer has its buckets and all its experts here
+    bool chain = residual && T > 1 && T <= 8 && layers[0]->layout == MOEXB_LAYOUT_TILED && c->bpairs && T < grouped_min_tokens(c, layers[0]->fmt);
+    for (int l = 0; l < n_layers && chain; l++) chain = layers[l]->n_local == layers[l]->n_routed;
     const void* xin = s->x_in;
+    const float* res = x_dtype == MOEXB_BF16 ? c->xf : static_cast<const float*>(s->x_in);   // the residual rows of the layer before
     int rc = MOEXB_OK;
     for (int l = 0; l < n_layers && rc == MOEXB_OK; l++) {
         // layer l leaves rmsnorm(x_{l+1}) and its split in the context, so layer l+1 starts at its router
         const int dt = l ? MOEXB_F32 : x_dtype;
-        if (residual) rc = layer_impl(c, layers[l], xin, dt, T, K, s->buf[l & 1], nullptr, nullptr, 2, s->cap, l > 0, l + 1 < n_layers);
+        if (residual) rc = layer_impl(c, layers[l], xin, dt, T, K, s->buf[l & 1], nullptr, nullptr, 2, s->cap, l > 0, l + 1 < n_layers, 0, -1,
+                                      chain && l ? res : nullptr, chain && l + 1 < n_layers);
         else rc = layer_impl(c, layers[l], xin, dt, T, K, s->buf[l & 1], nullptr, nullptr, 0, s->cap, false, false);
+        if (l) res = static_cast<const float*>(xin);
         xin = s->buf[l & 1];
     }
     e = cudaStreamEndCapture(s->cap, &s->graph);

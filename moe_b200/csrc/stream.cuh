@@ -21,6 +21,7 @@
 #pragma once
 #include "common.cuh"
 #include "rows.cuh"
+#include "router.cuh"
 
 namespace moexb {
 
@@ -473,26 +474,10 @@ __global__ void __launch_bounds__(256) layer_rows_k(const XT* __restrict__ x, fl
     }
 }
 
-// The end of a layer in one pass over the token's row: moe[t] = sum_{r<K} ypair[t*K+r] in rank order (+ extra[t]: the
-// shared expert's row), out[t] = x[t] + moe[t] when x is given (the residual block) else moe[t]; and, when xn_next is
-// given, the next layer's normalised input and its bf16 split straight from the registers. One block of 256 per token.
-template <bool F16>
-__global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __restrict__ ypair, const float* __restrict__ extra, const float* __restrict__ x,
-                                                              float* __restrict__ out, int K, float* __restrict__ xn_next,
-                                                              uint16_t* __restrict__ xs_next, float eps, int ex0, int ex1,
-                                                              const int* __restrict__ idx, int e_lo, int e_hi, int* __restrict__ cnt, int E) {
-    pdl_wait();
-    pdl_trigger();
-    const size_t t = blockIdx.x;
-    if (cnt && t == 0 && (int)threadIdx.x < E) cnt[threadIdx.x] = 0;   // the layer's bucket counts: its expert kernels are done
-    if ((int)t < ex0 || (int)t >= ex1) extra = nullptr;  // extra rows exist only for tokens [ex0, ex1)
-    // idx given: only the ranks whose expert lies in [e_lo, e_hi) were computed here (expert parallelism); skip the others
-    unsigned have = 0xffffffffu;
-    if (idx) {
-        have = 0;
-        for (int r = 0; r < K; r++) { const int e = idx[t * K + r]; if (e >= e_lo && e < e_hi) have |= 1u << r; }
-    }
-    float v[8];
+// A token's row after a layer, 8 values per thread of a block of 256 (4i..4i+3 and 1024+4i..1024+4i+3 of thread i): moe = sum_{r<K} of the
+// ranks' rows in rank order (have: which of the first 32 ranks there are), + extra (the shared expert's row), and x + moe when x is given.
+__device__ __forceinline__ void combine_row(const float* __restrict__ ypair, const float* __restrict__ extra, const float* __restrict__ x, size_t t, int K,
+                                            unsigned have, float (&v)[8]) {
     // both halves of the row in one round trip: the shared expert's row, the residual row and the first eight pair rows of
     // either half are requested before the first addition
     float4 ye[2], yx[2], y0[2][8];
@@ -524,10 +509,91 @@ __global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __res
         }
         if (extra) { acc.x += ye[h].x; acc.y += ye[h].y; acc.z += ye[h].z; acc.w += ye[h].w; }
         if (x) { acc.x = yx[h].x + acc.x; acc.y = yx[h].y + acc.y; acc.z = yx[h].z + acc.z; acc.w = yx[h].w + acc.w; }
-        *reinterpret_cast<float4*>(out + t * EH + k0) = acc;
         v[4 * h] = acc.x; v[4 * h + 1] = acc.y; v[4 * h + 2] = acc.z; v[4 * h + 3] = acc.w;
     }
+}
+__device__ __forceinline__ void store_row(const float (&v)[8], float* __restrict__ out) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) *reinterpret_cast<float4*>(out + 1024 * h + 4 * threadIdx.x) = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+}
+
+// The end of a layer in one pass over the token's row (combine_row) into out and, when xn_next is given, the next layer's normalised
+// input and its split straight from the registers. One block of 256 per token.
+template <bool F16>
+__global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __restrict__ ypair, const float* __restrict__ extra, const float* __restrict__ x,
+                                                              float* __restrict__ out, int K, float* __restrict__ xn_next,
+                                                              uint16_t* __restrict__ xs_next, float eps, int ex0, int ex1,
+                                                              const int* __restrict__ idx, int e_lo, int e_hi, int* __restrict__ cnt, int E) {
+    pdl_wait();
+    pdl_trigger();
+    const size_t t = blockIdx.x;
+    if (cnt && t == 0 && (int)threadIdx.x < E) cnt[threadIdx.x] = 0;   // the layer's bucket counts: its expert kernels are done
+    if ((int)t < ex0 || (int)t >= ex1) extra = nullptr;  // extra rows exist only for tokens [ex0, ex1)
+    // idx given: only the ranks whose expert lies in [e_lo, e_hi) were computed here (expert parallelism); skip the others
+    unsigned have = 0xffffffffu;
+    if (idx) {
+        have = 0;
+        for (int r = 0; r < K; r++) { const int e = idx[t * K + r]; if (e >= e_lo && e < e_hi) have |= 1u << r; }
+    }
+    float v[8];
+    combine_row(ypair, extra, x, t, K, have, v);
+    store_row(v, out + t * EH);
     if (xn_next) norm_split_row<F16>(v, xn_next + t * EH, xs_next ? xs_next + t * 2 * EH : nullptr, eps);
+}
+
+// The end of a residual block and the routing of the next one in one launch, for the 2 to 8 tokens of a stack: route_gemv_k whose blocks
+// make the token's row themselves. A block reads the row's ten addends (80 KB) from L2, which for 34 blocks a token is cheaper than what
+// it saves: a launch of T blocks and the hand-over behind it (stacks of
+// 2, 4 and 7 tokens 23.4, 24.8 and 32.2 -> 22.7, 24.0 and 29.9 us a layer, Q4_K 4 and 7 tokens 37.3 and 42.0 -> 35.4 and 39.6; two weight
+// rows per warp and half the blocks: the same). One block more per token leaves the row
+// (out) and its split (xs) for the experts; the bucket counts are cleared by the down kernel. The weight rows are on their way into
+// shared memory before the wait, every lane its own pieces. Sums and their order are those of the two kernels. 64 KB (f16: 32 KB) of
+// dynamic shared memory.
+template <typename WT, int NJ, bool F16>
+__global__ void __launch_bounds__(256, 2) combine_route_k(const WT* __restrict__ W, float* __restrict__ y, int E, int K, int norm, int* __restrict__ done, const TopkOut o,
+                                                          const float* __restrict__ ypair, const float* __restrict__ extra, const float* __restrict__ x,
+                                                          float* __restrict__ out, uint16_t* __restrict__ xs, float eps) {
+    extern __shared__ __align__(16) uint8_t wsm[];   // [warp][EH] WT
+    __shared__ __align__(16) float xn[EH];
+    const int O = E + 1, t = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x * 8 + warp;
+    const bool rows = blockIdx.x == gridDim.x - 1;   // the block that leaves the token's row
+    WT* wr = reinterpret_cast<WT*>(wsm) + (size_t)warp * EH;
+    if (!rows) {
+        const WT* src = W + (size_t)min(row, O - 1) * EH;
+#pragma unroll
+        for (int u = 0; u < EH / 128; u++) {
+            const int k = 128 * u + 4 * lane;
+            if constexpr (sizeof(WT) == 4) cp_async16(smem_u32(wr + k), src + k); else cp_async8(smem_u32(wr + k), src + k);
+        }
+    }
+    pdl_wait();
+    pdl_trigger();
+    float v[8];
+    combine_row(ypair, extra, x, t, K, 0xffffffffu, v);
+    norm_split_row<F16>(v, xn, rows ? xs + (size_t)t * 2 * EH : nullptr, eps);
+    if (rows) store_row(v, out + (size_t)t * EH);
+    else {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        float acc = 0.f;
+#pragma unroll
+        for (int u = 0; u < EH / 128; u++) {
+            const int k = 128 * u + 4 * lane;
+            float4 w;
+            if constexpr (sizeof(WT) == 4) w = *reinterpret_cast<const float4*>(wr + k);
+            else {
+                const uint2 h = *reinterpret_cast<const uint2*>(wr + k);
+                const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
+                w = make_float4(a.x, a.y, b.x, b.y);
+            }
+            const float4 p = *reinterpret_cast<const float4*>(xn + k);
+            acc = fmaf(w.x, p.x, acc); acc = fmaf(w.y, p.y, acc); acc = fmaf(w.z, p.z, acc); acc = fmaf(w.w, p.w, acc);
+        }
+        acc = warp_sum(acc);
+        if (lane == 0 && row < O) y[(size_t)t * O + row] = acc;
+    }
+    if (!last_block_done(done + t, gridDim.x)) return;
+    if (threadIdx.x < 32) topk_token<NJ, true>(y + (size_t)t * O, t, E, K, norm, lane, o);
 }
 
 // Exclusive prefix sum over the 1024 threads of a block; every thread also gets the total.

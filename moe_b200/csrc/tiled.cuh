@@ -220,6 +220,7 @@ struct TiledArgs {
     uint16_t* act_split;          // gate/up output [p][2][I], permuted
     float* ypair;                 // down output [p][H]
     int* err;
+    int* cnt; int n_cnt;          // down: bucket counts to clear (where no combine kernel follows that does), or null
 };
 
 // Where the work list of a launch comes from (SRC below).
@@ -354,7 +355,12 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     if (!DOWN && Q > 0) { request_columns(sub_at(r0 / RPS)); columns_requested = true; }
     if (lane == 0)
         for (int q = 0; q < D && q < Q; q++) issue(q);
-    if (DOWN) { pdl_wait(); pdl_trigger(); }
+    if (DOWN) {
+        pdl_wait();
+        pdl_trigger();
+        if (a.cnt && blockIdx.x == 0)   // gate/up, which read them, is done
+            for (int i = threadIdx.x; i < a.n_cnt; i += NW * 32) a.cnt[i] = 0;
+    }
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f}, acd[4] = {0.f, 0.f, 0.f, 0.f};  // acd: the second column block
     int cur_sub = -1, n = 0, start = 0;
