@@ -1299,9 +1299,12 @@ struct RouteEp { const EpDevice* dev; int row_bytes; unsigned phase; const unsig
 // the routing kernel (ROWS_F16, ROWS_BF16; only where route_splits)
 struct RouteOut { bool buckets = false, shared = false; int* idx = nullptr; float* w = nullptr; int x_dtype = MOEXB_F32, split = ROWS_NONE; };
 // A stack's layer whose router also makes its input: the end of the layer before (rows of ypair; residual rows x) into out and, split, into
-// the context (combine_route_k; 2 to 8 tokens, whose blocks are there at once, two per SM)
+// the context (combine_route_k; a dozen tokens at most)
 struct RouteCombine { const float* x; float* out; bool f16; };
-static bool route_splits(int T) { return T < 8; }
+// A block per eight outputs of a token, which also splits its rows, for as many tokens as have their blocks on the chip at once (8 of 256
+// experts; beyond, tiles of 8 tokens x 16 outputs). us a layer, tiles against blocks per token: 8 tokens 47.7 / 43.4, 9 bf16 tokens 49.5 /
+// 50.7, 12 and 16 tokens 54.3 / 54.7 and 59.4 / 59.5, 24 tokens 70.7 / 76.2.
+static bool route_splits(int T) { return T <= 8; }
 template <typename WT>
 static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr,
                         const RouteCombine* rc = nullptr) {
@@ -1335,7 +1338,7 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
         }
         // expert parallelism with few own tokens: one token per block row, so that each token's selection and dispatch stores are
         // done by a block of their own instead of one block sending a whole tile of 8
-        if (T < 8 || (rep && T <= 16)) {
+        if (route_splits(T) || (rep && T <= 16)) {
             constexpr int WARPS = 8;
             const dim3 grid((E + 1 + WARPS - 1) / WARPS + (ro.split ? 1 : 0), T);
             uint16_t* xs = ro.split ? c->xs : nullptr;
@@ -1407,7 +1410,7 @@ struct BucketCounts {
 
 // One layer. X: the layer input [T][H] of x_dtype. flags as moexb_layer_forward. pre_normed: the context already holds
 // rmsnorm(X) and its split (left there by the previous layer of a stack); next_norm: leave rmsnorm(out) and its
-// split in the context for the next layer. chain_x (a stack of 2 to 8 tokens): the layer before left its end to this one's router, whose
+// split in the context for the next layer. chain_x (a stack of 2 to 12 tokens): the layer before left its end to this one's router, whose
 // kernel makes X from chain_x, the residual rows of that layer; chain_next: this one leaves its end to the next one.
 static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, int T, int K, float* out, int* idx_out, float* w_out, int flags,
                       void* stream, bool pre_normed, bool next_norm, int sh0 = 0, int sh1 = -1, const float* chain_x = nullptr, bool chain_next = false) {
@@ -1645,8 +1648,10 @@ int moexb_stack_create(moexb_ctx* c, moexb_layer* const* layers, int n_layers, i
     const long long before = g_launches.load();
     e = cudaStreamBeginCapture(s->cap, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) { moexb_stack_destroy(s); return fail(MOEXB_ERR_CUDA, "stack_create: begin capture: %s", cudaGetErrorString(e)); }
-    // 2 to 8 tokens: a layer's end and the next one's routing are one kernel, where every layer has its buckets and all its experts here
-    bool chain = residual && T > 1 && T <= 8 && layers[0]->layout == MOEXB_LAYOUT_TILED && c->bpairs && T < grouped_min_tokens(c, layers[0]->fmt);
+    // 2 to 12 tokens (zero point 8): a layer's end and the next one's routing are one kernel, where every layer has its buckets and all its experts here
+    // (us a layer, two kernels against one: 9, 10, 12, 16, 20 tokens 40.0 / 37.8, 41.2 / 40.4, 44.5 / 44.1, 50.3 / 50.0, 54.8 / 58.0;
+    // zero point 8 and 12 tokens 45.9 / 41.8 and 58.2 / 61.2)
+    bool chain = residual && T > 1 && T <= (layers[0]->fmt == FMT_ZP ? 8 : 12) && layers[0]->layout == MOEXB_LAYOUT_TILED && c->bpairs && T < grouped_min_tokens(c, layers[0]->fmt);
     for (int l = 0; l < n_layers && chain; l++) chain = layers[l]->n_local == layers[l]->n_routed;
     const void* xin = s->x_in;
     const float* res = x_dtype == MOEXB_BF16 ? c->xf : static_cast<const float*>(s->x_in);   // the residual rows of the layer before

@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __res
     if (xn_next) norm_split_row<F16>(v, xn_next + t * EH, xs_next ? xs_next + t * 2 * EH : nullptr, eps);
 }
 
-// The end of a residual block and the routing of the next one in one launch, for the 2 to 8 tokens of a stack: route_gemv_k whose blocks
+// The end of a residual block and the routing of the next one in one launch, for the 2 to 12 tokens of a stack: route_gemv_k whose blocks
 // make the token's row themselves. A block reads the row's ten addends (80 KB) from L2, which for 34 blocks a token is cheaper than what
 // it saves: a launch of T blocks and the hand-over behind it (stacks of
 // 2, 4 and 7 tokens 23.4, 24.8 and 32.2 -> 22.7, 24.0 and 29.9 us a layer, Q4_K 4 and 7 tokens 37.3 and 42.0 -> 35.4 and 39.6; two weight

@@ -141,10 +141,10 @@ def test_k_slices_on_four_warps(fmt, tokens):
 @pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_ZP])
 @pytest.mark.parametrize("router, x_type", [(m.F32, torch.float32), (m.F16, torch.bfloat16)])
 def test_small_stack_equals_chained_layers(fmt, router, x_type):
-    """A stack of 2 to 8 tokens, in which the end of a layer and the routing of the next are one kernel (9: two): the bits of the layers
+    """A stack of 2 to 12 tokens, in which the end of a layer and the routing of the next are one kernel (13: two): the bits of the layers
     called one after the other, on the first run and on a repeated one, and the context takes plain calls afterwards."""
     E, NL = 64, 4
-    c = m.Context(0, max_tokens=9, max_experts=E, top_k=8)
+    c = m.Context(0, max_tokens=13, max_experts=E, top_k=8)
     rng = np.random.default_rng(17)
     layers = []
     for l in range(NL):
@@ -153,7 +153,7 @@ def test_small_stack_equals_chained_layers(fmt, router, x_type):
         L.set_router((rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32 if router == m.F32 else np.float16))
         layers.append(L)
     try:
-        for T in (2, 7, 8, 9):
+        for T in (2, 7, 8, 9, 12, 13):
             X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(DEV).to(x_type)
             s = m.Stack(c, layers, T, 8, m.F32 if x_type == torch.float32 else m.BF16)
             want = X
