@@ -1161,8 +1161,9 @@ static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, const GroupedM
 // Batches from this size on run on the grouped GEMM; where the lines cross depends on how many experts the tokens share. Zero-point blobs
 // from a third of the symmetric formats' size on: their streaming kernels take twice the MMAs and four pairs a pass. us a layer,
 // streaming against grouped, of independent tokens and of a 12-layer stack whose tokens have grown alike:
-//   symmetric   192 tokens 160 / 204 and 162 / 181, 256 tokens 194 / 221 and 194 / 193, 336 tokens 237 / 226 and 231 / 209
-//   zero point   72 tokens 209 / 232 and 167 / 116,  88 tokens 230 / 235 and 185 / 115, 128 tokens 286 / 238 and 250 / 143
+//   symmetric   192 tokens 160 / 193 and 162 / 181, 256 tokens 192 / 210 and 194 / 193, 304 tokens 217 / 214, 336 tokens 232 / 214 and 231 / 209
+//   zero point   72 tokens 206 / 212 and 167 / 116,  88 tokens 224 / 224 and 185 / 115, 128 tokens 285 / 228 and 250 / 143
+// (the stacks' figures are those of the grouped GEMM before its hand-offs were shortened, which took 2 to 5 % off it)
 static int grouped_min_tokens(const moexb_ctx* c, int fmt) {
     const int t = c->prefill_min_tokens;
     return fmt == FMT_ZP ? t / 3 + (t % 3 != 0) : t;   // (any threshold up to the largest int)
@@ -1298,9 +1299,9 @@ struct RouteEp { const EpDevice* dev; int row_bytes; unsigned phase; const unsig
 // pairs into the buckets (with the shared expert's); the caller's copies of ids and weights; split: the rows of x (x_dtype) are split by
 // the routing kernel (ROWS_F16, ROWS_BF16; only where route_splits)
 struct RouteOut { bool buckets = false, shared = false; int* idx = nullptr; float* w = nullptr; int x_dtype = MOEXB_F32, split = ROWS_NONE; };
-// A stack's layer whose router also makes its input: the end of the layer before (rows of ypair; residual rows x) into out and, split, into
-// the context (combine_route_k; a dozen tokens at most)
-struct RouteCombine { const float* x; float* out; bool f16; };
+// A layer whose router also makes its input rows and, split, leaves them in the context (combine_route_k): in a stack the end of the layer
+// before (ranks rows of ypair a token; residual rows x; out; a dozen tokens at most), or the norm of the rows x of x_dtype (ranks = 0)
+struct RouteCombine { const void* x; int x_dtype, ranks; float* out; bool f16; };
 // A block per eight outputs of a token, which also splits its rows, for as many tokens as have their blocks on the chip at once (8 of 256
 // experts; beyond, tiles of 8 tokens x 16 outputs). us a layer, tiles against blocks per token: 8 tokens 47.7 / 43.4, 9 bf16 tokens 49.5 /
 // 50.7, 12 and 16 tokens 54.3 / 54.7 and 59.4 / 59.5, 24 tokens 70.7 / 76.2.
@@ -1323,18 +1324,20 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
     if (rep) { o.ep = rep->dev; o.ep_row_bytes = rep->row_bytes; o.ep_phase = rep->phase; o.ep_step = rep->step; }
     auto run = [&]<int NJ>() -> int {
         if (rc) {
-            auto combine = [&]<bool F16>() -> int {
-                constexpr auto kernel = combine_route_k<WT, NJ, F16>;
+            auto combine = [&]<bool F16, typename XT>() -> int {
+                constexpr auto kernel = combine_route_k<WT, NJ, F16, XT>;
                 constexpr int SMEM = 8 * EH * (int)sizeof(WT);
                 static PerDeviceOnce once;
                 const cudaError_t attr_err = once.run([] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); });
                 if (attr_err != cudaSuccess) return fail(MOEXB_ERR_CUDA, "router kernel shared memory: %s", cudaGetErrorString(attr_err));
-                const float *ypair = c->ypair, *extra = c->ypair + (size_t)T * K * EH;
-                CUDA_TRY(launch_dep(kernel, dim3((E + 1 + 7) / 8 + 1, T), 256, SMEM, S(stream), W, logits, E, K, 1, c->route_done, o, ypair, extra, rc->x, rc->out, c->xs, 1e-6f));
+                const float *ypair = c->ypair, *extra = rc->ranks ? c->ypair + (size_t)T * K * EH : nullptr;
+                CUDA_TRY(launch_dep(kernel, dim3((E + 1 + 7) / 8 + 1, T), 256, SMEM, S(stream), W, logits, E, K, 1, c->route_done, o, ypair, extra, static_cast<const XT*>(rc->x), rc->ranks,
+                                    rc->out, c->xs, 1e-6f));
                 LAUNCHED("combine_route");
                 return MOEXB_OK;
             };
-            return rc->f16 ? combine.template operator()<true>() : combine.template operator()<false>();
+            if (rc->x_dtype == MOEXB_BF16) return rc->f16 ? combine.template operator()<true, __nv_bfloat16>() : combine.template operator()<false, __nv_bfloat16>();
+            return rc->f16 ? combine.template operator()<true, float>() : combine.template operator()<false, float>();
         }
         // expert parallelism with few own tokens: one token per block row, so that each token's selection and dispatch stores are
         // done by a block of their own instead of one block sending a whole tile of 8
@@ -1432,9 +1435,12 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     const void* xr = xin;
     RouteOut ro;
     int rc = MOEXB_OK;
+    // a few tokens: the routing kernel normalises and splits the rows itself (us a layer, by a launch before it against that: 9, 12, 16, 20
+    // tokens 50.0 / 47.6, 55.5 / 53.9, 60.2 / 59.4, 68.1 / 70.4; zero point 9 and 12 tokens 72.9 / 70.5, 89.7 / 88.8)
+    const bool norm_in_route = block && !pre_normed && streaming && !prefill && T <= 16;
     if (block) {
         xr = c->xn;
-        if (chain_x) {}
+        if (chain_x || norm_in_route) {}
         else if (!pre_normed || prefill) {   // (the previous layer leaves no rows for the grouped GEMM)
             rc = layer_rows(c, X, x_dtype, T, c->xf, true, c->xn, mode, c->xs, parts, stream);
         } else if (bf16) rc = layer_rows(c, X, x_dtype, T, c->xf, false, nullptr, ROWS_NONE, nullptr, 2, stream);
@@ -1448,8 +1454,8 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     ro.buckets = buckets; ro.shared = buckets && shared; ro.idx = idx_out; ro.w = w_out;
     if (buckets && c->buckets_dirty) { rc = clear_buckets(c, st); if (rc != MOEXB_OK) return rc; }
     BucketCounts counts{c, st, buckets};
-    const RouteCombine from_prev{chain_x, const_cast<float*>(xin), f16};
-    rc = layer_route(c, L, xr, T, K, stream, decode, ro, 0, nullptr, chain_x ? &from_prev : nullptr);
+    const RouteCombine rows = chain_x ? RouteCombine{chain_x, MOEXB_F32, K, const_cast<float*>(xin), f16} : RouteCombine{X, x_dtype, 0, bf16 ? c->xf : nullptr, f16};
+    rc = layer_route(c, L, xr, T, K, stream, decode, ro, 0, nullptr, chain_x || norm_in_route ? &rows : nullptr);
     if (rc != MOEXB_OK) return rc;
     if (c->selftest_fail) { c->selftest_fail = false; return fail(MOEXB_ERR_CUDA, "layer: the failure that a self-test asked for"); }
     int ranks = K;                  // rows of ypair per token that the final reduction adds

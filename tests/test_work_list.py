@@ -168,3 +168,34 @@ def test_small_stack_equals_chained_layers(fmt, router, x_type):
         for L in layers:
             L.close()
         c.close()
+
+
+@pytest.mark.parametrize("fmt, layout", [(m.FMT_SYM_F16, m.LAYOUT_TILED), (m.FMT_ZP, m.LAYOUT_TILED), (m.FMT_SYM_F32, m.LAYOUT_REFERENCE)])
+@pytest.mark.parametrize("x_type", [torch.float32, torch.bfloat16])
+def test_blocks_of_a_few_tokens(fmt, layout, x_type):
+    """Residual blocks whose norm and split are made by the routing kernel (1 to 16 tokens; 17: by a launch before it), against the oracle; a
+    bf16 row that begins on 4 bytes gives the same bits."""
+    E = 32
+    c = m.Context(0, max_tokens=17, max_experts=E, top_k=8)
+    L = m.Layer(c, fmt, E, layout=layout)
+    L.fill_synth(3, 0)
+    rng = np.random.default_rng(19)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    host = [m.synth_expert_host(fmt, 3, 0, e) for e in range(E + 1)]
+    try:
+        for T in (1, 2, 8, 9, 16, 17):
+            X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(x_type)
+            xf = X.float().numpy()
+            idx = torch.empty(T, 8, dtype=torch.int32, device=DEV)
+            got = L.forward(X.to(DEV), T, 8, idx=idx, flags=2)
+            assert c.status() == 0
+            ref, ids, _, _ = o.layer_forward(fmt, host, W, o.rmsnorm(xf), 8)
+            assert np.array_equal(idx.cpu().numpy(), ids)
+            check_ffn(got.cpu().numpy(), xf + ref, fmt, f"block of {T} {x_type} tokens")
+            if x_type == torch.bfloat16:
+                at2 = torch.empty(T * 2048 + 2, dtype=x_type, device=DEV)[2:]
+                at2.copy_(X.view(-1))
+                assert torch.equal(L.forward(at2.view(T, 2048), T, 8, flags=2), got)
+    finally:
+        L.close(); c.close()
