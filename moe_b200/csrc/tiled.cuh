@@ -220,7 +220,6 @@ struct TiledArgs {
     uint16_t* act_split;          // gate/up output [p][2][I], permuted
     float* ypair;                 // down output [p][H]
     int* err;
-    int* cnt; int n_cnt;          // down: bucket counts to clear (where no combine kernel follows that does), or null
 };
 
 // Where the work list of a launch comes from (SRC below).
@@ -358,8 +357,8 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     if (DOWN) {
         pdl_wait();
         pdl_trigger();
-        if (a.cnt && blockIdx.x == 0)   // gate/up, which read them, is done
-            for (int i = threadIdx.x; i < a.n_cnt; i += NW * 32) a.cnt[i] = 0;
+        if (ba.cnt && blockIdx.x == 0)   // bucket counts that no combine kernel will clear; gate/up, which read them, is done
+            for (int i = threadIdx.x; i < ba.E; i += NW * 32) const_cast<int*>(ba.cnt)[i] = 0;
     }
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f}, acd[4] = {0.f, 0.f, 0.f, 0.f};  // acd: the second column block
