@@ -212,6 +212,11 @@ int moexb_ctx_status(moexb_ctx* ctx, int* status);
  * raising its abort word (kernels.cuh:1055-1089). */
 int moexb_ctx_selftest_timeout(moexb_ctx* ctx, int which, int polls, int* status);
 
+/* The grouped GEMM's branch-free g / (1 + exp(-g)) against the division, for every float g: out[0] = values that differ (zeros of
+ * either sign are alike, and NaNs), out[1] = those of them where only one is NaN or infinite, or both infinite with other signs,
+ * out[2] = the largest distance of two finite values in units of the last place. Synchronous. */
+int moexb_ctx_selftest_swiglu(moexb_ctx* ctx, unsigned long long out[3]);
+
 /* The next layer-level call on the context that runs the experts returns MOEXB_ERR_CUDA after its router was enqueued, as if a
  * launch had failed there. What later calls on the context give must not depend on it. */
 int moexb_ctx_selftest_fail(moexb_ctx* ctx);

@@ -52,6 +52,7 @@ SIGNATURES = {
     "moexb_ctx_status": (_i, [_vp, C.POINTER(_i)]),
     "moexb_ctx_selftest_fail": (_i, [_vp]),
     "moexb_ctx_selftest_timeout": (_i, [_vp, _i, _i, C.POINTER(_i)]),
+    "moexb_ctx_selftest_swiglu": (_i, [_vp, C.POINTER(C.c_ulonglong)]),
     "moexb_pairs_reduce": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp, _vp]),
     "moexb_gated_add_rows": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "moexb_shared_expert_add": (_i, [_i, _vp, _vp, _i, _vp, _i, _vp, _vp, _vp]),

@@ -202,6 +202,13 @@ class Context:
         check(lib().moexb_ctx_selftest_timeout(self.h, which, polls, C.byref(st)))
         return st.value
 
+    def selftest_swiglu(self):
+        """moexb_ctx_selftest_swiglu: (values that differ from the division, of them NaN or infinite on one side, largest
+        distance in ulp) over every float gate value."""
+        out = (C.c_ulonglong * 3)()
+        check(lib().moexb_ctx_selftest_swiglu(self.h, out))
+        return tuple(out)
+
     def selftest_fail(self):
         """moexb_ctx_selftest_fail: the next layer call returns an error after its router was enqueued."""
         check(lib().moexb_ctx_selftest_fail(self.h))

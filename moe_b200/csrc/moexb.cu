@@ -1287,6 +1287,18 @@ extern "C" int moexb_ctx_selftest_timeout(moexb_ctx* c, int which, int polls, in
     return moexb_ctx_status(c, status);
 }
 
+extern "C" int moexb_ctx_selftest_swiglu(moexb_ctx* c, unsigned long long out[3]) {
+    REQUIRE(c && out, "ctx_selftest_swiglu: null pointer");
+    CUDA_TRY(cudaSetDevice(c->device));
+    unsigned long long* d = nullptr;
+    CUDA_TRY(cudaMalloc((void**)&d, 3 * sizeof(*d)));
+    cudaError_t e = cudaMemset(d, 0, 3 * sizeof(*d));
+    if (e == cudaSuccess) { selftest_swiglu_k<<<c->sms * 8, 256>>>(d); e = cudaGetLastError(); }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d, 3 * sizeof(*d), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? MOEXB_OK : fail(MOEXB_ERR_CUDA, "ctx_selftest_swiglu: %s", cudaGetErrorString(e));
+}
+
 extern "C" {
 
 // Router logits (column n_routed = the shared expert's gate logit) and top-K for T tokens, into the context workspace.

@@ -84,3 +84,51 @@ def test_grouped_gemm_repeats_bit_for_bit(fmt):
         assert c.status() == 0
     finally:
         L.close(); c.close()
+
+
+def test_the_branch_free_silu_is_the_division():
+    """Every float gate value, the infinities, NaN and the quotients near the end of the range among them: the bits of CUDA's correctly
+    rounded division, but for the sign of zero."""
+    c = m.Context(0, max_tokens=1, max_experts=E, top_k=K)
+    try:
+        assert c.selftest_swiglu() == (0, 0, 0)
+    finally:
+        c.close()
+
+
+def test_an_overflowed_gate_row_marks_its_tokens():
+    """One gate row of an expert overflows to +inf or -inf: silu of either is no finite number, so every token that selected the expert
+    has an output of none, as in the oracle and on the streaming kernels; the other tokens' outputs are those without the overflow."""
+    T, fmt = 40, m.FMT_SYM_F32
+    c = m.Context(0, max_tokens=T, max_experts=E, top_k=K)
+    L = m.Layer(c, fmt, E)
+    L.fill_synth(3, 0)
+    rng = np.random.default_rng(23)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    host = [m.synth_expert_host(fmt, 3, 0, e) for e in range(E + 1)]
+    X = rng.standard_normal((T, 2048)).astype(np.float32)
+    idx = torch.empty(T, K, dtype=torch.int32, device=DEV)
+    x = torch.from_numpy(X).to(DEV)
+    try:
+        c.set_prefill_min_tokens(1)
+        want = L.forward(x, T, K, idx=idx).cpu().numpy()
+        expert = int(np.bincount(idx.cpu().numpy().ravel(), minlength=E).argmax())
+        hit = (idx.cpu().numpy() == expert).any(axis=1)
+        row, group = 100, 5   # the scale of 64 inputs of one gate row: 32 groups a row
+        blob = host[expert].copy()
+        blob[m.Q_BYTES + (row * 32 + group) * 4:][:4] = np.frombuffer(np.float32(3e38).tobytes(), np.uint8)
+        host[expert] = blob
+        L.upload_blob(expert, blob)
+        with np.errstate(all="ignore"):
+            ref, _, _, _ = o.layer_forward(fmt, host, W, X, K)
+            assert np.array_equal(~np.isfinite(ref).all(axis=1), hit) and 0 < hit.sum() < T
+            for min_tokens in (1, 1 << 20):   # the grouped GEMM, the streaming kernels
+                c.set_prefill_min_tokens(min_tokens)
+                got = L.forward(x, T, K).cpu().numpy()
+                assert np.array_equal(~np.isfinite(got).any(axis=1), hit), min_tokens
+                if min_tokens == 1:
+                    assert np.array_equal(got[~hit], want[~hit])
+        assert c.status() == 0
+    finally:
+        L.close(); c.close()
