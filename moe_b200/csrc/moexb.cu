@@ -1125,21 +1125,22 @@ static bool plan_in_kernel(int fmt, int T, int K, int E) {
 // makes it and leaves it in the context for the down kernel; buckets = the router's; neither = it is in the context.
 static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int T, void* stream, const PlanArgs* plan = nullptr,
                          const BucketArgs* buckets = nullptr, bool clear = false) {
-    const TiledArgs a{c->subs, c->nsub, buckets ? buckets->pairs : pairs, c->xs, act32, c->act_split, ypair, c->err};
+    const TiledArgs a{c->subs, c->nsub, buckets ? buckets->pairs : pairs, c->xs, act32, c->act_split, ypair, c->err, nullptr, 0};
     TiledArgs d = a;
     d.xs = c->act_split;
+    if (clear && buckets) { d.clear = c->bcnt; d.experts = buckets->E; }
     PlanArgs pa = plan ? *plan : PlanArgs{};
     pa.subs_out = c->subs; pa.nsub_out = c->nsub;
-    const BucketArgs ba = buckets ? *buckets : BucketArgs{}, bd = clear ? ba : BucketArgs{};   // bd: what the down kernel clears
+    const BucketArgs ba = buckets ? *buckets : BucketArgs{};
     return by_fmt(fmt, [&]<int FMT>() {
         int rc;
         if (buckets) {
             rc = tiled_launch_one<FMT, false, TL_BUCKETS>(c, a, T, stream, pa, ba);
-            return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, bd);
+            return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, ba);
         }
         if constexpr (FMT == FMT_SYM_F16) rc = plan ? tiled_launch_one<FMT, false, TL_PLAN>(c, a, T, stream, pa, ba) : tiled_launch_one<FMT, false, TL_LIST>(c, a, T, stream, pa, ba);
         else rc = tiled_launch_one<FMT, false, TL_LIST>(c, a, T, stream, pa, ba);
-        return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, bd);
+        return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, ba);
     });
 }
 
