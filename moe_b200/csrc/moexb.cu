@@ -1314,10 +1314,12 @@ struct RouteOut { bool buckets = false, shared = false; int* idx = nullptr; floa
 // A layer whose router also makes its input rows and, split, leaves them in the context (combine_route_k): in a stack the end of the layer
 // before (ranks rows of ypair a token; residual rows x; out; a dozen tokens at most), or the norm of the rows x of x_dtype (ranks = 0)
 struct RouteCombine { const void* x; int x_dtype, ranks; float* out; bool f16; };
-// A block per eight outputs of a token, which also splits its rows, for as many tokens as have their blocks on the chip at once (8 of 256
-// experts; beyond, tiles of 8 tokens x 16 outputs). us a layer, tiles against blocks per token: 8 tokens 47.7 / 43.4, 9 bf16 tokens 49.5 /
-// 50.7, 12 and 16 tokens 54.3 / 54.7 and 59.4 / 59.5, 24 tokens 70.7 / 76.2.
-static bool route_splits(int T) { return T <= 8; }
+// A block per eight outputs of a token, which also splits its rows: up to 7 tokens, and 8 where the blocks are no more than two per SM (288
+// experts); beyond, tiles of 8 tokens x 16 outputs. us a layer, tiles against blocks per token: 8 tokens of 32, 128, 256, 512 and 1024 experts
+// 35.0 / 29.7, 42.4 / 36.6, 45.6 / 42.0, 59.3 / 60.1 and 67.0 / 75.7, of bf16 rows 35.0 / 31.1, 42.2 / 39.4, 45.5 / 45.6, 59.0 / 66.1 and
+// 67.1 / 86.0; 256 experts 9 bf16 tokens 49.5 / 50.7, 12 and 16 tokens 54.3 / 54.7 and 59.4 / 59.5, 24 tokens 70.7 / 76.2.
+static int route_blocks(int T, int E) { return T * ((E + 8) / 8); }
+static bool route_splits(const moexb_ctx* c, int T, int E) { return T < 8 || (T == 8 && route_blocks(T, E) <= 2 * c->sms); }
 template <typename WT>
 static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int K, void* stream, bool decode, const RouteOut& ro, int tok0 = 0, const RouteEp* rep = nullptr,
                         const RouteCombine* rc = nullptr) {
@@ -1353,7 +1355,7 @@ static int route_launch(moexb_ctx* c, moexb_layer* L, const void* x, int T, int 
         }
         // expert parallelism with few own tokens: one token per block row, so that each token's selection and dispatch stores are
         // done by a block of their own instead of one block sending a whole tile of 8
-        if (route_splits(T) || (rep && T <= 16)) {
+        if (route_splits(c, T, E) || (rep && T <= 16)) {
             constexpr int WARPS = 8;
             const dim3 grid((E + 1 + WARPS - 1) / WARPS + (ro.split ? 1 : 0), T);
             uint16_t* xs = ro.split ? c->xs : nullptr;
@@ -1456,7 +1458,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
         else if (!pre_normed || prefill) {   // (the previous layer leaves no rows for the grouped GEMM)
             rc = layer_rows(c, X, x_dtype, T, c->xf, true, c->xn, mode, c->xs, parts, stream);
         } else if (bf16) rc = layer_rows(c, X, x_dtype, T, c->xf, false, nullptr, ROWS_NONE, nullptr, 2, stream);
-    } else if (streaming && !prefill && route_splits(T)) {
+    } else if (streaming && !prefill && route_splits(c, T, E)) {
         xr = X; ro.x_dtype = x_dtype; ro.split = mode;
     } else if (mode != ROWS_NONE || bf16) rc = layer_rows(c, X, x_dtype, T, c->xf, false, nullptr, mode, c->xs, parts, stream);
     if (rc != MOEXB_OK) return rc;

@@ -199,3 +199,35 @@ def test_blocks_of_a_few_tokens(fmt, layout, x_type):
                 assert torch.equal(L.forward(at2.view(T, 2048), T, 8, flags=2), got)
     finally:
         L.close(); c.close()
+
+
+# experts, tokens, residual block; kernels of a call: routing, gate/up, down and combine, one more where a launch before the routing prepares
+# the rows, and one more for the work list of layers whose experts are too many for the buckets
+ROUTES = [(256, 8, False, 4), (288, 8, False, 5), (320, 8, False, 6), (1024, 7, False, 5), (1024, 8, False, 6)]
+
+
+@pytest.mark.parametrize("E, T, block, kernels", ROUTES)
+def test_the_rows_of_a_few_tokens_by_the_number_of_routing_blocks(E, T, block, kernels):
+    """Whether the routing kernel or a launch before it prepares the rows depends on the experts as well as on the tokens. The selected
+    experts are the oracle's on either side of the line, and the outputs those of calls of fewer tokens, which always leave it to the
+    routing kernel."""
+    c = m.Context(0, max_tokens=16, max_experts=E, top_k=8)
+    L = m.Layer(c, m.FMT_SYM_F16, E)
+    L.fill_synth(3, 0)
+    rng = np.random.default_rng(E + T)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    X = rng.standard_normal((T, 2048)).astype(np.float32)
+    x, flags = dev(X), 2 if block else 0
+    idx = torch.empty(T, 8, dtype=torch.int32, device=DEV)
+    try:
+        before = m.launch_count()
+        got = L.forward(x, T, 8, idx=idx, flags=flags).cpu().numpy()
+        assert m.launch_count() - before == kernels
+        ids, _ = o.router_topk(o.router_logits(W, o.rmsnorm(X) if block else X, T), E, 8, True, T, E + 1)
+        assert np.array_equal(idx.cpu().numpy(), ids)
+        parts = [L.forward(x[t:t + 4].contiguous(), min(4, T - t), 8, flags=flags).cpu().numpy() for t in range(0, T, 4)]
+        check_ffn(got, np.concatenate(parts), m.FMT_SYM_F16, f"{T} tokens of {E} experts against calls of 4")
+        assert c.status() == 0
+    finally:
+        L.close(); c.close()
