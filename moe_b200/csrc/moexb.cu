@@ -1449,9 +1449,12 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
     const void* xr = xin;
     RouteOut ro;
     int rc = MOEXB_OK;
-    // a few tokens: the routing kernel normalises and splits the rows itself (us a layer, by a launch before it against that: 9, 12, 16, 20
-    // tokens 50.0 / 47.6, 55.5 / 53.9, 60.2 / 59.4, 68.1 / 70.4; zero point 9 and 12 tokens 72.9 / 70.5, 89.7 / 88.8)
-    const bool norm_in_route = block && !pre_normed && streaming && !prefill && T <= 16;
+    // A few tokens: the routing kernel normalises and splits the rows itself, up to 16 tokens and as many blocks as read their outputs' weights
+    // in about the time of that launch (f16 weights are half as long). us a layer, by a launch before it against that: 256 experts 9, 12, 16,
+    // 20 tokens 50.0 / 47.6, 55.5 / 53.9, 60.2 / 59.4, 68.1 / 70.4; zero point 9 and 12 tokens 72.9 / 70.5, 89.7 / 88.8; 512 experts 12 and 16
+    // tokens 69.0 / 66.1 and 79.7 / 80.6, 1024 experts 8, 10, 12, 16 tokens 67.8 / 66.5, 72.8 / 73.1, 76.9 / 82.2, 88.4 / 99.5; f16 weights 512
+    // experts 16 tokens 82.0 / 77.8, 1024 experts 10, 12, 16 tokens 74.2 / 69.1, 78.4 / 77.7, 90.6 / 94.6.
+    const bool norm_in_route = block && !pre_normed && streaming && !prefill && T <= 16 && route_blocks(T, E) <= (L->router_dtype == MOEXB_F32 ? 7 : 11) * c->sms;
     if (block) {
         xr = c->xn;
         if (chain_x || norm_in_route) {}

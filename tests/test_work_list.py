@@ -203,19 +203,21 @@ def test_blocks_of_a_few_tokens(fmt, layout, x_type):
 
 # experts, tokens, residual block; kernels of a call: routing, gate/up, down and combine, one more where a launch before the routing prepares
 # the rows, and one more for the work list of layers whose experts are too many for the buckets
-ROUTES = [(256, 8, False, 4), (288, 8, False, 5), (320, 8, False, 6), (1024, 7, False, 5), (1024, 8, False, 6)]
+ROUTES = [(256, 8, False, m.F32, 4), (288, 8, False, m.F32, 5), (320, 8, False, m.F32, 6), (1024, 7, False, m.F32, 5), (1024, 8, False, m.F32, 6),
+          (256, 16, True, m.F32, 4), (512, 15, True, m.F32, 5), (512, 16, True, m.F32, 6), (1024, 8, True, m.F32, 5), (1024, 9, True, m.F32, 6),
+          (1024, 12, True, m.F16, 5), (1024, 13, True, m.F16, 6)]
 
 
-@pytest.mark.parametrize("E, T, block, kernels", ROUTES)
-def test_the_rows_of_a_few_tokens_by_the_number_of_routing_blocks(E, T, block, kernels):
+@pytest.mark.parametrize("E, T, block, router, kernels", ROUTES)
+def test_the_rows_of_a_few_tokens_by_the_number_of_routing_blocks(E, T, block, router, kernels):
     """Whether the routing kernel or a launch before it prepares the rows depends on the experts as well as on the tokens. The selected
     experts are the oracle's on either side of the line, and the outputs those of calls of fewer tokens, which always leave it to the
     routing kernel."""
     c = m.Context(0, max_tokens=16, max_experts=E, top_k=8)
-    L = m.Layer(c, m.FMT_SYM_F16, E)
+    L = m.Layer(c, m.FMT_SYM_F16, E, router_dtype=router)
     L.fill_synth(3, 0)
     rng = np.random.default_rng(E + T)
-    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32 if router == m.F32 else np.float16)
     L.set_router(W)
     X = rng.standard_normal((T, 2048)).astype(np.float32)
     x, flags = dev(X), 2 if block else 0
