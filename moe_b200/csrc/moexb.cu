@@ -1095,13 +1095,14 @@ static int tiled_launch_cfg(moexb_ctx* c, const TiledArgs& a, const PlanArgs& pa
 // From 8 tokens on the symmetric formats also take sub-items of up to 8 pairs (two column blocks; tiled_maxp below): the
 // gate/up columns of 8 pairs are 66 KB, so that kernel runs as one CTA of 16 warps per SM.
 template <int FMT, bool DOWN, int SRC>
-static int tiled_launch_one(moexb_ctx* c, const TiledArgs& a, int T, void* stream, const PlanArgs& pa, const BucketArgs& ba) {
+static int tiled_launch_one(moexb_ctx* c, const TiledArgs& a, int T, int K, void* stream, const PlanArgs& pa, const BucketArgs& ba) {
     static_assert(SRC != TL_PLAN || FMT == FMT_SYM_F16, "the in-kernel work list fits beside the ring of the fp16-scale format only");
-    // The K slices of a row tile on four warps: one zero-point token (9 sub-items, a slice per warp: 26.0 -> 21.6 us a layer; symmetric
+    // The K slices of a row tile on four warps: one zero-point token whose K + 1 sub-items give a CTA no more than a third of a whole round
+    // (K = 2, 4, 8, 11, 12, 15: 21.8 / 18.9, 24.1 / 19.5, 26.7 / 22.3, 30.1 / 29.5, 30.8 / 30.8, 32.0 / 32.2 us a layer, without and with; symmetric
     // formats 19.2 either way), and 8 to 15 tokens of the symmetric formats, where whole rounds are two or three per CTA and leave many
     // CTAs with one less (8, 9, 11, 14 tokens 47.9, 50.1, 55.8, 58.3 -> 46.7, 49.2, 52.6, 58.0 us; stacks of 10 and 12 43.7, 48.1 -> 41.6, 44.2;
     // 16 and 23 tokens 59.8, 71.5 -> 60.5, 72.1; zero point 9 and 14 tokens 71.4, 92.9 -> 73.1, 90.1).
-    if constexpr (!DOWN && FMT == FMT_ZP) { if (T == 1) return tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream); }
+    if constexpr (!DOWN && FMT == FMT_ZP) { if (T == 1 && 12 * (K + 1) <= c->sms) return tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream); }
     else if constexpr (!DOWN) {
         if (T >= 8 && T < 16) return c->pairs_per_pass == 4 ? tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream)
                                                             : tiled_launch_cfg<FMT, DOWN, 16, 2, 2, 1, SRC, true>(c, a, pa, ba, stream);
@@ -1123,7 +1124,7 @@ static bool plan_in_kernel(int fmt, int T, int K, int E) {
 
 // The same on blobs in the tiled layout (sub-item slots point into a tiled layer image). The work list: plan = the gate/up kernel
 // makes it and leaves it in the context for the down kernel; buckets = the router's; neither = it is in the context.
-static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int T, void* stream, const PlanArgs* plan = nullptr,
+static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* act32, float* ypair, int T, int K, void* stream, const PlanArgs* plan = nullptr,
                          const BucketArgs* buckets = nullptr, bool clear = false) {
     const TiledArgs a{c->subs, c->nsub, buckets ? buckets->pairs : pairs, c->xs, act32, c->act_split, ypair, c->err, nullptr, 0};
     TiledArgs d = a;
@@ -1135,12 +1136,12 @@ static int tiled_experts(moexb_ctx* c, int fmt, const moexb_pair* pairs, float* 
     return by_fmt(fmt, [&]<int FMT>() {
         int rc;
         if (buckets) {
-            rc = tiled_launch_one<FMT, false, TL_BUCKETS>(c, a, T, stream, pa, ba);
-            return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, ba);
+            rc = tiled_launch_one<FMT, false, TL_BUCKETS>(c, a, T, K, stream, pa, ba);
+            return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, K, stream, pa, ba);
         }
-        if constexpr (FMT == FMT_SYM_F16) rc = plan ? tiled_launch_one<FMT, false, TL_PLAN>(c, a, T, stream, pa, ba) : tiled_launch_one<FMT, false, TL_LIST>(c, a, T, stream, pa, ba);
-        else rc = tiled_launch_one<FMT, false, TL_LIST>(c, a, T, stream, pa, ba);
-        return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, stream, pa, ba);
+        if constexpr (FMT == FMT_SYM_F16) rc = plan ? tiled_launch_one<FMT, false, TL_PLAN>(c, a, T, K, stream, pa, ba) : tiled_launch_one<FMT, false, TL_LIST>(c, a, T, K, stream, pa, ba);
+        else rc = tiled_launch_one<FMT, false, TL_LIST>(c, a, T, K, stream, pa, ba);
+        return rc != MOEXB_OK ? rc : tiled_launch_one<FMT, true, TL_LIST>(c, d, T, K, stream, pa, ba);
     });
 }
 
@@ -1490,7 +1491,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
         }
         ranks = 0;
     } else if (decode) {
-        rc = tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream) : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, K + 1, stream);
+        rc = tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, K, stream) : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, K + 1, stream);
         if (rc != MOEXB_OK) return rc;
         ranks = K + 1;
     } else {
@@ -1512,7 +1513,7 @@ static int layer_impl(moexb_ctx* c, moexb_layer* L, const void* X, int x_dtype, 
             if (!all_local && !streaming) CUDA_TRY(cudaMemsetAsync(c->ypair, 0, (size_t)T * K * EH * sizeof(float), st));
         }
         rc = prefill ? grouped_experts(c, L, c->pairs, parts, c->ypair, stream, buckets ? &bk : nullptr)
-           : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, nullptr, buckets ? &bk : nullptr, chain_next)
+           : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, K, stream, nullptr, buckets ? &bk : nullptr, chain_next)
            : streaming ? stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T * (K + 1), stream)
                        : pairs_launch(c, L->fmt, c->items, c->nitems, min(E, T * K) + 1, c->pairs, xf, c->act, c->ypair, stream);
         if (rc != MOEXB_OK) return rc;
@@ -1950,7 +1951,7 @@ int moexb_ep_experts(moexb_ep* e, moexb_layer* L, int l, void* stream) {
         LAUNCHED("group_plan");
     }
     rc = prefill ? grouped_experts(c, L, c->pairs, e->parts, c->ypair, stream)
-       : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, stream, in_kernel ? &plan : nullptr)
+       : tiled ? tiled_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T, K, stream, in_kernel ? &plan : nullptr)
                : stream_experts(c, L->fmt, c->pairs, nullptr, c->ypair, T * (K + 1), stream);
     if (rc != MOEXB_OK) return rc;
     PROF(c, MOEXB_PROF_COMBINE, stream);

@@ -233,3 +233,24 @@ def test_the_rows_of_a_few_tokens_by_the_number_of_routing_blocks(E, T, block, r
         assert c.status() == 0
     finally:
         L.close(); c.close()
+
+
+@pytest.mark.parametrize("K", [1, 11, 12, 15])
+def test_one_zero_point_token_by_its_number_of_experts(K):
+    """The K slices of a row tile on four warps up to 11 experts, on one warp beyond, against the oracle."""
+    E = 32
+    c = m.Context(0, max_tokens=1, max_experts=E, top_k=15)
+    L = m.Layer(c, m.FMT_ZP, E)
+    L.fill_synth(3, 0)
+    rng = np.random.default_rng(K)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    L.set_router(W)
+    X = rng.standard_normal((1, 2048)).astype(np.float32)
+    idx = torch.empty(1, K, dtype=torch.int32, device=DEV)
+    try:
+        got = L.forward(dev(X), 1, K, idx=idx).cpu().numpy()
+        ref, ids, _, _ = o.layer_forward(m.FMT_ZP, [m.synth_expert_host(m.FMT_ZP, 3, 0, e) for e in range(E + 1)], W, X, K)
+        assert c.status() == 0 and np.array_equal(idx.cpu().numpy(), ids)
+        check_ffn(got, ref, m.FMT_ZP, f"one zero-point token through {K} experts")
+    finally:
+        L.close(); c.close()
