@@ -62,7 +62,7 @@ def test_pairs_and_one_token_calls(blobs, fmt):
 @pytest.mark.parametrize("fmt,min_tokens", [(m.FMT_SYM_F16, 1 << 20), (m.FMT_ZP, 1 << 20), (m.FMT_SYM_F16, 1), (m.FMT_ZP, 1)])
 @pytest.mark.parametrize("flags", [0, 2])
 def test_bf16_rows_of_a_layer(fmt, min_tokens, flags):
-    """bf16 rows on a 4-byte boundary, through the routing kernel (fewer than 8 tokens) and the kernel that prepares the rows."""
+    """bf16 rows on a 4-byte boundary, through the routing kernel (1 and 3 tokens, and blocks of 16) and the kernel that prepares the rows."""
     c = m.Context(0, max_tokens=16, max_experts=E, top_k=K)
     c.set_prefill_min_tokens(min_tokens)
     L = m.Layer(c, fmt, E)

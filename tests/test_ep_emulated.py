@@ -82,7 +82,9 @@ def oracle_chain(R, fmt, X, K):
 
 
 @pytest.mark.parametrize("world,T,fmt", [(2, 16, m.FMT_SYM_F16), (3, 5, m.FMT_SYM_F16), (4, 64, m.FMT_SYM_F16), (8, 64, m.FMT_SYM_F16),
-                                         (2, 7, m.FMT_ZP), (3, 20, m.FMT_SYM_F32)])
+                                         (2, 7, m.FMT_ZP), (3, 20, m.FMT_SYM_F32),
+                                         # K slices on four warps: work lists made in the kernel and by a planning launch
+                                         (2, 8, m.FMT_SYM_F16), (3, 15, m.FMT_SYM_F16), (2, 8, m.FMT_SYM_F32), (3, 15, m.FMT_SYM_F32), (1, 1, m.FMT_ZP)])
 def test_residual_blocks_match_the_oracle_chain(world, T, fmt):
     E, K, NL = 32, 8, 3
     R = Ranks(world, E, T, K, NL, fmt, seed=10 + world)

@@ -66,19 +66,24 @@ def test_a_threshold_of_any_size_keeps_batches_on_the_streaming_kernels(fmt):
 
 
 @pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_SYM_F32, m.FMT_ZP])
-def test_grouped_gemm_repeats_bit_for_bit(fmt):
-    """Tiles of 6 to 30 tokens over every expert: the weight ring turns over as fast as it can. A pair's result does not depend on its
-    place in a tile, so every run gives the same bits; weights that are overwritten before they are read do not."""
+@pytest.mark.parametrize("x_type", [torch.float32, torch.bfloat16])
+def test_grouped_gemm_repeats_bit_for_bit(fmt, x_type):
+    """Tiles of 6 to 30 tokens over every expert, with two activation rows a token and, of bf16 tokens, one, where the weight ring turns over
+    as fast as it can. The streaming kernels' results within the bars, and a pair's result does not depend on its place in a tile, so
+    every run gives the same bits; weights that are overwritten before they are read do not."""
     T, E = 512, 256
     c = m.Context(0, max_tokens=T, max_experts=E, top_k=K)
-    c.set_prefill_min_tokens(1)
     L = m.Layer(c, fmt, E)
     L.fill_synth(3, 0)
     rng = np.random.default_rng(11)
     L.set_router((rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32))
-    X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(DEV)
+    X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(DEV).to(x_type)
     try:
+        c.set_prefill_min_tokens(1 << 20)
+        want = L.forward(X, T, K).cpu().numpy()
+        c.set_prefill_min_tokens(1)
         first = L.forward(X, T, K).clone()
+        check_ffn(first.cpu().numpy(), want, fmt, f"grouped GEMM against the streaming kernels, {T} {x_type} tokens")
         for _ in range(40):
             assert torch.equal(L.forward(X, T, K), first)
         assert c.status() == 0

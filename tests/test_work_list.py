@@ -254,3 +254,94 @@ def test_one_zero_point_token_by_its_number_of_experts(K):
         check_ffn(got, ref, m.FMT_ZP, f"one zero-point token through {K} experts")
     finally:
         L.close(); c.close()
+
+
+@pytest.mark.parametrize("fmt", [m.FMT_SYM_F16, m.FMT_SYM_F32])
+def test_k_slices_on_four_warps_of_a_planned_list(fmt):
+    """The same form with the work list of a planning launch (288 experts): the partial sums lie behind a list of another size. 4 and 8 pairs a
+    pass agree bit for bit, and the kernels are resident as often as their grids assume."""
+    E, K = 288, 8
+    c = m.Context(0, max_tokens=15, max_experts=E, top_k=K)
+    L = m.Layer(c, fmt, E)
+    L.fill_synth(4, 0)
+    rng = np.random.default_rng(29)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32)
+    W[40:] *= 0.2   # most pairs go to 40 experts: wide sub-items too
+    L.set_router(W)
+    host = [m.synth_expert_host(fmt, 4, 0, e) for e in range(E + 1)]
+    try:
+        for T in (8, 15):
+            X = rng.standard_normal((T, 2048)).astype(np.float32)
+            idx = torch.empty(T, K, dtype=torch.int32, device=DEV)
+            outs = []
+            for p in (4, 8):
+                c.set_pairs_per_pass(p)
+                outs.append(L.forward(dev(X), T, K, idx=idx).cpu().numpy())
+            ref, ids, _, _ = o.layer_forward(fmt, host, W, X, K)
+            assert c.status() == 0 and np.array_equal(idx.cpu().numpy(), ids)
+            assert np.array_equal(outs[0], outs[1])
+            check_ffn(outs[1], ref, fmt, f"K slices on four warps, planned list, {T} tokens")
+    finally:
+        L.close(); c.close()
+    assert m.short_residency() == 0
+
+
+@pytest.mark.parametrize("x_type", [torch.float32, torch.bfloat16])
+def test_blocks_of_a_few_tokens_with_more_than_256_experts(x_type):
+    """The routing kernel that makes the norm, in its form for up to 1024 experts, against the oracle."""
+    E, K, fmt = 288, 8, m.FMT_SYM_F16
+    c = m.Context(0, max_tokens=16, max_experts=E, top_k=K)
+    L = m.Layer(c, fmt, E, router_dtype=m.F16)
+    L.fill_synth(4, 0)
+    rng = np.random.default_rng(31)
+    W = (rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float16)
+    L.set_router(W)
+    host = [m.synth_expert_host(fmt, 4, 0, e) for e in range(E + 1)]
+    try:
+        for T in (1, 8, 16):
+            X = torch.from_numpy(rng.standard_normal((T, 2048)).astype(np.float32)).to(x_type)
+            xf = X.float().numpy()
+            idx = torch.empty(T, K, dtype=torch.int32, device=DEV)
+            got = L.forward(X.to(DEV), T, K, idx=idx, flags=2).cpu().numpy()
+            ref, ids, _, _ = o.layer_forward(fmt, host, W, o.rmsnorm(xf), K)
+            assert c.status() == 0 and np.array_equal(idx.cpu().numpy(), ids)
+            check_ffn(got, xf + ref, fmt, f"block of {T} {x_type} tokens, {E} experts")
+    finally:
+        L.close(); c.close()
+
+
+@pytest.mark.parametrize("fmt, K", [(m.FMT_SYM_F32, 8), (m.FMT_SYM_F16, 3), (m.FMT_SYM_F16, 15), (m.FMT_ZP, 9)])
+def test_small_stack_of_other_numbers_of_experts(fmt, K):
+    """Stacks whose layers' ends and routings are one kernel, with fewer and more ranks than the eight it requests at once: the bits of the
+    layers called one after the other. A stack whose capture fails between leaves nothing behind."""
+    E, NL, T = 64, 3, 6
+    c = m.Context(0, max_tokens=T, max_experts=E, top_k=15)
+    rng = np.random.default_rng(K)
+    layers = []
+    for l in range(NL):
+        L = m.Layer(c, fmt, E)
+        L.fill_synth(3, l)
+        L.set_router((rng.standard_normal((E + 1, 2048)) * 0.02).astype(np.float32))
+        layers.append(L)
+    stacks = []
+    try:
+        X = dev(rng.standard_normal((T, 2048)).astype(np.float32))
+        want = X
+        for L in layers:
+            want = L.forward(want, T, K, flags=2)
+        stacks.append(m.Stack(c, layers, T, K))
+        assert stacks[0].kernel_count == 3 * NL + 1
+        assert torch.equal(stacks[0].run(X), want)
+        c.selftest_fail()
+        with pytest.raises(m.MoexbError, match="self-test"):
+            m.Stack(c, layers, T, K)
+        assert torch.equal(stacks[0].run(X), want)
+        stacks.append(m.Stack(c, layers, T, K))
+        assert torch.equal(stacks[1].run(X), want) and torch.equal(layers[0].forward(X, T, K, flags=2), layers[0].forward(X, T, K, flags=2))
+        assert c.status() == 0
+    finally:
+        for s in stacks:
+            s.close()
+        for L in layers:
+            L.close()
+        c.close()
