@@ -1101,7 +1101,11 @@ static int tiled_launch_one(moexb_ctx* c, const TiledArgs& a, int T, int K, void
     // (K = 2, 4, 8, 11, 12, 15: 21.8 / 18.9, 24.1 / 19.5, 26.7 / 22.3, 30.1 / 29.5, 30.8 / 30.8, 32.0 / 32.2 us a layer, without and with; symmetric
     // formats 19.2 either way), and 8 to 15 tokens of the symmetric formats, where whole rounds are two or three per CTA and leave many
     // CTAs with one less (8, 9, 11, 14 tokens 47.9, 50.1, 55.8, 58.3 -> 46.7, 49.2, 52.6, 58.0 us; stacks of 10 and 12 43.7, 48.1 -> 41.6, 44.2;
-    // 16 and 23 tokens 59.8, 71.5 -> 60.5, 72.1; zero point 9 and 14 tokens 71.4, 92.9 -> 73.1, 90.1).
+    // 16 and 23 tokens 59.8, 71.5 -> 60.5, 72.1; zero point 9 and 14 tokens 71.4, 92.9 -> 73.1, 90.1). What decides is how many whole rounds the
+    // list gives a CTA, which the host does not know: of 312 lists of 2 to 187 sub-items (8 to 15 tokens, 1 to 15 ranks, 32 to 512 experts) those
+    // of 0.8 to 1, 1.9 to 2, 2.5 to 3 and more than 3.5 rounds take up to 6.6 % longer, all others up to 27 % less, the mean 4.1 % less. 15 tokens
+    // of 256 experts take 57.4 -> 59.3 us when they are independent and 50.0 -> 45.9 when they share experts; a rank's 32 of 256 experts 25.0 -> 21.6
+    // (8 tokens) and 29.8 -> 28.0 (15). Asking for the list on the device cost what it gave: both loops in one kernel are compiled worse.
     if constexpr (!DOWN && FMT == FMT_ZP) { if (T == 1 && 12 * (K + 1) <= c->sms) return tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream); }
     else if constexpr (!DOWN) {
         if (T >= 8 && T < 16) return c->pairs_per_pass == 4 ? tiled_launch_cfg<FMT, DOWN, 16, 2, 1, 1, SRC, true>(c, a, pa, ba, stream)
@@ -1162,9 +1166,9 @@ static int grouped_launch_one(moexb_ctx* c, const GroupedArgs& a, const GroupedM
 // Batches from this size on run on the grouped GEMM; where the lines cross depends on how many experts the tokens share. Zero-point blobs
 // from a third of the symmetric formats' size on: their streaming kernels take twice the MMAs and four pairs a pass. us a layer,
 // streaming against grouped, of independent tokens and of a 12-layer stack whose tokens have grown alike:
-//   symmetric   192 tokens 160 / 193 and 162 / 181, 256 tokens 192 / 210 and 194 / 193, 304 tokens 217 / 214, 336 tokens 232 / 214 and 231 / 209
-//   zero point   72 tokens 206 / 212 and 167 / 116,  88 tokens 224 / 224 and 185 / 115, 128 tokens 285 / 228 and 250 / 143
-// (the stacks' figures are those of the grouped GEMM before its hand-offs were shortened, which took 2 to 5 % off it)
+//   symmetric   192 tokens 157 / 184 and 160 / 174, 256 tokens 188 / 202 and 195 / 186, 288 tokens 207 / 202 and 207 / 188, 336 tokens 230 / 207 and 229 / 194
+//   zero point   40 tokens 159 / 169 and 101 / 82, 72 tokens 209 / 213 and 154 / 110, 88 tokens 226 / 217 and 177 / 111, 128 tokens 283 / 219 and 242 / 124
+// Independent symmetric tokens cross at about 280, those of a stack at 225: at 256 the ones lose 7 % and the others gain 5 %.
 static int grouped_min_tokens(const moexb_ctx* c, int fmt) {
     const int t = c->prefill_min_tokens;
     return fmt == FMT_ZP ? t / 3 + (t % 3 != 0) : t;   // (any threshold up to the largest int)
@@ -1412,8 +1416,8 @@ static int clear_buckets(moexb_ctx* c, cudaStream_t st) {
     c->buckets_dirty = cap != cudaStreamCaptureStatusNone;
     return MOEXB_OK;
 }
-// The router adds to the bucket counts and the combine kernel clears them; a call that returns between the two clears them itself, so
-// that neither the next call nor the replay of a graph finds its pairs there. Where that fails too, the next call does it.
+// The router adds to the bucket counts; the combine kernel clears them, or the down kernel where there is none (a layer of a small stack that
+// leaves its end to the next one). A call that returns between the two clears them itself, so that neither the next call nor the replay of a graph finds its pairs there. Where that fails too, the next call does it.
 struct BucketCounts {
     moexb_ctx* c; cudaStream_t st; bool open = false;
     ~BucketCounts() {
@@ -1674,7 +1678,7 @@ int moexb_stack_create(moexb_ctx* c, moexb_layer* const* layers, int n_layers, i
     if (e != cudaSuccess) { moexb_stack_destroy(s); return fail(MOEXB_ERR_CUDA, "stack_create: begin capture: %s", cudaGetErrorString(e)); }
     // 2 to 12 tokens (zero point 8): a layer's end and the next one's routing are one kernel, where every layer has its buckets and all its experts here
     // (us a layer, two kernels against one: 9, 10, 12, 16, 20 tokens 40.0 / 37.8, 41.2 / 40.4, 44.5 / 44.1, 50.3 / 50.0, 54.8 / 58.0;
-    // zero point 8 and 12 tokens 45.9 / 41.8 and 58.2 / 61.2)
+    // zero point 8 and 12 tokens 45.9 / 41.8 and 58.2 / 61.2; 4 to 15 ranks and 32 to 256 experts, from 15 % less to 0.4 % more)
     bool chain = residual && T > 1 && T <= (layers[0]->fmt == FMT_ZP ? 8 : 12) && layers[0]->layout == MOEXB_LAYOUT_TILED && c->bpairs && T < grouped_min_tokens(c, layers[0]->fmt);
     for (int l = 0; l < n_layers && chain; l++) chain = layers[l]->n_local == layers[l]->n_routed;
     const void* xin = s->x_in;

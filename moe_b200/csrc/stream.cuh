@@ -548,7 +548,8 @@ __global__ void __launch_bounds__(256) reduce_residual_norm_k(const float* __res
 // shared memory before the wait, every lane its own pieces. Sums and their order are those of the two kernels. 64 KB (f16: 32 KB) of
 // dynamic shared memory.
 // ranks = 0: the first block of a stack or a block of its own. The row is x (f32 or bf16), out its widened copy, if wanted; the launch of
-// layer_rows_k is the one that is saved (1, 2, 4 Q4_K and 8 tokens 22.5, 25.8, 45.4 and 49.5 -> 20.8, 24.0, 42.7 and 42.8 us a layer).
+// layer_rows_k is the one that is saved (1, 2, 4 Q4_K and 8 tokens 22.5, 25.8, 45.4 and 49.5 -> 20.8, 24.0, 42.7 and 42.8 us a layer). Every
+// block makes the norm again, so that the line depends on the experts too (norm_in_route in layer_impl).
 template <typename WT, int NJ, bool F16, typename XT>
 __global__ void __launch_bounds__(256, 2) combine_route_k(const WT* __restrict__ W, float* __restrict__ y, int E, int K, int norm, int* __restrict__ done, const TopkOut o,
                                                           const float* __restrict__ ypair, const float* __restrict__ extra, const XT* __restrict__ x, int ranks,
@@ -777,7 +778,7 @@ __global__ void __launch_bounds__(1024) group_pairs_k(const int* __restrict__ id
 // without), and the list made from ids and weights inside the gate/up kernel 1.4 us more than this (4 tokens x 40 layers 1163, now
 // 1108 us).
 // The order of an expert's pairs is not pinned; a pair's result does not depend on its place. The combine kernel, which runs when
-// nothing reads the counts any more, clears them.
+// nothing reads the counts any more, clears them (the down kernel, where no combine kernel follows).
 constexpr int BK_MAX_E = 256, BK_LOCAL = 64;
 struct BucketArgs {
     const int* cnt;                   // [E] pairs of each expert

@@ -233,7 +233,7 @@ __host__ __device__ constexpr int tl_red_offset() { return NW * D * tl_slice_byt
 // Streaming expert kernel on the tiled layout. No producer warp: every warp is its own pipeline. A warp owns a ring of D
 // slice buffers; lane 0 issues one cp.async.bulk per slice (4-5 KB, one contiguous run of the blob) D slices ahead and
 // the warp waits on the slice's mbarrier before consuming it, so there is no cross-warp hand-off on the weight stream.
-// Work is split in rounds of NW consecutive row tiles of one sub-item (warp w takes tile w of the round); a CTA walks a
+// Work is split in rounds of NW consecutive row tiles of one sub-item (warp w takes tile w of the round; KSP: NW / 4 tiles); a CTA walks a
 // contiguous range of rounds, so its warps share the sub-item's 8 activation columns in shared memory and swap them
 // together when the range crosses into the next sub-item.
 // DOWN = false: row tile = 8 gate + 8 up rows, 4 slices (K = 2048); act = silu(gate) * up.
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(NW * 32, CPS) stream_tiled_k(const TiledArgs a
     uint8_t* ring = smem + warp * D * SB;
     uint64_t* full = bars + warp * D;
 
-    // slice q of this warp: round r0 + q / KS, row tile rin*NW + warp, K slice q % KS
+    // slice q of this warp: of round r0 + q / KSW, there row tile in_round of TPR, K slice q % KS (KSP: the warp's own)
     auto issue = [&](int q) {
         const int r = r0 + q / KSW, sub = r / RPS, rin = r % RPS, wt = rin * TPR + in_round;
         const uint8_t* src = sub_at(sub).slot + (size_t)(DOWN ? 256 + wt : wt * 4 + (KSP ? warp % KS : q % KS)) * SB;
